@@ -259,9 +259,12 @@ LJ_API lj_status lj_compute_half(lj_ctx* ctx, const lj_grid* g, const lj_params*
  * whose launch shape is fixed at 128 threads per particle, cudaLJ.cu:519-520).
  * Results do not depend on them except in the last bits of floating-point
  * sums.  pair_kernel, for particles binned with LJ_ORDER_X:
- *   0 = default: 10 when the grid averages 2 or more particles per cell, else 12,
- *   1 = one thread per target, neighbours through L1, its windows in shared
- *       memory (also the kernel of LJ_ORDER_INDEX),
+ *   0 = default: 1 when the grid averages 6 or more particles per cell, 10 from
+ *       2, else 12,
+ *   1 = cluster walk: a warp takes 8 consecutive targets of a row of cells,
+ *       keeps the candidates within the cutoff of their bounding box in shared
+ *       memory and evaluates that list, two candidates per step in paired FP32
+ *       instructions,
  *   6 = row passes: the 9 stencil rows walked in 5 warp-synchronous passes
  *       (opposite rows paired), coalesced neighbour loads, two candidates per
  *       step in paired FP32 instructions,
@@ -269,9 +272,10 @@ LJ_API lj_status lj_compute_half(lj_ctx* ctx, const lj_grid* g, const lj_params*
  *       merged, each candidate loaded once and tested against both targets in
  *       one paired FP32 evaluation, registers capped at 64 per thread, the
  *       windows parked in shared memory during the walk,
- *  11 = as 1 with the 9 rows walked whole (no row culling, no x-window
- *       searches): on sparse grids such as a sphere shell, where a row holds
- *       few particles, the searches cost more than the candidates they remove.
+ *  11 = one thread per target, neighbours through L1, the 9 rows walked whole
+ *       (no row culling, no x-window searches): on sparse grids such as a sphere
+ *       shell, where a row holds few particles, the searches cost more than the
+ *       candidates they remove.
  *  12 = targets paired inside their cell (a pair list built on the device:
  *       flags, their scan, the list; 12 bytes per target of scratch in the
  *       context): both targets of a lane share one 27-cell stencil, whose
@@ -281,12 +285,14 @@ LJ_API lj_status lj_compute_half(lj_ctx* ctx, const lj_grid* g, const lj_params*
  *       pick on a sphere shell and on a uniform grid of 0.5 particles per
  *       cell).  A target's results do not depend on its partner, so
  *       lj_compute_range gives the bits of lj_compute.
+ * Particles binned with LJ_ORDER_INDEX take the cluster walk (with whole cells
+ * for windows) where the value is 1 or the default rule gives 1, else the walk of 11.
  * The values 2-5 and 7-9 named variants that never won on any benchmark
  * workload (per-lane queues, register windows, cell-block tiles staged by TMA
  * bulk copies, scalar passes, SoA pairs); they are kept as aliases of the kernel
  * of their family: 2, 3, 4 run 1; 5, 7 run 6; 8, 9 run 10.
  * With a non-finite coordinate (reported as LJ_ERANGE) the outputs of the
- * particles whose windows hold it are unspecified under 6 and 10. */
+ * particles whose windows hold it are unspecified under 1, 6 and 10. */
 typedef struct {
     int pair_kernel;
     int scatter_passes; /* binning scatter in this many passes over cell ranges (0 = one pass per

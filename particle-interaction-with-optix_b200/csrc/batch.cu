@@ -8,7 +8,7 @@
 // range [first_s, first_s + n_s).  The pair kernel is persistent: CTAs take
 // (system, block of consecutive sorted targets) tiles from a device work
 // queue, largest estimated cost first, and evaluate each target with the same
-// per-target routine as the single-system kernel (pair_target), so per-target
+// per-target routine as the single-system kernel, so per-target
 // results equal a per-system run bit for bit.  Per-system totals are reduced
 // from per-target values in a fixed order (deterministic).  The whole step can
 // be captured once in a CUDA graph and replayed.
@@ -18,6 +18,7 @@
 #include <new>
 #include <vector>
 
+#include "pair_cluster.cuh"
 #include "pair_pass.cuh"
 
 namespace ljc {
@@ -28,8 +29,8 @@ struct SysDev {
     int cell_base;
     int first;
     int n;
-    int walk;  // 1: one target per lane (kernel 6's walk), 3: two targets per lane (kernel 10's), as the
-               // single-system default chooses for the system
+    int walk;  // 1: one target per lane (kernel 6's walk), 2: the cluster walk (kernel 1's), 3: two targets per
+               // lane (kernel 10's), as the single-system default chooses for the system
 };
 
 // ---------------------------------------------------------------- count
@@ -74,15 +75,16 @@ __global__ void __launch_bounds__(256) k_count_batched(const SysDev* __restrict_
 
 // ---------------------------------------------------------------- pair (persistent, tile queue)
 // Tile = (system, k0, k1): targets [k0, k1) of one system, at most
-// BLOCK * PPT of them (2 * BLOCK * PPT for MODE 3).  Each target runs the
-// per-target routine of the single-system kernel the default picks for the
-// system (MODE 1: pass_target, one target per lane, as kernel 6; MODE 3:
-// pass_target2, two targets per lane, as kernel 10), in the system's local
+// BLOCK * PPT of them (2 * BLOCK * PPT for MODE 2 and 3).  Each target runs the
+// routine of the single-system kernel the default picks for the
+// system (MODE 1: pass_target, one target per lane, as kernel 6; MODE 2:
+// cluster_stretch, as kernel 1; MODE 3: pass_target2, two targets per lane, as
+// kernel 10), in the system's local
 // indices, so per-particle results equal a per-system lj_compute with that
 // kernel bit for bit.  One launch per walk mode, over the tiles of the systems
 // using it.  Per-target raw sums go to te / tw / tnp for the per-system totals.
 template <int BLOCK, int PPT, int MODE>
-__global__ void __launch_bounds__(BLOCK) k_pair_batched(const SysDev* __restrict__ sys, const float4* __restrict__ p,
+__global__ void __launch_bounds__(BLOCK, MODE == 2 ? kCluWarpsPerSm * 32 / BLOCK : 1) k_pair_batched(const SysDev* __restrict__ sys, const float4* __restrict__ p,
                                                         const int* __restrict__ cs, const int* __restrict__ off,
                                                         const int4* __restrict__ tiles, int ntiles,
                                                         unsigned* tile_counter, float* __restrict__ energy,
@@ -99,6 +101,31 @@ __global__ void __launch_bounds__(BLOCK) k_pair_batched(const SysDev* __restrict
         const SysDev S = sys[d.x];
         const int ncell = S.g.gx * S.g.gy * S.g.gz;
         const float4* ps = p + S.first;
+        if (MODE == 2) {
+            // the groups of 16 targets that start in the tile, the block's warps in turn
+            __shared__ __align__(16) CluSmem sm[BLOCK / 32];
+            const int w = (int)(threadIdx.x >> 5);
+            cluster_stretch<true>(S.g, S.pp, ps, cs + S.first, S.cell_base, off + S.cell_base, S.first, S.n,
+                                  d.y - S.first, d.z - S.first, 0, S.n, w, BLOCK / 32, sm[w], status,
+                                  [&](int k, int s, bool valid, float v, float wv, unsigned np, int) {
+                                      wv += __shfl_xor_sync(0xffffffffu, wv, 16);
+                                      wv += __shfl_xor_sync(0xffffffffu, wv, 8);
+                                      np += __shfl_xor_sync(0xffffffffu, np, 16);
+                                      np += __shfl_xor_sync(0xffffffffu, np, 8);
+                                      if (!valid) return;
+                                      k += S.first;
+                                      if (s == 0) {
+                                          if (energy) energy[k] = S.pp.e4 * v;
+                                          te[k] = v;
+                                          tw[k] = wv;
+                                          tnp[k] = np;
+                                      } else if (force) {
+                                          force[3 * (size_t)k + (s - 1)] = -S.pp.fscale * v;
+                                      }
+                                  });
+            __syncthreads();  // s_t is reused by the next tile
+            continue;
+        }
         if (MODE == 3) {
             // two targets per thread (pass_target2): a = k, b = k + 1, windows parked in shared memory
             __shared__ int2 s_win[9][BLOCK];
@@ -243,7 +270,7 @@ struct lj_batch {
     int* d_firsts = nullptr;
     int4* d_tiles = nullptr;
     int ntiles = 0;
-    int ntiles1 = 0;  // tiles [0, ntiles1) use walk mode 1, the rest mode 3
+    int ntiles1 = 0, ntiles2 = 0;  // tiles [0, ntiles1) use walk mode 1, [ntiles1, ntiles2) mode 2, the rest mode 3
     size_t tiles_cap = 0;
     unsigned* d_counter = nullptr;
     int* counts = nullptr;
@@ -319,9 +346,10 @@ static lj_status build_grids(lj_batch* b) {
         d.cell_base = (int)base;
         d.first = y.first;
         d.n = y.n;
-        // the two-target walk where the single-system default takes kernel 10, else one target per
-        // lane (kernel 6's walk; the persistent tile queue has no pair list for kernel 12)
-        d.walk = default_pair_kernel(y.n, g) == 10 ? 3 : 1;
+        // the walk of the single-system default's kernel; kernel 6's where that is kernel 12 (the
+        // persistent tile queue has no pair list)
+        const int kernel = default_pair_kernel(y.n, g);
+        d.walk = kernel == 1 ? 2 : (kernel == 10 ? 3 : 1);
         base += (long long)g.dim[0] * g.dim[1] * g.dim[2];
         if (base > 2147483646LL) return LJ_EUNSUPPORTED;
     }
@@ -329,8 +357,8 @@ static lj_status build_grids(lj_batch* b) {
     return LJ_OK;
 }
 
-// Tiles of T = threads * per_thread consecutive targets per system (2T for systems on the two-target
-// walk): first those of the systems walked with mode 1, then mode 3, each group ordered by estimated
+// Tiles of T = threads * per_thread consecutive targets per system (2T for systems on the cluster or
+// the two-target walk): first those of the systems walked with mode 1, then 2, then 3, each ordered by estimated
 // cost (targets x expected candidates: n / box volume x cutoff^3), largest first.
 static std::vector<int4> build_tiles(const lj_batch* b) {
     const int T = b->cfg.threads * b->cfg.per_thread;
@@ -341,7 +369,7 @@ static std::vector<int4> build_tiles(const lj_batch* b) {
         for (int d = 0; d < 3; ++d) vol *= (double)y.hi[d] - (double)y.lo[d];
         const double rc = y.params.cutoff;
         const double per_target = (double)y.n / (vol > 0 ? vol : 1.0) * rc * rc * rc;
-        const int Ts = b->sd[s].walk == 3 ? 2 * T : T;  // the two-target walk takes 2 targets per thread
+        const int Ts = b->sd[s].walk == 1 ? T : 2 * T;
         for (int k0 = 0; k0 < y.n; k0 += Ts) {
             const int k1 = std::min(y.n, k0 + Ts);
             v.push_back({per_target * (k1 - k0), make_int4(s, y.first + k0, y.first + k1, 0)});
@@ -417,8 +445,10 @@ static lj_status build_plan(lj_ctx* ctx, lj_batch* b) {
                                       cudaMemcpyHostToDevice) != cudaSuccess))
         return LJ_ECUDA;
     b->ntiles = (int)tiles.size();
-    b->ntiles1 = count_tiles_below(b, tiles, 3);
+    b->ntiles1 = count_tiles_below(b, tiles, 2);
+    b->ntiles2 = count_tiles_below(b, tiles, 3);
     b->persistent_blocks[0] = ctx->sm_count * batched_occupancy(b->cfg.threads, b->cfg.per_thread, 1);
+    b->persistent_blocks[1] = ctx->sm_count * batched_occupancy(b->cfg.threads, b->cfg.per_thread, 2);
     b->persistent_blocks[2] = ctx->sm_count * batched_occupancy(b->cfg.threads, b->cfg.per_thread, 3);
     ++b->version;
     return LJ_OK;
@@ -448,7 +478,7 @@ static int occ_mode(int threads, int ppt) {
 }
 
 static int batched_occupancy(int threads, int ppt, int mode) {
-    return mode == 3 ? occ_mode<3>(threads, ppt) : occ_mode<1>(threads, ppt);
+    return mode == 3 ? occ_mode<3>(threads, ppt) : (mode == 2 ? occ_mode<2>(threads, ppt) : occ_mode<1>(threads, ppt));
 }
 
 // Tiles [t0, t1) with walk MODE; the persistent grid never exceeds the tile count.
@@ -464,7 +494,8 @@ static void launch_batched_mode(lj_ctx* ctx, lj_batch* b, const float* p4, float
 
 template <int BLOCK, int PPT>
 static void launch_batched_pair(lj_ctx* ctx, lj_batch* b, const float* p4, float* energy, float* force) {
-    launch_batched_mode<BLOCK, PPT, 3>(ctx, b, p4, energy, force, b->ntiles1, b->ntiles);
+    launch_batched_mode<BLOCK, PPT, 2>(ctx, b, p4, energy, force, b->ntiles1, b->ntiles2);
+    launch_batched_mode<BLOCK, PPT, 3>(ctx, b, p4, energy, force, b->ntiles2, b->ntiles);
     launch_batched_mode<BLOCK, PPT, 1>(ctx, b, p4, energy, force, 0, b->ntiles1);
 }
 
@@ -560,8 +591,8 @@ static lj_status batch_graph(lj_ctx* ctx, lj_batch* b, const float* x, const flo
 }
 
 // One plain lj_bin + lj_compute per system (the path the batched step replaces), each with the
-// single-system kernel of the walk the batched kernel takes for it (6: one target per lane, 10: two
-// targets per lane), so per-particle results are equal bit for bit.
+// single-system kernel of the walk the batched kernel takes for it (6: one target per lane, 1: the
+// cluster walk, 10: two targets per lane), so per-particle results are equal bit for bit.
 static lj_status batch_separate_one(lj_ctx* ctx, lj_batch* b, int s, const float* x, const float* y, const float* z,
                                     float* energy, float* force, int* index, lj_totals* totals);
 
@@ -570,7 +601,7 @@ static lj_status batch_separate(lj_ctx* ctx, lj_batch* b, const float* x, const 
     const lj_tuning saved = ctx->tuning;
     lj_status st = LJ_OK;
     for (int s = 0; s < b->nsys && st == LJ_OK; ++s) {
-        ctx->tuning.pair_kernel = b->sd[s].walk == 3 ? 10 : 6;
+        ctx->tuning.pair_kernel = b->sd[s].walk == 3 ? 10 : (b->sd[s].walk == 2 ? 1 : 6);
         st = batch_separate_one(ctx, b, s, x, y, z, energy, force, index, totals);
     }
     ctx->tuning = saved;

@@ -9,18 +9,12 @@
 // consecutive cells (contiguous in cell order) in lockstep passes, one float4
 // load per candidate shared by both targets.
 //
-// k_pair_config evaluates the truncated law with forces.  One thread per
-// sorted target particle.  For each of the 9 stencil rows it bounds the
-// squared distance from the target to the row in (y, z); rows that cannot
-// hold a partner are skipped, and, when particles are x-sorted within cells
-// (LJ_ORDER_X, so every row of 3 cells is x-sorted), binary search narrows
-// the row to the x-window [x - h, x + h], h = sqrt(rc^2 - dyz^2) plus a
-// rounding slack.  The windows are a superset of the interacting partners,
-// so the shared float distance test alone decides, and the pair count is
-// exact.  Pair math is FP32 from r^-2 (one approximate reciprocal), sums are
-// accumulated in registers, and the totals (energy, virial, pair count) are
-// reduced in FP64 / u64 per block and then by the last block in a fixed
-// order, so they are deterministic.
+// k_pair_config evaluates the truncated law with forces, one thread per sorted target particle, over
+// the 9 stencil rows walked whole (kernel 11, and sparse grids binned with LJ_ORDER_INDEX); the shared
+// float distance test alone decides, so the pair count is exact.  Pair math is FP32 from r^-2 (one
+// approximate reciprocal), sums are accumulated in registers, and the totals (energy, virial, pair
+// count) are reduced in FP64 / u64 per block and then by the last block in a fixed order, so they are
+// deterministic.
 #include <cfloat>
 #include <climits>
 
@@ -28,19 +22,21 @@
 
 namespace ljc {
 
-constexpr double kPairCell = 2.0;    // particles per cell from which the default takes two targets per lane
+constexpr double kClusterCell = 6.0;  // particles per cell from which the default takes the cluster walk
+constexpr double kPairCell = 2.0;     // ... and below that, two targets per lane
 
-// Default pair kernel for LJ_ORDER_X (measured on B200): the packed row passes with two targets per
-// lane (kernel 10) from 2 particles per cell up (10M at 10 per cell: 2.33 ms against 2.88 ms for one
-// target per lane; 80 per cell: 11.4 ms against 12.6 ms for the SoA walk); below, the targets paired
-// inside their cell over whole rows (kernel 12: a 4M sphere shell on 64M cells 0.517 ms against 0.597
-// for kernel 11 and 0.75 for kernel 6; 0.5M uniform on 100^3 cells 0.055 ms against 0.060 for
-// kernel 6), where windows merged across cells add more candidates than the shared loads save.
+// Default pair kernel (measured on B200, pair stage, 2M uniform particles): the cluster walk (1) from
+// 6 particles per cell up (484 against 514 us for kernel 10 at 10 per cell, 401 against 367 at 5), the
+// row passes with two targets per lane (10) from 2 (285 against 379 us for kernel 1 at 2 per cell), and
+// below, the targets paired inside their cell over whole rows (kernel 12: a 4M sphere shell on 64M cells
+// 0.517 ms against 0.597 for kernel 11 and 0.75 for kernel 6; 0.5M uniform on 100^3 cells 0.055 ms
+// against 0.060 for kernel 6), where windows merged across cells add more candidates than the shared
+// loads save.
 int default_pair_kernel(int n, const lj_grid& g) {
-    return (double)n / ((double)g.dim[0] * g.dim[1] * g.dim[2]) >= kPairCell ? 10 : 12;
+    const double per_cell = (double)n / ((double)g.dim[0] * g.dim[1] * g.dim[2]);
+    return per_cell >= kClusterCell ? 1 : (per_cell >= kPairCell ? 10 : 12);
 }
 
-template <bool XWIN>
 __global__ void __launch_bounds__(kPairThreads) k_pair_config(GridDev g, PairParams pp, const float4* __restrict__ p,
                                                               const int* __restrict__ cs,
                                                               const int* __restrict__ off, int n, int kb, int ke,
@@ -57,7 +53,7 @@ __global__ void __launch_bounds__(kPairThreads) k_pair_config(GridDev g, PairPar
             atomicOr(status, kFlagRange);
             c = 0;
         }
-        pair_target<XWIN, kPairThreads>(g, pp, p, off, n, k, c, s_win, ea, fx, fy, fz, wa, np);
+        pair_target<kPairThreads>(g, pp, p, off, n, k, c, s_win, ea, fx, fy, fz, wa, np);
         const int o = out_slot(pp, p, k, n, status);
         if (o >= 0 && energy) energy[o] = pp.e4 * ea;
         if (o >= 0 && force) {
@@ -276,11 +272,14 @@ lj_status launch_pair_config(lj_ctx* ctx, const lj_grid* g, const lj_params* prm
     pp.fscale = -pp.e24 / pp.sig2;
     pp.slack = grid_slack(*g);
     pp.by_index = by_index ? 1 : 0;
+    int kernel = ctx->tuning.pair_kernel;
+    if (kernel == 0) kernel = default_pair_kernel(n, *g);
+    // retired variants run the surviving kernel of their family: 2, 3, 4 -> 1; 5, 7 -> 6; 8, 9 -> 10
+    const bool cluster = kernel >= 1 && kernel <= 4;
+    if (cluster)
+        return launch_pair_cluster(ctx, g, pp, n, xyzi, cs, off, order == LJ_ORDER_X, energy, force, totals, kb, ke);
     if (order == LJ_ORDER_X) {
-        int kernel = ctx->tuning.pair_kernel;
-        if (kernel == 0) kernel = default_pair_kernel(n, *g);
         switch (kernel) {
-            // retired variants run the surviving kernel of their family: 2, 3, 4 -> 1; 5, 7 -> 6; 8, 9 -> 10
             case 5:
             case 6:
             case 7: return launch_pair_pass(ctx, g, pp, n, xyzi, cs, off, false, energy, force, totals, kb, ke);
@@ -288,9 +287,10 @@ lj_status launch_pair_config(lj_ctx* ctx, const lj_grid* g, const lj_params* prm
             case 9:
             case 10: return launch_pair_pass(ctx, g, pp, n, xyzi, cs, off, true, energy, force, totals, kb, ke);
             case 12: return launch_pair_cellpair(ctx, g, pp, n, xyzi, cs, off, energy, force, totals, kb, ke);
-            default: break;  // 1 (and 2, 3, 4): windows in shared memory; 11: whole rows (below)
+            default: break;  // 11
         }
     }
+    // kernel 11 (and LJ_ORDER_INDEX, unless it takes the cluster walk): the 9 rows walked whole
     const int blocks = (ke - kb + kPairThreads - 1) / kPairThreads;
     const size_t need = 256 + (size_t)blocks * sizeof(Partial);
     if (need > ctx->red_bytes) {
@@ -301,16 +301,8 @@ lj_status launch_pair_config(lj_ctx* ctx, const lj_grid* g, const lj_params* prm
     unsigned* counter = static_cast<unsigned*>(ctx->red);
     Partial* part = reinterpret_cast<Partial*>(static_cast<char*>(ctx->red) + 256);
     const float4* p4 = reinterpret_cast<const float4*>(xyzi);
-    // kernel 11 walks the 9 rows whole, without the culling and x-window searches: on sparse grids
-    // (few particles per row) the searches cost more than the candidates they remove
-    const bool xwin = order == LJ_ORDER_X && ctx->tuning.pair_kernel != 11;
-    if (xwin)
-        k_pair_config<true><<<blocks, kPairThreads, 0, ctx->stream>>>(to_dev(*g), pp, p4, cs, off, n, kb, ke, energy,
-                                                                      force, part, counter, totals, ctx->d_status);
-    else
-        k_pair_config<false><<<blocks, kPairThreads, 0, ctx->stream>>>(to_dev(*g), pp, p4, cs, off, n, kb, ke,
-                                                                       energy, force, part, counter, totals,
-                                                                       ctx->d_status);
+    k_pair_config<<<blocks, kPairThreads, 0, ctx->stream>>>(to_dev(*g), pp, p4, cs, off, n, kb, ke, energy, force, part,
+                                                            counter, totals, ctx->d_status);
     return last_launch_status();
 }
 

@@ -159,11 +159,9 @@ __device__ void reduce_totals(double e, double w, unsigned long long np, Partial
 }
 
 
-// Per-target work of the truncated law: windows and walk.  `c` is the
-// target's cell in grid g, `off` the offsets of that grid (values are indices
-// into p), `n` bounds every index.  Shared by the single-system kernel and
-// the batched kernel so both produce the same per-target results.
-template <bool XWIN, int BLOCK>
+// Per-target work of the truncated law over whole rows.  `c` is the target's cell in grid g, `off` the
+// offsets of that grid (values are indices into p), `n` bounds every index.
+template <int BLOCK>
 __device__ __forceinline__ void pair_target(const GridDev& g, const PairParams& pp, const float4* __restrict__ p,
                                             const int* __restrict__ off, int n, int k, int c,
                                             int2 (*s_win)[BLOCK], float& ea, float& fx, float& fy, float& fz,
@@ -173,36 +171,18 @@ __device__ __forceinline__ void pair_target(const GridDev& g, const PairParams& 
     int cx, cy, cz;
     decode_cell(g, c, cx, cy, cz);
     const int xl = max(cx - 1, 0), xh = min(cx + 1, g.gx - 1);
-    const float slack = pp.slack + 8.0f * FLT_EPSILON * fmaxf(fabsf(pi.x), fmaxf(fabsf(pi.y), fabsf(pi.z)));
     int nw = 0;
 #pragma unroll
     for (int dz = -1; dz <= 1; ++dz) {
         const int z = cz + dz;
         if (z < 0 || z >= g.gz) continue;
-        float dzm = 0.f;
-        if (XWIN) {
-            if (dz < 0) dzm = pi.z - fmaf((float)cz, g.w, g.oz);
-            if (dz > 0) dzm = fmaf((float)(cz + 1), g.w, g.oz) - pi.z;
-            dzm = fmaxf(dzm - slack, 0.f);
-        }
 #pragma unroll
         for (int dy = -1; dy <= 1; ++dy) {
             const int y = cy + dy;
             if (y < 0 || y >= g.gy) continue;
             const int rb = (z * g.gy + y) * g.gx;
-            int s = min(max(__ldg(&off[rb + xl]), 0), n);
-            int e = min(max(__ldg(&off[rb + xh + 1]), s), n);
-            if (XWIN) {
-                float dym = 0.f;
-                if (dy < 0) dym = pi.y - fmaf((float)cy, g.w, g.oy);
-                if (dy > 0) dym = fmaf((float)(cy + 1), g.w, g.oy) - pi.y;
-                dym = fmaxf(dym - slack, 0.f);
-                const float d2 = fmaf(dym, dym, dzm * dzm);
-                if (d2 >= pp.rc2w) continue;
-                const float h = sqrtf(pp.rc2w - d2) + slack;
-                s = lower_x(p, s, e, pi.x - h);
-                e = upper_x(p, s, e, pi.x + h);
-            }
+            const int s = min(max(__ldg(&off[rb + xl]), 0), n);
+            const int e = min(max(__ldg(&off[rb + xh + 1]), s), n);
             if (dz == 0 && dy == 0) {
                 s_win[nw++][tid] = make_int2(s, k);
                 s_win[nw++][tid] = make_int2(k + 1, e);
@@ -271,6 +251,10 @@ lj_status launch_pair_pass(lj_ctx* ctx, const lj_grid* g, const PairParams& pp, 
 lj_status launch_pair_cellpair(lj_ctx* ctx, const lj_grid* g, const PairParams& pp, int n, const float* xyzi,
                                const int* cs, const int* off, float* energy, float* force, lj_totals* totals,
                                int kb, int ke);
+// Cluster walk (pair_cluster.cu), kernel 1; xwin: the rows are x-sorted (LJ_ORDER_X).
+lj_status launch_pair_cluster(lj_ctx* ctx, const lj_grid* g, const PairParams& pp, int n, const float* xyzi,
+                              const int* cs, const int* off, bool xwin, float* energy, float* force,
+                              lj_totals* totals, int kb, int ke);
 // Exclusive scan of counts[ncells] into offsets[0..ncells] on the context's stream (bin.cu).
 lj_status launch_scan(lj_ctx* ctx, const int* counts, long long ncells, int* offsets);
 }  // namespace ljc

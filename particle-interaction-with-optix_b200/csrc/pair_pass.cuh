@@ -2,7 +2,7 @@
 // (per-target routine shared by k_pair_pass in pair_pass.cu and the batched
 // kernel in batch.cu).
 //
-// Same windows, float test and law as k_pair_config (pair.cu); what changes is
+// Same float test and law as k_pair_config (pair.cu); what changes is
 // the order in which a warp walks them.  The 9 stencil rows are taken in 5
 // passes, each pass walked by the whole warp in lockstep for as many steps as
 // its longest lane needs:
@@ -86,8 +86,8 @@ __device__ __forceinline__ void walk_pass(const float4* __restrict__ p, int k, i
 // The 9 row windows of target k (local indices in [0, n)): for row r = (dz + 1) * 3 + (dy + 1),
 // [ws[r], ws[r] + wl[r]), empty when the row is off the grid or its (y, z) distance bound exceeds the
 // cutoff.  `off` holds the offsets of the target's grid; obase is subtracted from them (the index of
-// the system's first particle when the offsets count from a larger array).  Same culling, slack and
-// searches as pair_target (pair_common.cuh), so the windows are identical.
+// the system's first particle when the offsets count from a larger array).  The
+// windows are a superset of the interacting partners.
 __device__ __forceinline__ void pass_windows(const GridDev& g, const PairParams& pp, const float4* __restrict__ p,
                                              const int* __restrict__ off, int obase, int n, const float4& pi, int c,
                                              int (&ws)[9], int (&wl)[9]) {

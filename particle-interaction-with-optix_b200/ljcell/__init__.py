@@ -58,10 +58,10 @@ class Particles(C.Structure):
 
 
 class Tuning(C.Structure):
-    """lj_tuning: implementation choices (pair_kernel 0 default, 1 one target per thread with windows in
-    shared memory, 6 row passes, 10 row passes with two targets per lane, 11 as 1 with whole rows, 12
-    targets paired inside their cell over whole rows; the retired values 2-5 and 7-9 run the kernel of
-    their family)."""
+    """lj_tuning: implementation choices (pair_kernel 0 default, 1 clusters of 8 targets walking a shared
+    candidate list, 6 row passes, 10 row passes with two targets per lane, 11 one target per thread over
+    whole rows, 12 targets paired inside their cell over whole rows; the retired values 2-5 and 7-9 run
+    the kernel of their family)."""
 
     _fields_ = [("pair_kernel", C.c_int), ("scatter_passes", C.c_int), ("reserved", C.c_int * 6)]
 

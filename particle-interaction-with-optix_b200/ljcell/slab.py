@@ -145,15 +145,18 @@ class SlabResult:
     halo: int            # halo particles received
 
 
-# Particles per cell from which the library's default pair kernel takes two consecutive targets
-# per lane with x-windows (kernel 10) instead of targets paired inside their cell over whole rows
-# (kernel 12).  The library applies it to n / ncells of the whole grid; a slab fills only its own
-# layers, so `step` applies it to the occupancy of those.
+# Particles per cell from which the library's default pair kernel is the cluster walk (kernel 1), and
+# from which it takes two consecutive targets per lane with x-windows (kernel 10) instead of targets
+# paired inside their cell over whole rows (kernel 12).  The library applies them to n / ncells of the
+# whole grid; a slab fills only its own layers, so `step` applies them to the occupancy of those.
+CLUSTER_CELL = 6.0
 PAIR_CELL = 2.0
 
 
 def pair_kernel_for(dom: SlabDomain, targets: int) -> int:
     cells = (dom.z1 - dom.z0) * dom.gx * dom.gy
+    if targets >= CLUSTER_CELL * cells:
+        return 1
     return 10 if targets >= PAIR_CELL * cells else 12
 
 
