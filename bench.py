@@ -58,9 +58,13 @@ SCATTER_REGION = 56 << 20   # bytes of scattered records per binning scatter pas
 
 
 def bin_launches(n: int, ncells: int) -> int:
-    """Kernels one lj_bin launches: count, scan, the scatter passes, rank, large-cell sort."""
-    passes = max(1, min(8, ncells, -(-16 * n // SCATTER_REGION)))
-    return 4 + passes
+    """Kernels one lj_bin launches: count, scan, the scatter passes, rank, large-cell sort; or, by segments
+    of cells (4 million particles and more, up to 256 per cell): count, the scatter passes, two sorts, and
+    the six ticket kernels behind the gate (a grid beyond 16384 x 8192 cells takes tickets)."""
+    passes = max(1, min(8, -(-16 * n // SCATTER_REGION)))
+    if n >= 4_000_000 and n <= 256 * ncells and ncells <= 16384 * 8192:
+        return 3 + passes + 6
+    return 4 + min(passes, ncells)
 
 CONFIGS = {
     "c1": dict(workload="uniform 100k, rc=0.05", n=100_000, dist="uniform", lo=(0, 0, 0), hi=(1, 1, 1), rc=0.05),

@@ -15,9 +15,13 @@
 #include <algorithm>
 #include <climits>
 
-#include "ljcell_internal.cuh"
+#include "bin_common.cuh"
 
 namespace ljc {
+
+// A kernel of the ticket path behind the segment path's gate (bin_segment.cu): it has work only when
+// the gate is open (nonzero); without a gate it always has.
+__device__ __forceinline__ bool closed(const unsigned* gate) { return gate && __ldg(gate) == 0u; }
 
 // ---------------------------------------------------------------- counting
 // One thread per particle, grid-stride by whole warps.  Lanes that share a
@@ -29,7 +33,8 @@ template <bool TICKETS>
 __global__ void __launch_bounds__(256) k_count(GridDev g, const float* __restrict__ x, const float* __restrict__ y,
                                                const float* __restrict__ z, int stride, int n,
                                                int* __restrict__ counts, int2* __restrict__ ct,
-                                               unsigned* status) {
+                                               unsigned* status, const unsigned* __restrict__ gate) {
+    if (closed(gate)) return;
     const int lane = threadIdx.x & 31;
     const long long gwarp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -78,7 +83,9 @@ __device__ __forceinline__ void st_state(unsigned long long* p, unsigned long lo
 __global__ void __launch_bounds__(kScanThreads) k_scan(const int* __restrict__ counts, int* __restrict__ offsets,
                                                        long long n, long long ntiles,
                                                        unsigned long long* tile_state, unsigned* tile_counter,
-                                                       int vec_ok, unsigned* status) {
+                                                       int vec_ok, unsigned* status,
+                                                       const unsigned* __restrict__ gate = nullptr) {
+    if (closed(gate)) return;
     __shared__ unsigned s_tile;
     __shared__ long long s_warp[8];
     __shared__ long long s_prefix;
@@ -213,7 +220,9 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const int* __restrict__ c
 __global__ void __launch_bounds__(256) k_scatter(const float* __restrict__ x, const float* __restrict__ y,
                                                  const float* __restrict__ z, int stride, int n,
                                                  const int2* __restrict__ ct, const int* __restrict__ offsets,
-                                                 float4* __restrict__ tmp, unsigned* status, int c_lo, int c_hi) {
+                                                 float4* __restrict__ tmp, unsigned* status, int c_lo, int c_hi,
+                                                 const unsigned* __restrict__ gate = nullptr) {
+    if (closed(gate)) return;
     constexpr int U = 4;
     const long long step = (long long)gridDim.x * blockDim.x;
     for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += U * step) {
@@ -247,25 +256,7 @@ __global__ void __launch_bounds__(256) k_scatter(const float* __restrict__ x, co
     }
 }
 
-// ---------------------------------------------------------------- within-cell sort
-// Keys: LJ_ORDER_INDEX sorts by original index; LJ_ORDER_X by x, then index.
-// Indices are unique, so keys are unique and the result is a pure function of
-// the input.
-template <int ORDER>
-__device__ __forceinline__ bool key_less(float xa, int ia, float xb, int ib) {
-    if (ORDER == LJ_ORDER_X) return (xa < xb) || (xa == xb && ia < ib);
-    return ia < ib;
-}
-
-struct SortOut {
-    float4* out4;
-    int* out_cell;
-    float* sx;
-    float* sy;
-    float* sz;
-    int* sidx;
-};
-
+// ---------------------------------------------------------------- within-cell sort (keys: bin_common.cuh)
 __device__ __forceinline__ void emit(const SortOut& o, long long slot, float4 r, int cell) {
     o.out4[slot] = r;
     o.out_cell[slot] = cell;
@@ -290,7 +281,9 @@ template <int ORDER>
 __global__ void __launch_bounds__(256) k_cell_rank(const float4* __restrict__ tmp, const int* __restrict__ offsets,
                                                    GridDev g, const BinSys* __restrict__ sys,
                                                    const int* __restrict__ firsts, int nsys, int n, SortOut so,
-                                                   int* large, int large_cap, unsigned* status) {
+                                                   int* large, int large_cap, unsigned* status,
+                                                   const unsigned* __restrict__ gate) {
+    if (closed(gate)) return;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
         const float4 r = tmp[s];
         int c;
@@ -415,9 +408,18 @@ __global__ void __launch_bounds__(1024) k_large_sort(float4* __restrict__ tmp, c
     }
 }
 
+// Zeroes counts behind the gate.
+__global__ void __launch_bounds__(256) k_zero(int* __restrict__ v, long long n, const unsigned* __restrict__ gate) {
+    if (closed(gate)) return;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        v[i] = 0;
+}
+
 // ---------------------------------------------------------------- descriptors / candidates
 __global__ void __launch_bounds__(256) k_descriptors(const int* __restrict__ offsets, long long ncells,
-                                                     lj_cell_desc* __restrict__ cells) {
+                                                     lj_cell_desc* __restrict__ cells,
+                                                     const unsigned* __restrict__ gate = nullptr) {
+    if (closed(gate)) return;
     for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < ncells;
          c += (long long)gridDim.x * blockDim.x) {
         const int o0 = offsets[c], o1 = offsets[c + 1];
@@ -527,7 +529,7 @@ static lj_status check_grid(const lj_grid* g, long long* ncells) {
     return LJ_OK;
 }
 
-lj_status launch_scan(lj_ctx* ctx, const int* counts, long long ncells, int* offsets) {
+static lj_status scan_gated(lj_ctx* ctx, const int* counts, long long ncells, int* offsets, const unsigned* gate) {
     const long long ntiles = (ncells + kScanTile - 1) / kScanTile;
     const size_t need = 256 + (size_t)(ntiles > 0 ? ntiles : 1) * sizeof(unsigned long long);
     lj_status s = grow(&ctx->scan_state, &ctx->scan_state_bytes, need);
@@ -541,12 +543,16 @@ lj_status launch_scan(lj_ctx* ctx, const int* counts, long long ncells, int* off
     unsigned long long* states = reinterpret_cast<unsigned long long*>(static_cast<char*>(ctx->scan_state) + 256);
     const int vec_ok = ((reinterpret_cast<uintptr_t>(counts) | reinterpret_cast<uintptr_t>(offsets)) & 15) == 0;
     k_scan<<<(unsigned)ntiles, kScanThreads, 0, ctx->stream>>>(counts, offsets, ncells, ntiles, states, counter,
-                                                              vec_ok, ctx->d_status);
+                                                              vec_ok, ctx->d_status, gate);
 #ifdef LJ_CHECKS
     if ((s = last_launch_status()) != LJ_OK) return s;
     k_chk_scan<<<grid_for(ctx, ncells, 256), 256, 0, ctx->stream>>>(counts, offsets, ncells, ctx->d_status);
 #endif
     return last_launch_status();
+}
+
+lj_status launch_scan(lj_ctx* ctx, const int* counts, long long ncells, int* offsets) {
+    return scan_gated(ctx, counts, ncells, offsets, nullptr);
 }
 
 }  // namespace ljc
@@ -563,7 +569,7 @@ extern "C" lj_status lj_count_cells(lj_ctx* ctx, const lj_grid* g, int n, const 
     if (cudaMemsetAsync(counts, 0, sizeof(int) * (size_t)nc, ctx->stream) != cudaSuccess) return LJ_ECUDA;
     if (n == 0) return LJ_OK;
     k_count<false><<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(to_dev(*g), x, y, z, stride, n, counts, nullptr,
-                                                                  ctx->d_status);
+                                                                  ctx->d_status, nullptr);
     return last_launch_status();
 }
 
@@ -583,8 +589,8 @@ extern "C" lj_status lj_cell_descriptors(lj_ctx* ctx, const int* offsets, long l
 
 namespace ljc {
 
-// Stage 1 of a cell-grid build: scratch for n particles, counts zeroed.
-lj_status bin_prepare(lj_ctx* ctx, int n, long long nc, int* counts) {
+// Scratch of a cell-grid build of n particles.
+static lj_status bin_scratch(lj_ctx* ctx, int n) {
     lj_status s;
     const size_t need = (size_t)(n > 0 ? n : 1);
     if (need > ctx->part_cap) {
@@ -614,9 +620,88 @@ lj_status bin_prepare(lj_ctx* ctx, int n, long long nc, int* counts) {
         ctx->large_cap = s == LJ_OK ? large_need : 0;
         if (s != LJ_OK) return s;
     }
+    return LJ_OK;
+}
+
+// Stage 1 of a cell-grid build: scratch for n particles, counts zeroed.
+lj_status bin_prepare(lj_ctx* ctx, int n, long long nc, int* counts) {
+    const lj_status s = bin_scratch(ctx, n);
+    if (s != LJ_OK) return s;
     if (cudaMemsetAsync(counts, 0, sizeof(int) * (size_t)nc, ctx->stream) != cudaSuccess) return LJ_ECUDA;
     if (cudaMemsetAsync(ctx->large_cells, 0, sizeof(int), ctx->stream) != cudaSuccess) return LJ_ECUDA;
     return LJ_OK;
+}
+
+#ifdef LJ_CHECKS
+// The sorted records' checks (not while a graph is being captured: they need scratch).
+static lj_status check_sorted(lj_ctx* ctx, long long nc, int n, lj_order order, const float* sorted_xyzi,
+                              const int* sorted_cell, const int* offsets, const GridDev& g, bool recompute) {
+    cudaStream_t st = ctx->stream;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) return LJ_ECUDA;
+    if (n == 0 || capturing != cudaStreamCaptureStatusNone) return LJ_OK;
+    lj_status s;
+    if ((s = grow(&ctx->check, &ctx->check_bytes, (size_t)n * sizeof(int))) != LJ_OK) return s;
+    int* seen = static_cast<int*>(ctx->check);
+    if (cudaMemsetAsync(seen, 0, (size_t)n * sizeof(int), st) != cudaSuccess) return LJ_ECUDA;
+    const float4* x4 = reinterpret_cast<const float4*>(sorted_xyzi);
+    if (order == LJ_ORDER_X)
+        k_chk_sorted<LJ_ORDER_X><<<grid_for(ctx, n, 256), 256, 0, st>>>(g, recompute, x4, sorted_cell, offsets, n, nc,
+                                                                        seen, ctx->d_status);
+    else
+        k_chk_sorted<LJ_ORDER_INDEX><<<grid_for(ctx, n, 256), 256, 0, st>>>(g, recompute, x4, sorted_cell, offsets, n,
+                                                                            nc, seen, ctx->d_status);
+    if ((s = last_launch_status()) != LJ_OK) return s;
+    k_chk_seen<<<grid_for(ctx, n, 256), 256, 0, st>>>(seen, n, ctx->d_status);
+    return last_launch_status();
+}
+#endif
+
+// The ticket path after its count kernel: scan, scatter, within-cell sort.  With a gate the kernels do
+// nothing unless it is open, and the scatter takes one pass.
+static lj_status ticket_finish(lj_ctx* ctx, long long nc, int n, const float* x, const float* y, const float* z,
+                               int stride, lj_order order, int* counts, int* offsets, const SortOut& so,
+                               const GridDev& g, const BinSys* sys, const int* firsts, int nsys,
+                               const unsigned* gate) {
+    lj_status s;
+    cudaStream_t st = ctx->stream;
+    if ((s = scan_gated(ctx, counts, nc, offsets, gate)) != LJ_OK) return s;
+    if (n == 0) return LJ_OK;
+#ifdef LJ_CHECKS
+    if (!gate) {
+        k_chk_tickets<<<grid_for(ctx, n, 256), 256, 0, st>>>(ctx->cell_ticket, counts, n, nc, ctx->d_status);
+        if ((s = last_launch_status()) != LJ_OK) return s;
+    }
+#endif
+    // passes: the tuning's scatter_passes, else enough that each pass writes about kScatterRegion bytes
+    long long passes = gate ? 1 : ctx->tuning.scatter_passes;
+    if (passes <= 0) passes = ((long long)n * (long long)sizeof(float4) + kScatterRegion - 1) / kScatterRegion;
+    passes = std::max(1LL, std::min(passes, std::min(8LL, nc)));
+    for (long long q = 0; q < passes; ++q) {
+        const int c_lo = (int)(nc * q / passes), c_hi = (int)(nc * (q + 1) / passes);
+        k_scatter<<<grid_for(ctx, n, 256), 256, 0, st>>>(x, y, z, stride, n, ctx->cell_ticket, offsets, ctx->tmp4,
+                                                         ctx->d_status, c_lo, c_hi, gate);
+        if ((s = last_launch_status()) != LJ_OK) return s;
+    }
+    const int lcap = (int)ctx->large_cap;
+    const auto rank = order == LJ_ORDER_X ? k_cell_rank<LJ_ORDER_X> : k_cell_rank<LJ_ORDER_INDEX>;
+    rank<<<grid_for(ctx, n, 256), 256, 0, st>>>(ctx->tmp4, offsets, g, sys, firsts, nsys, n, so, ctx->large_cells,
+                                                lcap, ctx->d_status, gate);
+    if ((s = last_launch_status()) != LJ_OK) return s;
+    const auto sort = order == LJ_ORDER_X ? k_large_sort<LJ_ORDER_X> : k_large_sort<LJ_ORDER_INDEX>;
+    sort<<<ctx->sm_count, 1024, 0, st>>>(ctx->tmp4, offsets, n, so, ctx->large_cells, lcap);
+    return last_launch_status();
+}
+
+static SortOut sort_out(float* sorted_xyzi, int* sorted_cell, const lj_particles* sorted) {
+    SortOut so{reinterpret_cast<float4*>(sorted_xyzi), sorted_cell, nullptr, nullptr, nullptr, nullptr};
+    if (sorted) {
+        so.sx = sorted->x;
+        so.sy = sorted->y;
+        so.sz = sorted->z;
+        so.sidx = sorted->index;
+    }
+    return so;
 }
 
 // Stages after a count kernel has filled counts and ctx->cell_ticket: scan,
@@ -625,75 +710,48 @@ lj_status bin_finish(lj_ctx* ctx, long long nc, int n, const float* x, const flo
                      lj_order order, int* counts, int* offsets, lj_cell_desc* cells, lj_particles* sorted,
                      float* sorted_xyzi, int* sorted_cell, const GridDev& g, const BinSys* sys, const int* firsts,
                      int nsys) {
-    lj_status s;
-    cudaStream_t st = ctx->stream;
-    if ((s = launch_scan(ctx, counts, nc, offsets)) != LJ_OK) return s;
-#ifdef LJ_CHECKS
-    if (n > 0) {
-        k_chk_tickets<<<grid_for(ctx, n, 256), 256, 0, st>>>(ctx->cell_ticket, counts, n, nc, ctx->d_status);
-        if ((s = last_launch_status()) != LJ_OK) return s;
-    }
-#endif
-    if (n > 0) {
-        // passes: the tuning's scatter_passes, else enough that each pass writes about kScatterRegion bytes
-        long long passes = ctx->tuning.scatter_passes;
-        if (passes <= 0) passes = ((long long)n * (long long)sizeof(float4) + kScatterRegion - 1) / kScatterRegion;
-        passes = std::max(1LL, std::min(passes, std::min(8LL, nc)));
-        for (long long q = 0; q < passes; ++q) {
-            const int c_lo = (int)(nc * q / passes), c_hi = (int)(nc * (q + 1) / passes);
-            k_scatter<<<grid_for(ctx, n, 256), 256, 0, st>>>(x, y, z, stride, n, ctx->cell_ticket, offsets,
-                                                             ctx->tmp4, ctx->d_status, c_lo, c_hi);
-            if ((s = last_launch_status()) != LJ_OK) return s;
-        }
-    }
-    SortOut so{reinterpret_cast<float4*>(sorted_xyzi), sorted_cell, nullptr, nullptr, nullptr, nullptr};
-    if (sorted) {
-        so.sx = sorted->x;
-        so.sy = sorted->y;
-        so.sz = sorted->z;
-        so.sidx = sorted->index;
-    }
-    const int lcap = (int)ctx->large_cap;
-    if (n > 0) {
-        if (order == LJ_ORDER_X) {
-            k_cell_rank<LJ_ORDER_X><<<grid_for(ctx, n, 256), 256, 0, st>>>(ctx->tmp4, offsets, g, sys, firsts, nsys, n,
-                                                                           so, ctx->large_cells, lcap, ctx->d_status);
-            if ((s = last_launch_status()) != LJ_OK) return s;
-            k_large_sort<LJ_ORDER_X><<<ctx->sm_count, 1024, 0, st>>>(ctx->tmp4, offsets, n, so, ctx->large_cells,
-                                                                     lcap);
-        } else {
-            k_cell_rank<LJ_ORDER_INDEX><<<grid_for(ctx, n, 256), 256, 0, st>>>(ctx->tmp4, offsets, g, sys, firsts, nsys,
-                                                                               n, so, ctx->large_cells, lcap,
-                                                                               ctx->d_status);
-            if ((s = last_launch_status()) != LJ_OK) return s;
-            k_large_sort<LJ_ORDER_INDEX><<<ctx->sm_count, 1024, 0, st>>>(ctx->tmp4, offsets, n, so,
-                                                                         ctx->large_cells, lcap);
-        }
-        if ((s = last_launch_status()) != LJ_OK) return s;
-    }
+    lj_status s = ticket_finish(ctx, nc, n, x, y, z, stride, order, counts, offsets,
+                                sort_out(sorted_xyzi, sorted_cell, sorted), g, sys, firsts, nsys, nullptr);
+    if (s != LJ_OK) return s;
     if (cells) {
-        k_descriptors<<<grid_for(ctx, nc, 256), 256, 0, st>>>(offsets, nc, cells);
+        k_descriptors<<<grid_for(ctx, nc, 256), 256, 0, ctx->stream>>>(offsets, nc, cells);
+        if ((s = last_launch_status()) != LJ_OK) return s;
     }
 #ifdef LJ_CHECKS
-    // the permutation check needs scratch, which cannot be allocated while a graph is being captured
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) return LJ_ECUDA;
-    if (n > 0 && capturing == cudaStreamCaptureStatusNone) {
-        if ((s = grow(&ctx->check, &ctx->check_bytes, (size_t)n * sizeof(int))) != LJ_OK) return s;
-        int* seen = static_cast<int*>(ctx->check);
-        if (cudaMemsetAsync(seen, 0, (size_t)n * sizeof(int), st) != cudaSuccess) return LJ_ECUDA;
-        const float4* x4 = reinterpret_cast<const float4*>(sorted_xyzi);
-        if (order == LJ_ORDER_X)
-            k_chk_sorted<LJ_ORDER_X><<<grid_for(ctx, n, 256), 256, 0, st>>>(g, sys == nullptr, x4, sorted_cell, offsets,
-                                                                            n, nc, seen, ctx->d_status);
-        else
-            k_chk_sorted<LJ_ORDER_INDEX><<<grid_for(ctx, n, 256), 256, 0, st>>>(g, sys == nullptr, x4, sorted_cell,
-                                                                                offsets, n, nc, seen, ctx->d_status);
-        if ((s = last_launch_status()) != LJ_OK) return s;
-        k_chk_seen<<<grid_for(ctx, n, 256), 256, 0, st>>>(seen, n, ctx->d_status);
-    }
+    if ((s = check_sorted(ctx, nc, n, order, sorted_xyzi, sorted_cell, offsets, g, sys == nullptr)) != LJ_OK) return s;
 #endif
-    return last_launch_status();
+    return LJ_OK;
+}
+
+// The segment path, with the ticket path behind its gate for particles crowded into few segments.
+static lj_status bin_segments(lj_ctx* ctx, const SegPlan& plan, long long nc, int n, const float* x, const float* y,
+                              const float* z, int stride, lj_order order, int* counts, int* offsets,
+                              lj_cell_desc* cells, lj_particles* sorted, float* sorted_xyzi, int* sorted_cell,
+                              const GridDev& g) {
+    lj_status s = bin_scratch(ctx, n);
+    if (s != LJ_OK) return s;
+    const SortOut so = sort_out(sorted_xyzi, sorted_cell, sorted);
+    const unsigned* gate = nullptr;
+    if ((s = launch_segment_bin(ctx, plan, nc, n, x, y, z, stride, order, counts, offsets, cells, so, g, &gate)) != LJ_OK)
+        return s;
+    cudaStream_t st = ctx->stream;
+    if (cudaMemsetAsync(ctx->large_cells, 0, sizeof(int), st) != cudaSuccess) return LJ_ECUDA;
+    k_zero<<<grid_for(ctx, nc, 256), 256, 0, st>>>(counts, nc, gate);
+    if ((s = last_launch_status()) != LJ_OK) return s;
+    k_count<true><<<grid_for(ctx, n, 256), 256, 0, st>>>(g, x, y, z, stride, n, counts, ctx->cell_ticket, ctx->d_status,
+                                                         gate);
+    if ((s = last_launch_status()) != LJ_OK) return s;
+    if ((s = ticket_finish(ctx, nc, n, x, y, z, stride, order, counts, offsets, so, g, nullptr, nullptr, 0, gate)) !=
+        LJ_OK)
+        return s;
+    if (cells) {
+        k_descriptors<<<grid_for(ctx, nc, 256), 256, 0, st>>>(offsets, nc, cells, gate);
+        if ((s = last_launch_status()) != LJ_OK) return s;
+    }
+#ifdef LJ_CHECKS
+    if ((s = check_sorted(ctx, nc, n, order, sorted_xyzi, sorted_cell, offsets, g, true)) != LJ_OK) return s;
+#endif
+    return LJ_OK;
 }
 
 }  // namespace ljc
@@ -709,10 +767,14 @@ extern "C" lj_status lj_bin(lj_ctx* ctx, const lj_grid* g, int n, const float* x
     if (s != LJ_OK) return s;
     if (n > 0 && (!x || !y || !z || !sorted_xyzi || !sorted_cell)) return LJ_EINVAL;
     if (reinterpret_cast<uintptr_t>(sorted_xyzi) & 15) return LJ_EINVAL;
+    const SegPlan plan = segment_plan(ctx, n, nc);
+    if (plan.nseg)
+        return bin_segments(ctx, plan, nc, n, x, y, z, stride, order, counts, offsets, cells, sorted, sorted_xyzi,
+                            sorted_cell, to_dev(*g));
     if ((s = bin_prepare(ctx, n, nc, counts)) != LJ_OK) return s;
     if (n > 0) {
         k_count<true><<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(to_dev(*g), x, y, z, stride, n, counts,
-                                                                      ctx->cell_ticket, ctx->d_status);
+                                                                      ctx->cell_ticket, ctx->d_status, nullptr);
         if ((s = last_launch_status()) != LJ_OK) return s;
     }
     return bin_finish(ctx, nc, n, x, y, z, stride, order, counts, offsets, cells, sorted, sorted_xyzi, sorted_cell,
