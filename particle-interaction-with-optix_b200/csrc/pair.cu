@@ -1,6 +1,7 @@
 // pair.cu -- the interaction stage on the device.
 //
-// k_pair_compat replaces ComputeParticleInterationsParPartNoLoop
+// k_pair_compat (and k_compat_cells in pair_compat.cu, on filled grids) replaces
+// ComputeParticleInterationsParPartNoLoop
 // (cudaLJ.cu:299-341) with the reference's law and stencil: every particle of
 // the clamped 27-cell block except itself, r = sqrt(d.d + 1e-5),
 // 4 eps ((1/r)^12 - (1/r)^6) with eps = sigma = 1, no cutoff; 1/r from the
@@ -24,6 +25,14 @@ namespace ljc {
 
 constexpr double kClusterCell = 6.0;  // particles per cell from which the default takes the cluster walk
 constexpr double kPairCell = 2.0;     // ... and below that, two targets per lane
+
+// Particles per cell from which the reference law takes a warp per cell (pair_compat.cu) instead of two
+// targets per lane.  Measured, 2M uniform particles, two targets per lane -> warp per cell: 485 -> 348 us
+// at 8 per cell, 764 -> 437 at 16, 2495 -> 1463 at 64, but 291 -> 494 at 4 (the warps of thin cells spend
+// their time on the stencil's offsets).  Grids whose cells all run at once take it at any density: 10,000
+// particles at 4 per cell 45 -> 10 us, 1,000 at 8 per cell 49 -> 9.
+constexpr double kCompatCell = 6.0;
+constexpr int kCompatWarpsPerSm = 32;
 
 // Default pair kernel (measured on B200, pair stage, 2M uniform particles): the cluster walk (1) from
 // 6 particles per cell up (484 against 514 us for kernel 10 at 10 per cell, 401 against 367 at 5), the
@@ -317,6 +326,9 @@ extern "C" lj_status lj_compute_compat(lj_ctx* ctx, const lj_grid* g, int n, con
     if (!(g->width > 0.0f) || g->dim[0] < 1 || g->dim[1] < 1 || g->dim[2] < 1) return LJ_EINVAL;
     if (reinterpret_cast<uintptr_t>(sorted_xyzi) & 15) return LJ_EINVAL;
     if (n == 0) return LJ_OK;
+    const double nc = (double)g->dim[0] * g->dim[1] * g->dim[2];
+    if (n >= kCompatCell * nc || nc <= (double)ctx->sm_count * kCompatWarpsPerSm)
+        return launch_compat_cells(ctx, g, n, sorted_xyzi, offsets, v);
     k_pair_compat<<<(n + 2 * kPairThreads - 1) / (2 * kPairThreads), kPairThreads, 0, ctx->stream>>>(
         to_dev(*g), reinterpret_cast<const float4*>(sorted_xyzi), sorted_cell, offsets, n, v, ctx->d_status);
     return last_launch_status();

@@ -255,6 +255,8 @@ lj_status launch_pair_cellpair(lj_ctx* ctx, const lj_grid* g, const PairParams& 
 lj_status launch_pair_cluster(lj_ctx* ctx, const lj_grid* g, const PairParams& pp, int n, const float* xyzi,
                               const int* cs, const int* off, bool xwin, float* energy, float* force,
                               lj_totals* totals, int kb, int ke);
+// Reference law, one warp per cell (pair_compat.cu).
+lj_status launch_compat_cells(lj_ctx* ctx, const lj_grid* g, int n, const float* xyzi, const int* off, float* v);
 // Exclusive scan of counts[ncells] into offsets[0..ncells] on the context's stream (bin.cu).
 lj_status launch_scan(lj_ctx* ctx, const int* counts, long long ncells, int* offsets);
 }  // namespace ljc
