@@ -767,6 +767,17 @@ extern "C" lj_status lj_bin(lj_ctx* ctx, const lj_grid* g, int n, const float* x
     if (s != LJ_OK) return s;
     if (n > 0 && (!x || !y || !z || !sorted_xyzi || !sorted_cell)) return LJ_EINVAL;
     if (reinterpret_cast<uintptr_t>(sorted_xyzi) & 15) return LJ_EINVAL;
+    if (small_bin_takes(ctx, n, nc)) {
+        s = launch_small_bin(ctx, nc, n, x, y, z, stride, order, counts, offsets, cells,
+                             sort_out(sorted_xyzi, sorted_cell, sorted), to_dev(*g));
+#ifdef LJ_CHECKS
+        if (s != LJ_OK) return s;
+        k_chk_scan<<<grid_for(ctx, nc, 256), 256, 0, ctx->stream>>>(counts, offsets, nc, ctx->d_status);
+        if ((s = last_launch_status()) != LJ_OK) return s;
+        s = check_sorted(ctx, nc, n, order, sorted_xyzi, sorted_cell, offsets, to_dev(*g), true);
+#endif
+        return s;
+    }
     const SegPlan plan = segment_plan(ctx, n, nc);
     if (plan.nseg)
         return bin_segments(ctx, plan, nc, n, x, y, z, stride, order, counts, offsets, cells, sorted, sorted_xyzi,

@@ -34,6 +34,7 @@ constexpr int kSegAim = 768;            // particles per segment to aim for (up 
 constexpr int kSegThreads = 1024;       // count and scatter
 constexpr int kSegSmall = 2048;         // records of a segment in the small sort kernel ...
 constexpr int kSegLarge = 10240;        // ... and in the large one; a segment above opens the gate
+constexpr int kSmallParticles = 4096;  // a system that one block bins (of at most kSegCells cells)
 constexpr int kSegMinParticles = 4000000;
 constexpr long long kSegRegion = 56LL << 20;  // bytes of records one scatter pass writes (L2 holds 126 MB)
 
@@ -224,10 +225,11 @@ __device__ __forceinline__ float x_of_key(unsigned k) {
     return __uint_as_float(k ^ ((unsigned)((int)~k >> 31) | 0x80000000u));
 }
 
-// One segment: its m records (at most CAP) at tmp + s0, its W cells from c0 on.  The records are read
-// twice (the second time from L2) rather than held in registers, which would halve the blocks per SM.
-template <int ORDER, int THREADS, int CAP>
-__device__ __forceinline__ void seg_sort(const GridDev& g, int c0, int W, int s0, int m, const float4* __restrict__ tmp,
+// One segment: its m records (at most CAP), load(i) the i-th, sorted to s0 on; its W cells from c0 on.
+// The records are read twice (the second time from L2) rather than held in registers, which would halve
+// the blocks per SM.
+template <int ORDER, int THREADS, int CAP, class Load>
+__device__ __forceinline__ void seg_sort(const GridDev& g, int c0, int W, int s0, int m, Load load,
                                          int* __restrict__ counts, int* __restrict__ offsets, bool vec,
                                          lj_cell_desc* __restrict__ cells, const SortOut& so, const float* __restrict__ x, int stride,
                                          uint4* s_rec, int* s_cnt,
@@ -258,7 +260,7 @@ __device__ __forceinline__ void seg_sort(const GridDev& g, int c0, int W, int s0
 #pragma unroll
     for (int u = 0; u < PER; ++u)
         if (u * THREADS + tid < m) {
-            const float4 r = __ldcg(&tmp[s0 + u * THREADS + tid]);
+            const float4 r = load(u * THREADS + tid);
             const int c = min(max(cell_of(g, r.x, r.y, r.z) - c0, 0), W - 1);
             where[u] = (c << 16) | atomicAdd(&s_cnt[c], 1);
         }
@@ -319,7 +321,7 @@ __device__ __forceinline__ void seg_sort(const GridDev& g, int c0, int W, int s0
     for (int u = 0; u < PER; ++u)
         if (u * THREADS + tid < m) {
             const int c = where[u] >> 16, at = s_cnt[c] + (where[u] & 0xffff);
-            const float4 r = __ldcg(&tmp[s0 + u * THREADS + tid]);
+            const float4 r = load(u * THREADS + tid);
             s_rec[at] = make_uint4(__float_as_uint(r.y), __float_as_uint(r.z), __float_as_uint(r.w), x_key(r.x));
             s_cell[at] = (unsigned short)c;
         }
@@ -370,9 +372,53 @@ __global__ void __launch_bounds__(THREADS, SMALL ? 6 : 1) k_seg_sort(GridDev g, 
         const int s0 = sc.start[b], m = sc.start[b + 1] - s0;
         if (m < 0 || m > CAP || s0 < 0 || s0 + m > n) continue;
         const int c0 = b << shift, W = min(1 << shift, ncell - c0);
-        seg_sort<ORDER, THREADS, CAP>(g, c0, W, s0, m, tmp, counts, offsets, vec != 0, cells, so, x, stride, s_rec, s_cnt, s_cell);
+        seg_sort<ORDER, THREADS, CAP>(g, c0, W, s0, m, [&](int i) { return __ldcg(&tmp[s0 + i]); }, counts, offsets, vec != 0, cells, so, x, stride, s_rec, s_cnt, s_cell);
         if (!SMALL) __syncthreads();
     }
+}
+
+// A whole small system as one segment: one launch instead of the ticket path's six kernels and three
+// memsets, which its smallest systems spend their time on.
+template <int ORDER>
+__global__ void __launch_bounds__(kSegThreads) k_bin_small(GridDev g, int ncell, const float* __restrict__ x,
+                                                           const float* __restrict__ y, const float* __restrict__ z,
+                                                           int stride, int n, int* __restrict__ counts,
+                                                           int* __restrict__ offsets, int vec,
+                                                           lj_cell_desc* __restrict__ cells, SortOut so,
+                                                           unsigned* status) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    uint4* s_rec = reinterpret_cast<uint4*>(s_raw);
+    unsigned short* s_cell = reinterpret_cast<unsigned short*>(s_raw + (size_t)kSmallParticles * 16);
+    int* s_cnt = reinterpret_cast<int*>(s_raw + (size_t)kSmallParticles * 18);
+    if (threadIdx.x == 0) offsets[ncell] = n;
+    bool bad = false;
+    seg_sort<ORDER, kSegThreads, kSmallParticles>(
+        g, 0, ncell, 0, n,
+        [&](int i) {
+            const float4 r = make_float4(__ldg(&x[(long long)i * stride]), __ldg(&y[(long long)i * stride]),
+                                         __ldg(&z[(long long)i * stride]), __int_as_float(i));
+            bad |= !(isfinite(r.x) && isfinite(r.y) && isfinite(r.z));
+            return r;
+        },
+        counts, offsets, vec != 0, cells, so, x, stride, s_rec, s_cnt, s_cell);
+    if (bad) atomicOr(status, kFlagNonFinite);
+}
+
+bool small_bin_takes(const lj_ctx* ctx, int n, long long nc) {
+    return n >= 1 && n <= kSmallParticles && nc <= kSegCells && ctx->tuning.scatter_passes == 0;
+}
+
+lj_status launch_small_bin(lj_ctx* ctx, long long nc, int n, const float* x, const float* y, const float* z, int stride,
+                           lj_order order, int* counts, int* offsets, lj_cell_desc* cells, const SortOut& so,
+                           const GridDev& g) {
+    const auto kernel = order == LJ_ORDER_X ? k_bin_small<LJ_ORDER_X> : k_bin_small<LJ_ORDER_INDEX>;
+    const size_t bytes = (size_t)kSmallParticles * 18 + (((size_t)nc * sizeof(int) + 15) & ~(size_t)15);
+    const int vec = ((reinterpret_cast<uintptr_t>(counts) | reinterpret_cast<uintptr_t>(offsets)) & 15) == 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
+        return LJ_ECUDA;
+    kernel<<<1, kSegThreads, bytes, ctx->stream>>>(g, (int)nc, x, y, z, stride, n, counts, offsets, vec, cells, so,
+                                                   ctx->d_status);
+    return last_launch_status();
 }
 
 // Segments of a power of two of cells, kSegAim to twice as many particles on average.  Taken from

@@ -1,7 +1,7 @@
 """The binning by segments of cells (large systems) against the oracle, bit for bit: the smallest size
 that takes it, ragged sizes and grids (a last segment of a few cells), both orders, point3d input with
 every optional output, segments for the large sort kernel, particles crowded into few segments (the
-ticket kernels behind the gate), nearly sorted input and points outside the box."""
+ticket kernels behind the gate), nearly sorted input and points outside the box; and the binning of small systems by one block."""
 import numpy as np
 import pytest
 
@@ -92,3 +92,37 @@ def test_segment_binning_reports_a_non_finite_position(torch_cuda, ctx):
         ctx.sync()
     assert ei.value.status == ljcell.LJ_ERANGE
     ctx.sync()
+
+
+@pytest.mark.parametrize("order", [0, 1])
+@pytest.mark.parametrize("n,box,rc", [(1, 1.0, 0.25), (31, 1.0, 0.25), (1000, 1.0, 0.25), (1025, 1.0, 0.3), (4095, 1.0, 0.05),
+                                      (4096, 1.0, 0.0501), (4097, 1.0, 0.05), (3000, 1.0, 0.0496), (777, 1.0, 1.0),
+                                      (4096, 0.1, 0.05), (2000, 3.0, 0.151)])
+def test_small_system_binning_bit_exact(torch_cuda, ctx, n, box, rc, order):
+    """One block bins systems of up to 4096 particles and 8192 cells: both sides of its limits, cell
+    counts that are no multiple of four, all particles in one cell, particles beyond the box, and equal x
+    (-0 among them)."""
+    import ljcell
+
+    torch = torch_cuda
+    p = uniform(n, n + order) * np.float32(box)
+    p[::7, 0] = np.float32(0.0)
+    p[::14, 0] = np.float32(-0.0)
+    p[::5, 1] -= np.float32(0.1)
+    x, y, z = (np.ascontiguousarray(p[:, k]) for k in range(3))
+    g, og = ljcell.grid_from_box(*UNIT, rc), O.grid_from_box(*UNIT, rc)
+    ob = O.bin_particles(og, x, y, z, order)
+    aos = dev(torch, p.reshape(-1))
+    for stride in (1, 3):
+        d = (aos, aos[1:], aos[2:]) if stride == 3 else tuple(dev(torch, a) for a in (x, y, z))
+        b = ctx.bin(g, *d, stride=stride, order=order, soa=stride == 3, cells=stride == 3)
+        ctx.sync()
+        np.testing.assert_array_equal(np_(b.counts), ob.counts)
+        np.testing.assert_array_equal(np_(b.offsets), ob.offsets)
+        r = np_(b.xyzi)[:n]
+        np.testing.assert_array_equal(r[:, 3].view(np.int32), ob.perm)
+        np.testing.assert_array_equal(r[:, :3].view(np.int32), p[ob.perm].view(np.int32))
+        np.testing.assert_array_equal(np_(b.cell)[:n], ob.cell_sorted)
+        if stride == 3:
+            np.testing.assert_array_equal(np_(b.cells), np.stack([ob.counts, ob.offsets[:-1]], 1))
+            np.testing.assert_array_equal(np_(b.index)[:n], ob.perm)
