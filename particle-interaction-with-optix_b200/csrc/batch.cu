@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(BLOCK, MODE == 2 ? kCluWarpsPerSm * 32 / BLOCK
             __shared__ __align__(16) CluSmem sm[BLOCK / 32];
             const int w = (int)(threadIdx.x >> 5);
             cluster_stretch<true>(S.g, S.pp, ps, cs + S.first, S.cell_base, off + S.cell_base, S.first, S.n,
-                                  d.y - S.first, d.z - S.first, 0, S.n, w, BLOCK / 32, sm[w], status,
+                                  d.y - S.first, d.z - S.first, 0, S.n, w, BLOCK / 32, -1, sm[w], status,
                                   [&](int k, int s, bool valid, float v, float wv, unsigned np, int) {
                                       wv += __shfl_xor_sync(0xffffffffu, wv, 16);
                                       wv += __shfl_xor_sync(0xffffffffu, wv, 8);

@@ -120,7 +120,8 @@ __device__ __forceinline__ void clu_walk(const CluSmem& sm, int cnt, int s, floa
 }
 
 // Evaluates the groups that start in [a, b), one warp (all 32 lanes must call): of consecutive groups
-// every turns-th from the turn-th on, so that a block's warps share their candidates in L1.  p, cs, off:
+// every turns-th from the turn-th on, so that a block's warps share their candidates in L1; of a group
+// both clusters, or (only >= 0) the only-th.  p, cs, off:
 // the system's sorted records, cell ids (minus cbase) and offsets (minus obase); n particles; groups
 // without a target of [kb, ke) are skipped.  emit(k, s, valid, v, w, np, id) is called by all
 // lanes for each cluster: valid: k is a target of the lane; v: the target's sum of s^12 - s^6 in lane
@@ -130,7 +131,7 @@ template <bool XWIN, class Emit>
 __device__ __forceinline__ void cluster_stretch(const GridDev& g, const PairParams& pp, const float4* __restrict__ p,
                                                 const int* __restrict__ cs, int cbase, const int* __restrict__ off,
                                                 int obase, int n, int a, int b, int kb, int ke, int turn, int turns,
-                                                CluSmem& sm, unsigned* status, Emit emit) {
+                                                int only, CluSmem& sm, unsigned* status, Emit emit) {
     const int lane = (int)(threadIdx.x & 31u), t = lane & 7, s = lane >> 3;
     const unsigned below = lanemask_lt();
     const int ncell = g.gx * g.gy * g.gz;
@@ -233,7 +234,7 @@ __device__ __forceinline__ void cluster_stretch(const GridDev& g, const PairPara
         }
         const int4 rng = lane < nr ? sm.range[lane] : make_int4(INT_MAX, 0, 0, 0);
         __syncwarp();
-        for (int cl = gs; cl < ge; cl += kCluTargets) {
+        for (int cl = only < 0 ? gs : gs + only * kCluTargets; cl < ge; cl += only < 0 ? kCluTargets : kCluGroup) {
             const int nt = min(kCluTargets, ge - cl);
             const int k = cl + min(t, nt - 1);  // lanes past the end repeat the last target
             const float4 pi = __ldg(&p[k]);
