@@ -34,6 +34,8 @@ __global__ void __launch_bounds__(256) k_count(GridDev g, const float* __restric
                                                const float* __restrict__ z, int stride, int n,
                                                int* __restrict__ counts, int2* __restrict__ ct,
                                                unsigned* status, const unsigned* __restrict__ gate) {
+    chain_wait();
+    chain_next();
     if (closed(gate)) return;
     const int lane = threadIdx.x & 31;
     const long long gwarp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -85,6 +87,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const int* __restrict__ c
                                                        unsigned long long* tile_state, unsigned* tile_counter,
                                                        int vec_ok, unsigned* status,
                                                        const unsigned* __restrict__ gate = nullptr) {
+    chain_wait();
+    chain_next();
     if (closed(gate)) return;
     __shared__ unsigned s_tile;
     __shared__ long long s_warp[8];
@@ -222,6 +226,8 @@ __global__ void __launch_bounds__(256) k_scatter(const float* __restrict__ x, co
                                                  const int2* __restrict__ ct, const int* __restrict__ offsets,
                                                  float4* __restrict__ tmp, unsigned* status, int c_lo, int c_hi,
                                                  const unsigned* __restrict__ gate = nullptr) {
+    chain_wait();
+    chain_next();
     if (closed(gate)) return;
     constexpr int U = 4;
     const long long step = (long long)gridDim.x * blockDim.x;
@@ -283,6 +289,8 @@ __global__ void __launch_bounds__(256) k_cell_rank(const float4* __restrict__ tm
                                                    const int* __restrict__ firsts, int nsys, int n, SortOut so,
                                                    int* large, int large_cap, unsigned* status,
                                                    const unsigned* __restrict__ gate) {
+    chain_wait();
+    chain_next();
     if (closed(gate)) return;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
         const float4 r = tmp[s];
@@ -344,6 +352,8 @@ template <int ORDER>
 __global__ void __launch_bounds__(1024) k_large_sort(float4* __restrict__ tmp, const int* __restrict__ offsets,
                                                      int n, SortOut so, const int* __restrict__ large,
                                                      int large_cap) {
+    chain_wait();
+    chain_next();
     __shared__ float4 sbuf[2048];
     const int count = min(large[0], large_cap);
     const int tid = threadIdx.x;
@@ -410,6 +420,8 @@ __global__ void __launch_bounds__(1024) k_large_sort(float4* __restrict__ tmp, c
 
 // Zeroes counts behind the gate.
 __global__ void __launch_bounds__(256) k_zero(int* __restrict__ v, long long n, const unsigned* __restrict__ gate) {
+    chain_wait();
+    chain_next();
     if (closed(gate)) return;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         v[i] = 0;
@@ -419,6 +431,8 @@ __global__ void __launch_bounds__(256) k_zero(int* __restrict__ v, long long n, 
 __global__ void __launch_bounds__(256) k_descriptors(const int* __restrict__ offsets, long long ncells,
                                                      lj_cell_desc* __restrict__ cells,
                                                      const unsigned* __restrict__ gate = nullptr) {
+    chain_wait();
+    chain_next();
     if (closed(gate)) return;
     for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < ncells;
          c += (long long)gridDim.x * blockDim.x) {
@@ -529,21 +543,28 @@ static lj_status check_grid(const lj_grid* g, long long* ncells) {
     return LJ_OK;
 }
 
-static lj_status scan_gated(lj_ctx* ctx, const int* counts, long long ncells, int* offsets, const unsigned* gate) {
+// The scan's look-back state for ncells counts, zeroed.
+lj_status scan_prepare(lj_ctx* ctx, long long ncells) {
     const long long ntiles = (ncells + kScanTile - 1) / kScanTile;
     const size_t need = 256 + (size_t)(ntiles > 0 ? ntiles : 1) * sizeof(unsigned long long);
-    lj_status s = grow(&ctx->scan_state, &ctx->scan_state_bytes, need);
+    const lj_status s = grow(&ctx->scan_state, &ctx->scan_state_bytes, need);
     if (s != LJ_OK) return s;
+    return cudaMemsetAsync(ctx->scan_state, 0, need, ctx->stream) == cudaSuccess ? LJ_OK : LJ_ECUDA;
+}
+
+// The scan after scan_prepare on the same stream.
+lj_status scan_prepared(lj_ctx* ctx, const int* counts, long long ncells, int* offsets, const unsigned* gate) {
+    const long long ntiles = (ncells + kScanTile - 1) / kScanTile;
+    lj_status s = LJ_OK;
     if (ncells == 0) {
         if (cudaMemsetAsync(offsets, 0, sizeof(int), ctx->stream) != cudaSuccess) return LJ_ECUDA;
         return LJ_OK;
     }
-    if (cudaMemsetAsync(ctx->scan_state, 0, need, ctx->stream) != cudaSuccess) return LJ_ECUDA;
     unsigned* counter = reinterpret_cast<unsigned*>(ctx->scan_state);
     unsigned long long* states = reinterpret_cast<unsigned long long*>(static_cast<char*>(ctx->scan_state) + 256);
     const int vec_ok = ((reinterpret_cast<uintptr_t>(counts) | reinterpret_cast<uintptr_t>(offsets)) & 15) == 0;
-    k_scan<<<(unsigned)ntiles, kScanThreads, 0, ctx->stream>>>(counts, offsets, ncells, ntiles, states, counter,
-                                                              vec_ok, ctx->d_status, gate);
+    chain_launch(k_scan, (unsigned)ntiles, kScanThreads, 0, ctx->stream, counts, offsets, ncells, ntiles, states, counter,
+                 vec_ok, ctx->d_status, gate);
 #ifdef LJ_CHECKS
     if ((s = last_launch_status()) != LJ_OK) return s;
     k_chk_scan<<<grid_for(ctx, ncells, 256), 256, 0, ctx->stream>>>(counts, offsets, ncells, ctx->d_status);
@@ -552,7 +573,8 @@ static lj_status scan_gated(lj_ctx* ctx, const int* counts, long long ncells, in
 }
 
 lj_status launch_scan(lj_ctx* ctx, const int* counts, long long ncells, int* offsets) {
-    return scan_gated(ctx, counts, ncells, offsets, nullptr);
+    const lj_status s = scan_prepare(ctx, ncells);
+    return s != LJ_OK ? s : scan_prepared(ctx, counts, ncells, offsets, nullptr);
 }
 
 }  // namespace ljc
@@ -623,10 +645,12 @@ static lj_status bin_scratch(lj_ctx* ctx, int n) {
     return LJ_OK;
 }
 
-// Stage 1 of a cell-grid build: scratch for n particles, counts zeroed.
+// Stage 1 of a cell-grid build: scratch for n particles, the scan's state, counts zeroed.  All memsets
+// of the build come here, so that its kernels follow one another.
 lj_status bin_prepare(lj_ctx* ctx, int n, long long nc, int* counts) {
-    const lj_status s = bin_scratch(ctx, n);
+    lj_status s = bin_scratch(ctx, n);
     if (s != LJ_OK) return s;
+    if ((s = scan_prepare(ctx, nc)) != LJ_OK) return s;
     if (cudaMemsetAsync(counts, 0, sizeof(int) * (size_t)nc, ctx->stream) != cudaSuccess) return LJ_ECUDA;
     if (cudaMemsetAsync(ctx->large_cells, 0, sizeof(int), ctx->stream) != cudaSuccess) return LJ_ECUDA;
     return LJ_OK;
@@ -665,7 +689,7 @@ static lj_status ticket_finish(lj_ctx* ctx, long long nc, int n, const float* x,
                                const unsigned* gate) {
     lj_status s;
     cudaStream_t st = ctx->stream;
-    if ((s = scan_gated(ctx, counts, nc, offsets, gate)) != LJ_OK) return s;
+    if ((s = scan_prepared(ctx, counts, nc, offsets, gate)) != LJ_OK) return s;
     if (n == 0) return LJ_OK;
 #ifdef LJ_CHECKS
     if (!gate) {
@@ -679,17 +703,17 @@ static lj_status ticket_finish(lj_ctx* ctx, long long nc, int n, const float* x,
     passes = std::max(1LL, std::min(passes, std::min(8LL, nc)));
     for (long long q = 0; q < passes; ++q) {
         const int c_lo = (int)(nc * q / passes), c_hi = (int)(nc * (q + 1) / passes);
-        k_scatter<<<grid_for(ctx, n, 256), 256, 0, st>>>(x, y, z, stride, n, ctx->cell_ticket, offsets, ctx->tmp4,
-                                                         ctx->d_status, c_lo, c_hi, gate);
+        chain_launch(k_scatter, grid_for(ctx, n, 256), 256, 0, st, x, y, z, stride, n, ctx->cell_ticket, offsets, ctx->tmp4,
+                     ctx->d_status, c_lo, c_hi, gate);
         if ((s = last_launch_status()) != LJ_OK) return s;
     }
     const int lcap = (int)ctx->large_cap;
     const auto rank = order == LJ_ORDER_X ? k_cell_rank<LJ_ORDER_X> : k_cell_rank<LJ_ORDER_INDEX>;
-    rank<<<grid_for(ctx, n, 256), 256, 0, st>>>(ctx->tmp4, offsets, g, sys, firsts, nsys, n, so, ctx->large_cells,
-                                                lcap, ctx->d_status, gate);
+    chain_launch(rank, grid_for(ctx, n, 256), 256, 0, st, ctx->tmp4, offsets, g, sys, firsts, nsys, n, so,
+                 ctx->large_cells, lcap, ctx->d_status, gate);
     if ((s = last_launch_status()) != LJ_OK) return s;
     const auto sort = order == LJ_ORDER_X ? k_large_sort<LJ_ORDER_X> : k_large_sort<LJ_ORDER_INDEX>;
-    sort<<<ctx->sm_count, 1024, 0, st>>>(ctx->tmp4, offsets, n, so, ctx->large_cells, lcap);
+    chain_launch(sort, ctx->sm_count, 1024, 0, st, ctx->tmp4, offsets, n, so, ctx->large_cells, lcap);
     return last_launch_status();
 }
 
@@ -714,7 +738,7 @@ lj_status bin_finish(lj_ctx* ctx, long long nc, int n, const float* x, const flo
                                 sort_out(sorted_xyzi, sorted_cell, sorted), g, sys, firsts, nsys, nullptr);
     if (s != LJ_OK) return s;
     if (cells) {
-        k_descriptors<<<grid_for(ctx, nc, 256), 256, 0, ctx->stream>>>(offsets, nc, cells);
+        chain_launch(k_descriptors, grid_for(ctx, nc, 256), 256, 0, ctx->stream, offsets, nc, cells, nullptr);
         if ((s = last_launch_status()) != LJ_OK) return s;
     }
 #ifdef LJ_CHECKS
@@ -732,20 +756,21 @@ static lj_status bin_segments(lj_ctx* ctx, const SegPlan& plan, long long nc, in
     if (s != LJ_OK) return s;
     const SortOut so = sort_out(sorted_xyzi, sorted_cell, sorted);
     const unsigned* gate = nullptr;
+    if ((s = scan_prepare(ctx, nc)) != LJ_OK) return s;
+    if (cudaMemsetAsync(ctx->large_cells, 0, sizeof(int), ctx->stream) != cudaSuccess) return LJ_ECUDA;
     if ((s = launch_segment_bin(ctx, plan, nc, n, x, y, z, stride, order, counts, offsets, cells, so, g, &gate)) != LJ_OK)
         return s;
     cudaStream_t st = ctx->stream;
-    if (cudaMemsetAsync(ctx->large_cells, 0, sizeof(int), st) != cudaSuccess) return LJ_ECUDA;
-    k_zero<<<grid_for(ctx, nc, 256), 256, 0, st>>>(counts, nc, gate);
+    chain_launch(k_zero, grid_for(ctx, nc, 256), 256, 0, st, counts, nc, gate);
     if ((s = last_launch_status()) != LJ_OK) return s;
-    k_count<true><<<grid_for(ctx, n, 256), 256, 0, st>>>(g, x, y, z, stride, n, counts, ctx->cell_ticket, ctx->d_status,
-                                                         gate);
+    chain_launch(k_count<true>, grid_for(ctx, n, 256), 256, 0, st, g, x, y, z, stride, n, counts, ctx->cell_ticket,
+                 ctx->d_status, gate);
     if ((s = last_launch_status()) != LJ_OK) return s;
     if ((s = ticket_finish(ctx, nc, n, x, y, z, stride, order, counts, offsets, so, g, nullptr, nullptr, 0, gate)) !=
         LJ_OK)
         return s;
     if (cells) {
-        k_descriptors<<<grid_for(ctx, nc, 256), 256, 0, st>>>(offsets, nc, cells, gate);
+        chain_launch(k_descriptors, grid_for(ctx, nc, 256), 256, 0, st, offsets, nc, cells, gate);
         if ((s = last_launch_status()) != LJ_OK) return s;
     }
 #ifdef LJ_CHECKS
@@ -1040,7 +1065,7 @@ extern "C" lj_status lj_reorder(lj_ctx* ctx, int n, float* points, float radius)
     const float4* p4 = reinterpret_cast<const float4*>(points);
     k_reorder_count<<<grid_for(ctx, n, 256), 256, 0, st>>>(p4, n, rk, counts, ctx->cell_ticket, ctx->d_status);
     if ((s = last_launch_status()) != LJ_OK) return s;
-    if ((s = launch_scan(ctx, counts, nkeys, offsets)) != LJ_OK) return s;
+    if ((s = scan_prepared(ctx, counts, nkeys, offsets, nullptr)) != LJ_OK) return s;
     k_scatter<<<grid_for(ctx, n, 256), 256, 0, st>>>(points, points + 1, points + 2, 4, n, ctx->cell_ticket, offsets,
                                                      ctx->tmp4, ctx->d_status, 0, INT_MAX);
     if ((s = last_launch_status()) != LJ_OK) return s;

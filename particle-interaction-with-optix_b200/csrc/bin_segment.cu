@@ -124,6 +124,7 @@ __global__ void __launch_bounds__(kSegThreads) k_seg_count(GridDev g, const floa
                                                            int stride, int n, int shift, int nseg, SegScratch sc,
                                                            unsigned* status) {
     extern __shared__ int s_hist[];
+    chain_next();
     for (int i = threadIdx.x; i < nseg; i += kSegThreads) s_hist[i] = 0;
     __syncthreads();
     const long long lo = (long long)n * blockIdx.x / gridDim.x, hi = (long long)n * (blockIdx.x + 1) / gridDim.x;
@@ -175,6 +176,8 @@ __global__ void __launch_bounds__(kSegThreads) k_seg_scatter(const float* __rest
                                                              float4* __restrict__ tmp, unsigned* status, int seg_lo,
                                                              int seg_hi) {
     extern __shared__ int s_next[];
+    chain_wait();
+    chain_next();
     if (sc.gate[0]) return;
     if (sc.gate[4]) {  // nearly sorted particles: the writes of all segments are in order anyway
         if (seg_lo > 0) return;
@@ -364,6 +367,8 @@ __global__ void __launch_bounds__(THREADS, SMALL ? 6 : 1) k_seg_sort(GridDev g, 
     uint4* s_rec = reinterpret_cast<uint4*>(s_raw);
     int* s_cnt = reinterpret_cast<int*>(s_raw + (size_t)CAP * 18);
     unsigned short* s_cell = reinterpret_cast<unsigned short*>(s_raw + (size_t)CAP * 16);
+    chain_wait();
+    chain_next();
     if (sc.gate[0]) return;
     if (SMALL && blockIdx.x == 0 && threadIdx.x == 0) offsets[ncell] = n;
     const int items = SMALL ? nseg : min((int)sc.gate[1], nseg);
@@ -450,11 +455,11 @@ static lj_status launch_seg_sorts(lj_ctx* ctx, const SegPlan& plan, long long nc
     if (cudaFuncSetAttribute(small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b_small) != cudaSuccess ||
         cudaFuncSetAttribute(large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b_large) != cudaSuccess)
         return LJ_ECUDA;
-    small<<<plan.nseg, 256, b_small, ctx->stream>>>(g, (int)nc, n, plan.shift, plan.nseg, sc, ctx->tmp4, counts, offsets,
+    chain_launch(small, plan.nseg, 256, b_small, ctx->stream, g, (int)nc, n, plan.shift, plan.nseg, sc, ctx->tmp4, counts, offsets,
                                                     vec, cells, so, x, stride);
     lj_status s;
     if ((s = last_launch_status()) != LJ_OK) return s;
-    large<<<std::min(ctx->sm_count, plan.nseg), 1024, b_large, ctx->stream>>>(g, (int)nc, n, plan.shift, plan.nseg, sc,
+    chain_launch(large, std::min(ctx->sm_count, plan.nseg), 1024, b_large, ctx->stream, g, (int)nc, n, plan.shift, plan.nseg, sc,
                                                                              ctx->tmp4, counts, offsets, vec, cells, so, x, stride);
     return last_launch_status();
 }
@@ -488,8 +493,8 @@ lj_status launch_segment_bin(lj_ctx* ctx, const SegPlan& plan, long long nc, int
     const long long passes = std::max(1LL, std::min(8LL, ((long long)n * 16 + kSegRegion - 1) / kSegRegion));
     for (long long q = 0; q < passes; ++q) {
         const int s_lo = (int)(plan.nseg * q / passes), s_hi = (int)(plan.nseg * (q + 1) / passes);
-        k_seg_scatter<<<blocks, kSegThreads, hist, st>>>(x, y, z, stride, n, plan.nseg, sc, ctx->tmp4,
-                                                         ctx->d_status, s_lo, s_hi);
+        chain_launch(k_seg_scatter, blocks, kSegThreads, hist, st, x, y, z, stride, n, plan.nseg, sc, ctx->tmp4,
+                     ctx->d_status, s_lo, s_hi);
         if ((s = last_launch_status()) != LJ_OK) return s;
     }
     return order == LJ_ORDER_X

@@ -156,6 +156,29 @@ struct lj_ctx {
 };
 
 namespace ljc {
+// Launch chaining inside one call's kernel sequence: a kernel launched with chain_launch may be scheduled
+// while its predecessor's last blocks still run; it calls chain_wait before its first access to memory
+// (which returns when every earlier grid it depends on has completed and its writes are visible), and
+// chain_next lets its own successor be scheduled in turn.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+inline void chain_launch(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
+                         A... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 // Blocks for a grid-stride loop over `items`: enough for every item, at most `waves` per SM.
 inline int grid_for(const lj_ctx* ctx, long long items, int per_block, int waves = 8) {
     long long b = (items + per_block - 1) / per_block;

@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(kPairThreads) k_pair_config(GridDev g, PairPar
                                                               Partial* part, unsigned* counter, lj_totals* totals,
                                                               unsigned* status) {
     __shared__ int2 s_win[kMaxWin][kPairThreads];
+    chain_wait();
     const int k = kb + blockIdx.x * kPairThreads + threadIdx.x;   // targets [kb, ke) of the n sorted particles
     float ea = 0.f, fx = 0.f, fy = 0.f, fz = 0.f, wa = 0.f;
     unsigned np = 0;
@@ -205,6 +206,7 @@ __global__ void __launch_bounds__(kPairThreads) k_pair_compat(GridDev g, const f
                                                               const int* __restrict__ cs,
                                                               const int* __restrict__ off, int n,
                                                               float* __restrict__ v, unsigned* status) {
+    chain_wait();
     const int ka = 2 * (blockIdx.x * kPairThreads + (int)threadIdx.x), kb = ka + 1;
     const bool activeA = ka < n, activeB = kb < n;
     const int ncell = g.gx * g.gy * g.gz;
@@ -310,8 +312,8 @@ lj_status launch_pair_config(lj_ctx* ctx, const lj_grid* g, const lj_params* prm
     unsigned* counter = static_cast<unsigned*>(ctx->red);
     Partial* part = reinterpret_cast<Partial*>(static_cast<char*>(ctx->red) + 256);
     const float4* p4 = reinterpret_cast<const float4*>(xyzi);
-    k_pair_config<<<blocks, kPairThreads, 0, ctx->stream>>>(to_dev(*g), pp, p4, cs, off, n, kb, ke, energy, force, part,
-                                                            counter, totals, ctx->d_status);
+    chain_launch(k_pair_config, blocks, kPairThreads, 0, ctx->stream, to_dev(*g), pp, p4, cs, off, n, kb, ke, energy,
+                 force, part, counter, totals, ctx->d_status);
     return last_launch_status();
 }
 
@@ -329,8 +331,8 @@ extern "C" lj_status lj_compute_compat(lj_ctx* ctx, const lj_grid* g, int n, con
     const double nc = (double)g->dim[0] * g->dim[1] * g->dim[2];
     if (n >= kCompatCell * nc || nc <= (double)ctx->sm_count * kCompatWarpsPerSm)
         return launch_compat_cells(ctx, g, n, sorted_xyzi, offsets, v);
-    k_pair_compat<<<(n + 2 * kPairThreads - 1) / (2 * kPairThreads), kPairThreads, 0, ctx->stream>>>(
-        to_dev(*g), reinterpret_cast<const float4*>(sorted_xyzi), sorted_cell, offsets, n, v, ctx->d_status);
+    chain_launch(k_pair_compat, (n + 2 * kPairThreads - 1) / (2 * kPairThreads), kPairThreads, 0, ctx->stream, to_dev(*g),
+                 reinterpret_cast<const float4*>(sorted_xyzi), sorted_cell, offsets, n, v, ctx->d_status);
     return last_launch_status();
 }
 

@@ -18,6 +18,8 @@ __global__ void __launch_bounds__(32 * kCluWarps, kCluWarpsPerSm / kCluWarps)
                    float* __restrict__ energy, float* __restrict__ force, Partial* part, unsigned* counter,
                    lj_totals* totals, unsigned* status) {
     __shared__ __align__(16) CluSmem sm[kCluWarps];
+    chain_wait();
+    chain_next();
     const int w = (int)(threadIdx.x >> 5);
     const long long first = a0 + (long long)blockIdx.x * stretch;
     double te = 0.0, tw = 0.0;
@@ -74,8 +76,8 @@ lj_status launch_pair_cluster(lj_ctx* ctx, const lj_grid* g, const PairParams& p
     const float4* p4 = reinterpret_cast<const float4*>(xyzi);
     const auto kernel = xwin ? (split ? k_pair_cluster<true, true> : k_pair_cluster<true, false>)
                              : (split ? k_pair_cluster<false, true> : k_pair_cluster<false, false>);
-    kernel<<<blocks, 32 * kCluWarps, 0, ctx->stream>>>(to_dev(*g), pp, p4, cs, off, n, kb, ke, a0, stretch, energy,
-                                                       force, part, counter, totals, ctx->d_status);
+    chain_launch(kernel, blocks, 32 * kCluWarps, 0, ctx->stream, to_dev(*g), pp, p4, cs, off, n, kb, ke, a0, stretch,
+                 energy, force, part, counter, totals, ctx->d_status);
     return last_launch_status();
 }
 

@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(32 * kCellWarps, 8) k_compat_cells(GridDev g, 
                                                                      const int* __restrict__ off, int n,
                                                                      float* __restrict__ v) {
     __shared__ __align__(16) CellSmem smem[kCellWarps];
+    chain_wait();
     CellSmem& sm = smem[threadIdx.x >> 5];
     const int lane = (int)(threadIdx.x & 31u), t = lane % kCellLanes, group = lane / kCellLanes;
     const unsigned below = lanemask_lt();
@@ -185,8 +186,8 @@ __global__ void __launch_bounds__(32 * kCellWarps, 8) k_compat_cells(GridDev g, 
 
 lj_status launch_compat_cells(lj_ctx* ctx, const lj_grid* g, int n, const float* xyzi, const int* off, float* v) {
     const long long nc = (long long)g->dim[0] * g->dim[1] * g->dim[2];
-    k_compat_cells<<<(unsigned)((nc + kCellWarps - 1) / kCellWarps), 32 * kCellWarps, 0, ctx->stream>>>(
-        to_dev(*g), reinterpret_cast<const float4*>(xyzi), off, n, v);
+    chain_launch(k_compat_cells, (unsigned)((nc + kCellWarps - 1) / kCellWarps), 32 * kCellWarps, 0, ctx->stream,
+                 to_dev(*g), reinterpret_cast<const float4*>(xyzi), off, n, v);
     return last_launch_status();
 }
 

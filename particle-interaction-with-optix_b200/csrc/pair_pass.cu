@@ -14,6 +14,7 @@ __global__ void __launch_bounds__(kPassThreads) k_pair_pass(GridDev g, PairParam
                                                             int n, int kb, int ke, float* __restrict__ energy,
                                                             float* __restrict__ force, Partial* part,
                                                             unsigned* counter, lj_totals* totals, unsigned* status) {
+    chain_wait();
     const int k = kb + blockIdx.x * kPassThreads + threadIdx.x;
     const bool active = k < ke;
     int c = 0;
@@ -49,6 +50,7 @@ __global__ void __launch_bounds__(BLOCK, 8) k_pair_pass2(GridDev g, PairParams p
                                                              int n, int kb, int ke, float* __restrict__ energy,
                                                              float* __restrict__ force, Partial* part,
                                                              unsigned* counter, lj_totals* totals, unsigned* status) {
+    chain_wait();
     const int ka = kb + 2 * (blockIdx.x * BLOCK + threadIdx.x);
     const bool activeA = ka < ke, activeB = ka + 1 < ke;
     const int ncell = g.gx * g.gy * g.gz;
@@ -117,6 +119,8 @@ __global__ void __launch_bounds__(BLOCK, 8) k_pair_pass2(GridDev g, PairParams p
 __global__ void __launch_bounds__(256) k_cellpair_flags(const int* __restrict__ cs, const int* __restrict__ off,
                                                         int ncell, int kb, int ke, int* __restrict__ flag,
                                                         unsigned* status) {
+    chain_wait();
+    chain_next();
     for (int k = kb + blockIdx.x * blockDim.x + threadIdx.x; k < ke; k += gridDim.x * blockDim.x) {
         const int c = __ldg(&cs[k]);
         int f = 1;  // a target whose cell id is out of range stays alone (and is reported)
@@ -133,6 +137,8 @@ __global__ void __launch_bounds__(256) k_cellpair_flags(const int* __restrict__ 
 // list[pos[i]] = kb + i for every flagged i: the pairs' first targets in sorted order.
 __global__ void __launch_bounds__(256) k_cellpair_list(const int* __restrict__ flag, const int* __restrict__ pos,
                                                        int nk, int kb, int* __restrict__ list) {
+    chain_wait();
+    chain_next();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nk; i += gridDim.x * blockDim.x) {
         const int q = pos[i];
         if (flag[i] && q >= 0 && q < nk) list[q] = kb + i;
@@ -150,6 +156,7 @@ __global__ void __launch_bounds__(BLOCK, 8) k_pair_cellpair(GridDev g, PairParam
                                                             Partial* part, unsigned* counter, lj_totals* totals,
                                                             unsigned* status) {
     __shared__ int2 s_win[9][BLOCK];
+    chain_wait();
     const int t = blockIdx.x * BLOCK + threadIdx.x;
     const int ncell = g.gx * g.gy * g.gz;
     const bool activeA = t < min(__ldg(npairs_p), nk);
@@ -242,16 +249,16 @@ lj_status launch_pair_cellpair(lj_ctx* ctx, const lj_grid* g, const PairParams& 
     int* list = pos + words;
     cudaStream_t st = ctx->stream;
     const int ncell = g->dim[0] * g->dim[1] * g->dim[2];
+    if ((s = scan_prepare(ctx, nk)) != LJ_OK) return s;
     k_cellpair_flags<<<grid_for(ctx, nk, 256), 256, 0, st>>>(cs, off, ncell, kb, ke, flag, ctx->d_status);
     if ((s = last_launch_status()) != LJ_OK) return s;
-    if ((s = launch_scan(ctx, flag, nk, pos)) != LJ_OK) return s;
-    k_cellpair_list<<<grid_for(ctx, nk, 256), 256, 0, st>>>(flag, pos, (int)nk, kb, list);
+    if ((s = scan_prepared(ctx, flag, nk, pos, nullptr)) != LJ_OK) return s;
+    chain_launch(k_cellpair_list, grid_for(ctx, nk, 256), 256, 0, st, flag, pos, (int)nk, kb, list);
     if ((s = last_launch_status()) != LJ_OK) return s;
     unsigned* counter = static_cast<unsigned*>(ctx->red);
     Partial* part = reinterpret_cast<Partial*>(static_cast<char*>(ctx->red) + 256);
-    k_pair_cellpair<><<<blocks, kPassThreads, 0, st>>>(to_dev(*g), pp, reinterpret_cast<const float4*>(xyzi), cs, off,
-                                                       n, (int)nk, ke, list, pos + nk, energy, force, part, counter,
-                                                       totals, ctx->d_status);
+    chain_launch(k_pair_cellpair<>, blocks, kPassThreads, 0, st, to_dev(*g), pp, reinterpret_cast<const float4*>(xyzi),
+                 cs, off, n, (int)nk, ke, list, pos + nk, energy, force, part, counter, totals, ctx->d_status);
     return last_launch_status();
 }
 
@@ -271,11 +278,11 @@ lj_status launch_pair_pass(lj_ctx* ctx, const lj_grid* g, const PairParams& pp, 
     const float4* p4 = reinterpret_cast<const float4*>(xyzi);
     const GridDev gd = to_dev(*g);
     if (two)
-        k_pair_pass2<><<<blocks, kPassThreads, 0, ctx->stream>>>(gd, pp, p4, cs, off, n, kb, ke, energy, force, part,
-                                                                counter, totals, ctx->d_status);
+        chain_launch(k_pair_pass2<>, blocks, kPassThreads, 0, ctx->stream, gd, pp, p4, cs, off, n, kb, ke, energy, force,
+                     part, counter, totals, ctx->d_status);
     else
-        k_pair_pass<<<blocks, kPassThreads, 0, ctx->stream>>>(gd, pp, p4, cs, off, n, kb, ke, energy, force, part,
-                                                              counter, totals, ctx->d_status);
+        chain_launch(k_pair_pass, blocks, kPassThreads, 0, ctx->stream, gd, pp, p4, cs, off, n, kb, ke, energy, force,
+                     part, counter, totals, ctx->d_status);
     return last_launch_status();
 }
 

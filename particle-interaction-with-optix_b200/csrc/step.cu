@@ -48,6 +48,8 @@ __global__ void __launch_bounds__(256) k_verlet_drift(const float4* __restrict__
 __global__ void __launch_bounds__(256) k_verlet_carry(float4* __restrict__ rec, const float* __restrict__ vh,
                                                       const int* __restrict__ ids, int n, float* __restrict__ vel,
                                                       unsigned* status) {
+    chain_wait();
+    chain_next();
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
         float4 r = rec[s];
         int o = __float_as_int(r.w);
@@ -67,6 +69,7 @@ __global__ void __launch_bounds__(256) k_verlet_carry(float4* __restrict__ rec, 
 // Second half kick with the new forces.
 __global__ void __launch_bounds__(256) k_verlet_kick(const float* __restrict__ force, int n3, float h,
                                                      float* __restrict__ vel) {
+    chain_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x)
         vel[i] = __fadd_rn(vel[i], __fmul_rn(h, force[i]));
 }
@@ -103,15 +106,15 @@ extern "C" lj_status lj_step_verlet(lj_ctx* ctx, const lj_grid* g, const lj_para
         LJ_OK)
         return s;
     if (n > 0) {
-        k_verlet_carry<<<blocks, 256, 0, ctx->stream>>>(rec, vh, ids, n, vel, ctx->d_status);
+        chain_launch(k_verlet_carry, blocks, 256, 0, ctx->stream, rec, vh, ids, n, vel, ctx->d_status);
         if ((s = last_launch_status()) != LJ_OK) return s;
     }
     if ((s = lj_compute(ctx, g, p, n, xyzi, sorted_cell, offsets, LJ_ORDER_X, energy, force, totals)) != LJ_OK)
         return s;
     if (n > 0) {
         const int n3 = 3 * n;
-        k_verlet_kick<<<std::max(1, std::min((n3 + 255) / 256, ctx->sm_count * 8)), 256, 0, ctx->stream>>>(
-            force, n3, h, vel);
+        chain_launch(k_verlet_kick, std::max(1, std::min((n3 + 255) / 256, ctx->sm_count * 8)), 256, 0, ctx->stream, force,
+                     n3, h, vel);
         if ((s = last_launch_status()) != LJ_OK) return s;
     }
     return LJ_OK;
