@@ -211,19 +211,43 @@ __global__ void __launch_bounds__(BLOCK, MODE == 2 ? kCluWarpsPerSm * 32 / BLOCK
 }
 
 
-// One block per system: totals from the per-target sums, in index order.
+// Totals of system blockIdx.x / shares from its per-target sums: `shares` blocks take a share each, in a
+// fixed order, and the last of them to finish adds the shares in block order (deterministic).  One block
+// per system took 358 us for 128 systems of up to 200,000 particles (its threads walk a system's sums one
+// load after the other), 15% of the step.
+constexpr int kMaxShares = 32;
+constexpr int kShareParticles = 4096;  // of the largest system, per share
+constexpr int kTotalUnroll = 4;
+
 __global__ void __launch_bounds__(256) k_sys_totals(const SysDev* __restrict__ sys, const float* __restrict__ te,
                                                     const float* __restrict__ tw, const unsigned* __restrict__ tnp,
+                                                    int shares, lj_totals* __restrict__ share,
+                                                    unsigned* __restrict__ done,
                                                     lj_totals* __restrict__ totals) {
     __shared__ double s_e[8], s_w[8];
     __shared__ unsigned long long s_p[8];
-    const SysDev S = sys[blockIdx.x];
+    const int s = (int)blockIdx.x / shares, part = (int)blockIdx.x % shares;
+    const SysDev S = sys[s];
     double e = 0.0, w = 0.0;
     unsigned long long np = 0;
-    for (int k = S.first + threadIdx.x; k < S.first + S.n; k += blockDim.x) {
-        e += 0.5 * (double)S.pp.e4 * (double)te[k];
-        w += 0.5 * (double)S.pp.e24 * (double)tw[k];
-        np += tnp[k];
+    const long long end = (long long)S.first + S.n;
+    const int step = shares * 256;
+    for (long long k0 = (long long)S.first + part * 256 + (int)threadIdx.x; k0 < end; k0 += kTotalUnroll * step) {
+        float ve[kTotalUnroll], vw[kTotalUnroll];
+        unsigned vp[kTotalUnroll];
+#pragma unroll
+        for (int u = 0; u < kTotalUnroll; ++u) {
+            const long long k = k0 + u * step;
+            ve[u] = k < end ? te[k] : 0.f;
+            vw[u] = k < end ? tw[k] : 0.f;
+            vp[u] = k < end ? tnp[k] : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < kTotalUnroll; ++u) {
+            e += 0.5 * (double)S.pp.e4 * (double)ve[u];
+            w += 0.5 * (double)S.pp.e24 * (double)vw[u];
+            np += vp[u];
+        }
     }
     e = warp_sum(e);
     w = warp_sum(w);
@@ -235,15 +259,31 @@ __global__ void __launch_bounds__(256) k_sys_totals(const SysDev* __restrict__ s
         s_p[warp] = np;
     }
     __syncthreads();
+    if (threadIdx.x >= 32) return;
+    lj_totals* mine = share + (size_t)s * kMaxShares;
+    bool last = false;
     if (threadIdx.x == 0) {
         double fe = 0.0, fw = 0.0;
         unsigned long long fp = 0;
-        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
+        for (int i = 0; i < 8; ++i) {
             fe += s_e[i];
             fw += s_w[i];
             fp += s_p[i];
         }
-        totals[blockIdx.x] = lj_totals{fe, fw, fp, 0ULL};
+        mine[part] = lj_totals{fe, fw, fp, 0ULL};
+        __threadfence();
+        last = atomicAdd(&done[s], 1u) == (unsigned)shares - 1u;
+    }
+    if (!__shfl_sync(0xffffffffu, last ? 1 : 0, 0)) return;
+    __threadfence();
+    const bool in = (int)threadIdx.x < shares;
+    const lj_totals* t = mine + threadIdx.x;
+    e = warp_sum(in ? __ldcg(&t->energy) : 0.0);
+    w = warp_sum(in ? __ldcg(&t->virial) : 0.0);
+    np = warp_sum(in ? (unsigned long long)__ldcg(&t->pairs) : 0ULL);
+    if (threadIdx.x == 0) {
+        totals[s] = lj_totals{e, w, np, 0ULL};
+        done[s] = 0u;  // ready for the next step
     }
 }
 
@@ -281,6 +321,8 @@ struct lj_batch {
     float* te = nullptr;
     float* tw = nullptr;
     unsigned* tnp = nullptr;
+    lj_totals* share = nullptr;  // [nsys * kMaxShares] shares of the systems' totals
+    unsigned* done = nullptr;    // [nsys] blocks that have written theirs
     int persistent_blocks[3] = {0, 0, 0};  // grid of the persistent pair kernel per walk mode
     // graph replay
     cudaStream_t gstream = nullptr;
@@ -305,6 +347,8 @@ static void free_plan_buffers(lj_batch* b) {
     cudaFree(b->te);
     cudaFree(b->tw);
     cudaFree(b->tnp);
+    cudaFree(b->share);
+    cudaFree(b->done);
     b->d_sys = nullptr;
     b->d_binsys = nullptr;
     b->d_firsts = nullptr;
@@ -315,6 +359,8 @@ static void free_plan_buffers(lj_batch* b) {
     b->cell = nullptr;
     b->te = b->tw = nullptr;
     b->tnp = nullptr;
+    b->share = nullptr;
+    b->done = nullptr;
     b->tiles_cap = b->cells_cap = 0;
 }
 
@@ -415,8 +461,11 @@ static lj_status build_plan(lj_ctx* ctx, lj_batch* b) {
             (st = dev_alloc(&b->tnp, N)) != LJ_OK || (st = dev_alloc(&b->d_sys, (size_t)b->nsys)) != LJ_OK ||
             (st = dev_alloc(&b->d_firsts, (size_t)b->nsys)) != LJ_OK ||
             (st = dev_alloc(&b->d_binsys, (size_t)b->nsys)) != LJ_OK ||
-            (st = dev_alloc(&b->d_counter, (size_t)64)) != LJ_OK)
+            (st = dev_alloc(&b->d_counter, (size_t)64)) != LJ_OK ||
+            (st = dev_alloc(&b->share, (size_t)b->nsys * kMaxShares)) != LJ_OK ||
+            (st = dev_alloc(&b->done, (size_t)b->nsys)) != LJ_OK)
             return st;
+        if (cudaMemset(b->done, 0, sizeof(unsigned) * (size_t)b->nsys) != cudaSuccess) return LJ_ECUDA;
     }
     if ((size_t)b->total_cells + 1 > b->cells_cap) {
         cudaFree(b->counts);
@@ -534,7 +583,11 @@ static lj_status batch_step(lj_ctx* ctx, lj_batch* b, const float* x, const floa
                : launch_batched_pair<128, 2>(ctx, b, xyzi, energy, force);
     if ((st = last_launch_status()) != LJ_OK) return st;
     if (totals) {
-        k_sys_totals<<<b->nsys, 256, 0, s>>>(b->d_sys, b->te, b->tw, b->tnp, totals);
+        int most = 0;
+        for (const lj_system& y : b->sys) most = std::max(most, y.n);
+        const int shares = std::max(1, std::min(kMaxShares, most / kShareParticles));
+        k_sys_totals<<<(unsigned)b->nsys * (unsigned)shares, 256, 0, s>>>(b->d_sys, b->te, b->tw, b->tnp, shares,
+                                                                          b->share, b->done, totals);
         if ((st = last_launch_status()) != LJ_OK) return st;
     }
     return LJ_OK;
