@@ -372,7 +372,8 @@ LJ_API lj_status lj_batch_autotune(lj_ctx* ctx, lj_batch* b, const float* x, con
  * (stored position = (x, oy + (cy + uy) w, oz + (cz + uz) w)): half the bytes
  * of the float4 layout per neighbour load.  Pair math in FP32 (cell units),
  * each particle's energy and force summed per stencil window (or per pass of
- * the row-pass walks) and those sums added with compensation (TwoSum), totals
+ * the row-pass walks, per plane of rows and lane of the cluster walk) and those
+ * sums added with compensation (TwoSum), totals
  * reduced in FP64.  Results
  * are those of the stored positions: binary16 rounds the y, z offsets to
  * 2^-11 .. 2^-12 of a cell width, and the pair count follows the mixed
@@ -383,8 +384,9 @@ LJ_API lj_status lj_batch_autotune(lj_ctx* ctx, lj_batch* b, const float* x, con
 LJ_API lj_status lj_pack_mixed(lj_ctx* ctx, const lj_grid* g, int n, const float* sorted_xyzi,
                                const int* sorted_cell, float* rec);
 /* Energy, force (sorted order) and totals from the records; as lj_compute.
- * Walk by the tuning's pair_kernel: 0 (default) and 8-10 row passes with two
- * targets per lane; 1 flat walk, windows in shared memory; 2 flat walk,
+ * Walk by the tuning's pair_kernel: 0 (default) the cluster walk from 40
+ * particles per cell (from 8 on small systems), else as 8-10; 8-10 row passes
+ * with two targets per lane; 1 flat walk, windows in shared memory; 2 flat walk,
  * windows in registers; any other value row passes with one target per lane. */
 LJ_API lj_status lj_compute_mixed(lj_ctx* ctx, const lj_grid* g, const lj_params* p, int n, const float* rec,
                                   const int* sorted_cell, const int* offsets, float* energy, float* force,

@@ -20,7 +20,7 @@
 // pair.cu.
 #include <cuda_fp16.h>
 
-#include "pair_common.cuh"
+#include "pair_cluster.cuh"
 
 namespace ljc {
 
@@ -691,6 +691,277 @@ __global__ void __launch_bounds__(kMixThreads, 6) k_pair_mixed_pass2(GridDev g, 
         0.5 * (double)mp.e24 * ((double)a.w.x + (double)a.w.y), (unsigned long long)a.np, part, counter, totals);
 }
 
+// ---------------------------------------------------------------- cluster walk
+// The cluster walk of pair_cluster.cuh on the 8-byte records: 8 consecutive targets of a row of cells per
+// warp, ranges found for 16, the candidates within the cutoff of the cluster's box kept in shared memory.
+// The list of a stencil row holds x and the row's own binary16 offsets widened, and the row's walk uses
+// the targets' frame for it, so every difference rounds as in the other walks and the distance test is
+// theirs.  Each lane sums a quarter of its target's candidates of a plane of three rows in plain FP32
+// (even and odd candidates apart) and adds those sums with TwoSum; the four lanes of a target are
+// combined with TwoSum as well.
+//
+// Bound as the plain walk, plus one paired product per two evaluations (the scaling of dx) and the lists'
+// filling up to 16 per row, which thin rows pay most for.  Measured on B200 against the row passes of two
+// targets per lane, pair stage, uniform particles: 2M at 80 per cell 2105 against 2720 us, at 40 1421
+// against 1466, but at 20 1059 against 899; 50,000 at 20 per cell 54 against 88, 10,000 at 10 35 against
+// 45 (with 28 warps per SM and spills 2255 us at 80 per cell, with 20 warps 2114).
+struct MixClu {
+    float2 x, y, z;  // minus the target's x, and minus its y, z in the row's frame
+};
+
+__device__ __forceinline__ void mix_clu_eval(float2 qx, float2 qy, float2 qz, const MixClu& t, float2 invw, float rc2u,
+                                             float2 nsig2, CluAcc& a) {
+    const float2 dx = __fmul2_rn(__fadd2_rn(qx, t.x), invw);
+    const float2 dy = __fadd2_rn(qy, t.y);
+    const float2 dz = __fadd2_rn(qz, t.z);
+    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+    float2 ir2;
+    ir2.x = rcp_count(r2.x, rc2u, a.np);
+    ir2.y = rcp_count(r2.y, rc2u, a.np);
+    clu_law(dx, dy, dz, ir2, nsig2, a);
+}
+
+__device__ __forceinline__ void mix_clu_walk(const CluSmem& sm, int cnt, int s, const MixClu& t, float2 invw, float rc2u,
+                                             float2 nsig2, CluAcc& a) {
+#pragma unroll 2
+    for (int v = 4 * s; v < cnt; v += 16) {
+        const float4 X = *reinterpret_cast<const float4*>(&sm.x[v]);
+        const float4 Y = *reinterpret_cast<const float4*>(&sm.y[v]);
+        const float4 Z = *reinterpret_cast<const float4*>(&sm.z[v]);
+        mix_clu_eval(make_float2(X.x, X.y), make_float2(Y.x, Y.y), make_float2(Z.x, Z.y), t, invw, rc2u, nsig2, a);
+        mix_clu_eval(make_float2(X.z, X.w), make_float2(Y.z, Y.w), make_float2(Z.z, Z.w), t, invw, rc2u, nsig2, a);
+    }
+}
+
+constexpr int kMixCluWarps = 4;
+constexpr int kMixCluWarpsPerSm = 24;       // 80 registers: the compensated sums leave no room for 28 warps
+constexpr double kMixClusterCell = 40.0;    // particles per cell from which the default takes it ...
+constexpr double kMixClusterFew = 8.0;      // ... and where all groups run at once
+
+__global__ void __launch_bounds__(32 * kMixCluWarps, kMixCluWarpsPerSm / kMixCluWarps)
+    k_pair_mixed_cluster(GridDev g, MixParams mp, const float2* __restrict__ rec, const int* __restrict__ cs,
+                         const int* __restrict__ off, int n, int stretch, float* __restrict__ energy,
+                         float* __restrict__ force, Partial* part, unsigned* counter, lj_totals* totals,
+                         unsigned* status) {
+    __shared__ __align__(16) CluSmem smem[kMixCluWarps];
+    CluSmem& sm = smem[threadIdx.x >> 5];
+    const int lane = (int)(threadIdx.x & 31u), t = lane & 7, s = lane >> 3;
+    const unsigned below = lanemask_lt();
+    const int ncell = g.gx * g.gy * g.gz;
+    const float rc2u = mp.rc2u;
+    const float2 nsig2 = make_float2(-mp.sig2u, -mp.sig2u), invw = make_float2(mp.invw, mp.invw);
+    double te = 0.0, tw = 0.0;
+    unsigned long long tp = 0;
+    const long long first = (long long)blockIdx.x * stretch;
+    const int b = (int)min(first + stretch, (long long)n);
+    int gs = (int)min(first, (long long)n), se = gs, row0 = 0, cy = 0, cz = 0, turn = (int)(threadIdx.x >> 5);
+    bool entered = false;
+    while (gs < b) {
+        if (gs >= se) {  // a new segment of cells (groups are counted from its start)
+            int c = __ldg(&cs[gs]);
+            if (c < 0 || c >= ncell) {
+                if (lane == 0) atomicOr(status, kFlagRange);
+                c = 0;
+            }
+            const int row = c / g.gx, cx = c - row * g.gx;
+            cz = row / g.gy;
+            cy = row - cz * g.gy;
+            row0 = row * g.gx;
+            const int c0 = row0 + cx / kCluSegment * kCluSegment, c1 = min(c0 + kCluSegment, row0 + g.gx);
+            const int ss = min(max(__ldg(&off[c0]), 0), gs);
+            se = min(max(__ldg(&off[c1]), gs + 1), n);
+            if (!entered) {
+                entered = true;
+                gs = min(ss + (gs - ss + kCluGroup - 1) / kCluGroup * kCluGroup, se);
+                if (gs >= se) continue;
+                if (gs >= b) break;
+            }
+        }
+        const int ge = min(gs + kCluGroup, se);
+        if (turn != 0) {
+            --turn;
+            gs = ge;
+            continue;
+        }
+        turn = kMixCluWarps - 1;
+        // candidate ranges of the group's box: lanes 0-8 find the start, lanes 9-17 the end of stencil row r
+        {
+            const int k = min(gs + (lane & (kCluGroup - 1)), ge - 1);
+            const float2 q = __ldg(&rec[k]);
+            const float2 u = unpack_yz(q.y);
+            const int ck = __ldg(&cs[k]) - row0;
+            const int cxa = min(max(__shfl_sync(0xffffffffu, ck, 0), 0), g.gx - 1);
+            const int cxb = min(max(__shfl_sync(0xffffffffu, ck, kCluGroup - 1), cxa), g.gx - 1);
+            const float x0 = warp_min(q.x), x1 = warp_max(q.x), y0 = warp_min(u.x), y1 = warp_max(u.x), z0 = warp_min(u.y),
+                        z1 = warp_max(u.y);
+            int pos = 0;
+            const bool second = lane >= 9;
+            const int r = second ? lane - 9 : lane;
+            if (r < 9) {
+                const int rz = r / 3, dz = rz - 1, dy = r - 3 * rz - 1;
+                const int z = cz + dz, y = cy + dy;
+                if (z >= 0 && z < g.gz && y >= 0 && y < g.gy) {
+                    const float slack = mp.slack + 8.0f * FLT_EPSILON * fmaxf(fabsf(x0), fabsf(x1));
+                    const float slack_u = 1e-5f;
+                    float dzm = dz < 0 ? z0 : (dz > 0 ? 1.0f - z1 : 0.f);
+                    float dym = dy < 0 ? y0 : (dy > 0 ? 1.0f - y1 : 0.f);
+                    dzm = fmaxf(dzm - slack_u, 0.f);
+                    dym = fmaxf(dym - slack_u, 0.f);
+                    const float d2 = fmaf(dym, dym, dzm * dzm);
+                    if (d2 < mp.rc2uw) {
+                        const int rb = (z * g.gy + y) * g.gx;
+                        int lo = min(max(__ldg(&off[rb + max(cxa - 1, 0)]), 0), n);
+                        int hi = min(max(__ldg(&off[rb + min(cxb + 1, g.gx - 1) + 1]), lo), n);
+                        const float h = sqrtf(mp.rc2uw - d2) * mp.w + slack;
+                        const float v = second ? x1 + h : x0 - h;
+                        while (lo < hi) {  // first x >= v (starts) or x > v (ends)
+                            const int mid = (lo + hi) >> 1;
+                            const float x = __ldg(&rec[mid].x);
+                            if (x < v || (second && x == v))
+                                lo = mid + 1;
+                            else
+                                hi = mid;
+                        }
+                        pos = lo;
+                    }
+                }
+            }
+            const int re = __shfl_down_sync(0xffffffffu, pos, 9);
+            if (lane < 9) sm.range[lane] = make_int4(pos, re, 0, 0);
+            __syncwarp();
+        }
+        for (int cl = gs; cl < ge; cl += kCluTargets) {
+            const int nt = min(kCluTargets, ge - cl);
+            const int k = cl + min(t, nt - 1);  // lanes past the end repeat the last target
+            const float2 q = __ldg(&rec[k]);
+            const float2 u = unpack_yz(q.y);
+            const float bx0 = warp_min(q.x), bx1 = warp_max(q.x), by0 = warp_min(u.x), by1 = warp_max(u.x),
+                        bz0 = warp_min(u.y), bz1 = warp_max(u.y);
+            CluAcc acc;
+            acc.s12 = acc.ns6 = acc.fx = acc.fy = acc.fz = make_float2(0.f, 0.f);
+            acc.np = 0;
+            float se_ = 0.f, ce = 0.f, sx = 0.f, cx_ = 0.f, sy = 0.f, cy_ = 0.f, sz = 0.f, cz_ = 0.f;
+            double wv = 0.0;
+            MixClu tt;
+            tt.x = make_float2(-q.x, -q.x);
+            {  // the cluster's own targets: lane group s takes targets 2s and 2s + 1
+                const int c0 = 2 * s, c1 = c0 + 1;
+                const float2 dx = __fmul2_rn(__fadd2_rn(make_float2(__shfl_sync(0xffffffffu, q.x, c0),
+                                                                    __shfl_sync(0xffffffffu, q.x, c1)), tt.x), invw);
+                const float2 dy = __fadd2_rn(make_float2(__shfl_sync(0xffffffffu, u.x, c0),
+                                                         __shfl_sync(0xffffffffu, u.x, c1)), make_float2(-u.x, -u.x));
+                const float2 dz = __fadd2_rn(make_float2(__shfl_sync(0xffffffffu, u.y, c0),
+                                                         __shfl_sync(0xffffffffu, u.y, c1)), make_float2(-u.y, -u.y));
+                const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
+                const float inf = __int_as_float(0x7f800000);
+                float2 ir2;
+                ir2.x = rcp_count(c0 != t && c0 < nt ? r2.x : inf, rc2u, acc.np);
+                ir2.y = rcp_count(c1 != t && c1 < nt ? r2.y : inf, rc2u, acc.np);
+                clu_law(dx, dy, dz, ir2, nsig2, acc);
+            }
+#pragma unroll 1
+            for (int r = 0; r < 9; ++r) {
+                const int4 rg = sm.range[r];
+                const float fy = (float)(r % 3 - 1), fz = (float)(r / 3 - 1);
+                const float ty = u.x - fy, tz = u.y - fz;
+                tt.y = make_float2(-ty, -ty);
+                tt.z = make_float2(-tz, -tz);
+                const float y0 = by0 - fy, y1 = by1 - fy, z0 = bz0 - fz, z1 = bz1 - fz;
+                int cnt = 0;
+                // scan: 64 records a step; the box test rounds as the distance test does, operation by
+                // operation on smaller magnitudes, so it drops no candidate that a target accepts
+                for (int j0 = rg.x; j0 < rg.y; j0 += 64) {
+                    const int j = j0 + 2 * lane;
+                    const bool ok0 = j < rg.y, ok1 = j + 1 < rg.y;
+                    const float2 a0 = __ldg(&rec[ok0 ? j : cl]), a1 = __ldg(&rec[ok1 ? j + 1 : cl]);
+                    const float2 u0 = unpack_yz(a0.y), u1 = unpack_yz(a1.y);
+                    const float dx0 = fmaxf(fmaxf(bx0 - a0.x, a0.x - bx1), 0.f) * mp.invw;
+                    const float dx1 = fmaxf(fmaxf(bx0 - a1.x, a1.x - bx1), 0.f) * mp.invw;
+                    const float dy0 = fmaxf(fmaxf(y0 - u0.x, u0.x - y1), 0.f), dy1 = fmaxf(fmaxf(y0 - u1.x, u1.x - y1), 0.f);
+                    const float dz0 = fmaxf(fmaxf(z0 - u0.y, u0.y - z1), 0.f), dz1 = fmaxf(fmaxf(z0 - u1.y, u1.y - z1), 0.f);
+                    const float d0 = fmaf(dz0, dz0, fmaf(dy0, dy0, dx0 * dx0));
+                    const float d1 = fmaf(dz1, dz1, fmaf(dy1, dy1, dx1 * dx1));
+                    const unsigned own = (unsigned)(j - cl);
+                    const bool keep0 = ok0 && d0 < rc2u && own >= (unsigned)nt;
+                    const bool keep1 = ok1 && d1 < rc2u && own + 1u >= (unsigned)nt;
+                    const unsigned m0 = __ballot_sync(0xffffffffu, keep0), m1 = __ballot_sync(0xffffffffu, keep1);
+                    const int mid = cnt + __popc(m0);
+                    if (keep0) {
+                        const int w = cnt + __popc(m0 & below);
+                        sm.x[w] = a0.x;
+                        sm.y[w] = u0.x;
+                        sm.z[w] = u0.y;
+                    }
+                    if (keep1) {
+                        const int w = mid + __popc(m1 & below);
+                        sm.x[w] = a1.x;
+                        sm.y[w] = u1.x;
+                        sm.z[w] = u1.y;
+                    }
+                    cnt = mid + __popc(m1);
+                    if (cnt > kCluList - 64 && j0 + 64 < rg.y) {  // no room for another step: walk the whole runs, keep the rest
+                        __syncwarp();
+                        const int whole = cnt & ~15;
+                        mix_clu_walk(sm, whole, s, tt, invw, rc2u, nsig2, acc);
+                        __syncwarp();
+                        const int rest = cnt - whole;
+                        if (lane < rest) {
+                            sm.x[lane] = sm.x[whole + lane];
+                            sm.y[lane] = sm.y[whole + lane];
+                            sm.z[lane] = sm.z[whole + lane];
+                        }
+                        cnt = rest;
+                    }
+                }
+                if (cnt) {  // fill the last run with candidates beyond any cutoff, in every coordinate finite
+                    if (lane < ((16 - cnt) & 15)) sm.x[cnt + lane] = sm.y[cnt + lane] = sm.z[cnt + lane] = 1e12f;
+                    __syncwarp();
+                    mix_clu_walk(sm, (cnt + 15) & ~15, s, tt, invw, rc2u, nsig2, acc);
+                    __syncwarp();
+                }
+                if (r % 3 == 2) {  // a plane of rows done: its sums with compensation
+                    const float s12 = acc.s12.x + acc.s12.y, ns6 = acc.ns6.x + acc.ns6.y;
+                    two_sum_add(se_, ce, s12 + ns6);
+                    two_sum_add(sx, cx_, acc.fx.x + acc.fx.y);
+                    two_sum_add(sy, cy_, acc.fy.x + acc.fy.y);
+                    two_sum_add(sz, cz_, acc.fz.x + acc.fz.y);
+                    wv += (double)fmaf(2.0f, s12, ns6);
+                    acc.s12 = acc.ns6 = acc.fx = acc.fy = acc.fz = make_float2(0.f, 0.f);
+                }
+            }
+#pragma unroll
+            for (int o = 8; o < 32; o <<= 1) {
+                const float ee = __shfl_xor_sync(0xffffffffu, se_, o), ex = __shfl_xor_sync(0xffffffffu, sx, o),
+                            ey = __shfl_xor_sync(0xffffffffu, sy, o), ez = __shfl_xor_sync(0xffffffffu, sz, o);
+                const float de = __shfl_xor_sync(0xffffffffu, ce, o), dx = __shfl_xor_sync(0xffffffffu, cx_, o),
+                            dy = __shfl_xor_sync(0xffffffffu, cy_, o), dz = __shfl_xor_sync(0xffffffffu, cz_, o);
+                two_sum_add(se_, ce, ee);
+                two_sum_add(sx, cx_, ex);
+                two_sum_add(sy, cy_, ey);
+                two_sum_add(sz, cz_, ez);
+                ce += de;
+                cx_ += dx;
+                cy_ += dy;
+                cz_ += dz;
+            }
+            if (t < nt) {
+                tw += wv;
+                tp += acc.np;
+                if (s == 0) {
+                    te += (double)(se_ + ce);
+                    if (energy) energy[k] = mp.e4 * (se_ + ce);
+                } else if (force) {
+                    const float f = s == 1 ? sx + cx_ : (s == 2 ? sy + cy_ : sz + cz_);
+                    force[3 * (size_t)k + (s - 1)] = -mp.fscale * f;
+                }
+            }
+        }
+        gs = ge;
+    }
+    __syncwarp();
+    reduce_totals<32 * kMixCluWarps>(0.5 * (double)mp.e4 * te, 0.5 * (double)mp.e24 * tw, tp, part, counter, totals);
+}
+
 }  // namespace ljc
 
 using namespace ljc;
@@ -733,8 +1004,12 @@ extern "C" lj_status lj_compute_mixed(lj_ctx* ctx, const lj_grid* g, const lj_pa
     mp.e24 = 24.0f * p->epsilon;
     mp.fscale = -mp.e24 * g->width / sig2;
     mp.slack = grid_slack(*g);
-    const bool two = ctx->tuning.pair_kernel == 0 || ctx->tuning.pair_kernel >= 8;  // two targets per lane
-    const int per_block = two ? 2 * kMixThreads : kMixThreads;
+    const double per_cell = (double)n / ((double)g->dim[0] * g->dim[1] * g->dim[2]);
+    const bool cluster = ctx->tuning.pair_kernel == 0 &&
+                         (per_cell >= kMixClusterCell ||
+                          (per_cell >= kMixClusterFew && n <= ctx->sm_count * kMixCluWarpsPerSm * kCluGroup));
+    const bool two = !cluster && (ctx->tuning.pair_kernel == 0 || ctx->tuning.pair_kernel >= 8);  // two targets per lane
+    const int per_block = cluster ? kMixCluWarps * kCluGroup : (two ? 2 * kMixThreads : kMixThreads);
     const int blocks = (n + per_block - 1) / per_block;
     const size_t need = 256 + (size_t)blocks * sizeof(Partial);
     if (need > ctx->red_bytes) {
@@ -744,10 +1019,14 @@ extern "C" lj_status lj_compute_mixed(lj_ctx* ctx, const lj_grid* g, const lj_pa
     }
     unsigned* counter = static_cast<unsigned*>(ctx->red);
     Partial* part = reinterpret_cast<Partial*>(static_cast<char*>(ctx->red) + 256);
-    // row passes with two targets per lane by default (and with the tuning's two-target kernels 8-10);
-    // pair_kernel 1 (windows in shared memory) or 2 (windows in registers) asks for a flat walk, the
-    // others for row passes with one target per lane
-    if (two)
+    // by default the cluster walk on dense or small systems, else row passes with two targets per lane (as
+    // with the tuning's kernels 8-10); pair_kernel 1 (windows in shared memory) or 2 (windows in registers)
+    // asks for a flat walk, the others for row passes with one target per lane
+    if (cluster)
+        k_pair_mixed_cluster<<<blocks, 32 * kMixCluWarps, 0, ctx->stream>>>(
+            to_dev(*g), mp, reinterpret_cast<const float2*>(rec), sorted_cell, offsets, n, per_block, energy, force, part,
+            counter, totals, ctx->d_status);
+    else if (two)
         k_pair_mixed_pass2<<<blocks, kMixThreads, 0, ctx->stream>>>(to_dev(*g), mp,
                                                                     reinterpret_cast<const float2*>(rec), sorted_cell,
                                                                     offsets, n, energy, force, part, counter, totals,

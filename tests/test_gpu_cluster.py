@@ -61,3 +61,29 @@ def test_cluster_walk_edges(torch_cuda, ctx, name, order):
         assert torch.equal(pe[kb:ke].view(torch.int32), e[kb:ke].view(torch.int32))
         assert torch.equal(pf[kb:ke].view(torch.int32), f[kb:ke].view(torch.int32))
         assert bool(torch.isnan(pe[:kb]).all()) and bool(torch.isnan(pe[ke:n]).all())
+
+
+@pytest.mark.parametrize("name", [f"one_cell_{n}" for n in (8, 9, 15, 16, 17, 31, 33)] + ["row_of_33_cells", "list_overflows",
+                                                                                          "cutoff_below_width"])
+def test_mixed_cluster_walk_edges(torch_cuda, ctx, name):
+    """The mixed form's cluster walk at the same edges, against FP64 on the stored positions."""
+    import ljcell
+
+    torch = torch_cuda
+    (lo, hi), width, rc, n = SHAPES[name]
+    rng = np.random.default_rng(n)
+    lo32, hi32 = np.array(lo, np.float32), np.array(hi, np.float32)
+    pts = (lo32 + (hi32 - lo32) * rng.random((n, 3), dtype=np.float32)).astype(np.float32)
+    x, y, z = (np.ascontiguousarray(pts[:, k]) for k in range(3))
+    g, og = ljcell.grid_from_box(lo, hi, width), O.grid_from_box(lo, hi, width)
+    assert n >= 8 * g.ncells
+    p = ljcell.params(rc, sigma=rc / 10)
+    b = ctx.bin(g, dev(torch, x), dev(torch, y), dev(torch, z))
+    e, f, tot = ctx.compute_mixed(g, p, b, ctx.pack_mixed(g, b))
+    ctx.sync()
+    ob = O.bin_particles(og, x, y, z, O.ORDER_X)
+    ref = O.mixed_forces(og, ob, *O.pack_mixed(og, ob), rc, 1.0, p.sigma)
+    assert ljcell.totals_from_tensor(tot)["pairs"] == ref.pairs
+    fe, ee = ref.force_errors(np_(f)[:n]), ref.energy_errors(np_(e)[:n])
+    assert fe["max_scaled"] <= FORCE_SCALED_TOL and fe["normwise"] <= FORCE_NORMWISE_TOL
+    assert ee["max_scaled"] <= ENERGY_SCALED_TOL
