@@ -59,11 +59,11 @@ lj_status launch_pair_cluster(lj_ctx* ctx, const lj_grid* g, const PairParams& p
     const long long nk = ke - a0;
     // a group's clusters to two warps while all of them run at once (1,000 particles at 12 per cell 18.4
     // against 24.5 us, 30,000 25.4 against 30.7, but 60,000 38.9 against 36.9: each of the two warps finds
-    // the group's ranges); then groups per warp: 1 while that leaves one wave of warps, at most 4
+    // the group's ranges); then more groups per warp with the size of the launch
     const long long wave = (long long)ctx->sm_count * kCluWarpsPerSm * kCluGroup;
     const bool split = 2 * nk <= wave;
     const int stretch = split ? kCluWarps / 2 * kCluGroup
-                              : kCluWarps * kCluGroup * (nk <= wave ? 1 : (nk <= 4 * wave ? 2 : 4));
+                              : kCluWarps * kCluGroup * clu_groups_per_warp((double)nk / (double)wave);
     const int blocks = (int)((nk + stretch - 1) / stretch);
     const size_t need = 256 + (size_t)blocks * sizeof(Partial);
     if (need > ctx->red_bytes) {

@@ -1009,7 +1009,8 @@ extern "C" lj_status lj_compute_mixed(lj_ctx* ctx, const lj_grid* g, const lj_pa
                          (per_cell >= kMixClusterCell ||
                           (per_cell >= kMixClusterFew && n <= ctx->sm_count * kMixCluWarpsPerSm * kCluGroup));
     const bool two = !cluster && (ctx->tuning.pair_kernel == 0 || ctx->tuning.pair_kernel >= 8);  // two targets per lane
-    const int per_block = cluster ? kMixCluWarps * kCluGroup : (two ? 2 * kMixThreads : kMixThreads);
+    const double waves = (double)n / ((double)ctx->sm_count * kMixCluWarpsPerSm * kCluGroup);
+    const int per_block = cluster ? kMixCluWarps * kCluGroup * clu_groups_per_warp(waves) : (two ? 2 * kMixThreads : kMixThreads);
     const int blocks = (n + per_block - 1) / per_block;
     const size_t need = 256 + (size_t)blocks * sizeof(Partial);
     if (need > ctx->red_bytes) {
