@@ -66,6 +66,11 @@ def bin_launches(n: int, ncells: int) -> int:
         return 3 + passes + 6
     return 4 + min(passes, ncells)
 
+def compat_kernel(n: int, ncells: int) -> str:
+    """The reference law's kernel: a warp per cell from 6 particles per cell (or on few cells)."""
+    return "k_compat_cells" if n >= 6 * ncells else "k_pair_compat"
+
+
 CONFIGS = {
     "c1": dict(workload="uniform 100k, rc=0.05", n=100_000, dist="uniform", lo=(0, 0, 0), hi=(1, 1, 1), rc=0.05),
     "c2": dict(workload="uniform 10M, rc=0.01", n=10_000_000, dist="uniform", lo=(0, 0, 0), hi=(1, 1, 1), rc=0.01),
@@ -392,8 +397,9 @@ def run_ours(args, cfg):
     pair_ms = float(np.median(t_pair))
     achieved = algo_flops / (pair_ms * 1e-3) / 1e12
     useful = (algo_flops if mode == "compat" else FLOP_INTERACTING * pairs) / (pair_ms * 1e-3) / 1e12
-    kname = {"config": kernel_name(pair_kernel) if pair_kernel else "", "mixed": "k_pair_mixed_pass2",
-             "compat": "k_pair_compat"}[mode]
+    kname = {"config": kernel_name(pair_kernel) if pair_kernel else "",
+             "mixed": "k_pair_mixed_cluster" if n >= 40 * g.ncells else "k_pair_mixed_pass2",
+             "compat": compat_kernel(n, g.ncells)}[mode]
     traffic = read_traffic(kname, cfg["workload"])
 
     # errors of the last step's outputs against an FP64 reference on a stratified target sample
@@ -416,7 +422,7 @@ def run_ours(args, cfg):
         ctx.sync()
         ccand = int(cc.item())
         rate = ccand / (compat_ms * 1e-3)
-        compat = {"ms": compat_ms, "kernel": "k_pair_compat", "candidate_pairs": ccand,
+        compat = {"ms": compat_ms, "kernel": compat_kernel(n, g.ncells), "candidate_pairs": ccand,
                   "candidate_pairs_per_s": rate,
                   "gflops_reference_definition": 18 * rate / 1e9,   # NbFlopsPerInteraction = 18, cudaLJ.cu:550
                   "fp32_frac": 18 * rate / 1e12 / peak_tflops,
@@ -709,7 +715,7 @@ def mixed_workload(ctx, cfg, seed, flush, reps=10):
     err_plain = error_stats(*ref_caller, e[:n], f[:n])
     out = {"workload": cfg["workload"] + ", mixed precision", "ms_pair_plain": t_plain,
            "plain_kernel": kernel_name(kern), "ms_pack_mixed": t_pack, "ms_pack_and_pair_mixed": t_mixed,
-           "mixed_kernel": {0: "k_pair_mixed_pass2", 1: "k_pair_mixed", 2: "k_pair_mixed_reg"}[mk],
+           "mixed_kernel": {0: "k_pair_mixed_cluster" if n >= 40 * g.ncells else "k_pair_mixed_pass2", 1: "k_pair_mixed", 2: "k_pair_mixed_reg"}[mk],
            "speedup_vs_plain": t_plain / t_mixed, "pairs_plain": plain_pairs, "pairs_mixed": mixed_pairs,
            "errors_vs_fp64": {
                "mixed_vs_caller_positions": err_mixed_caller,
