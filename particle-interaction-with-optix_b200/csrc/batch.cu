@@ -29,8 +29,9 @@ struct SysDev {
     int cell_base;
     int first;
     int n;
-    int walk;  // 1: one target per lane (kernel 6's walk), 2: the cluster walk (kernel 1's), 3: two targets per
-               // lane (kernel 10's), as the single-system default chooses for the system
+    int walk;  // 1: one target per lane (kernel 6's walk), 2: the cluster walk (kernel 1's), as the single-system
+               // default chooses for the system; 4: chosen after the binning, 2 or 3 (two targets per lane,
+               // kernel 10's walk), from the cells that hold its particles (k_sys_walk)
 };
 
 // ---------------------------------------------------------------- count
@@ -83,9 +84,45 @@ __global__ void __launch_bounds__(256) k_count_batched(const SysDev* __restrict_
 // indices, so per-particle results equal a per-system lj_compute with that
 // kernel bit for bit.  One launch per walk mode, over the tiles of the systems
 // using it.  Per-target raw sums go to te / tw / tnp for the per-system totals.
+// Walk of a system whose particles average 2 to 6 per cell of its whole grid (walk 4): the mean occupancy of
+// the cells of 256 of its particles.  On a uniform system that is the average plus 1, below 8, where two
+// targets per lane win (2M at 3 per cell 317 against 381 us); on a shell, whose grid is mostly empty, its
+// cells hold 8 and more, where the cluster walk wins (200,000 particles at 23 per occupied cell 88 against
+// 270 us).  One warp; cell and off in one numbering, n particles from cell[0] on.
+constexpr float kShellOccupancy = 8.0f;
+
+__device__ __forceinline__ int sampled_walk(const int* __restrict__ cell, const int* __restrict__ off, int n, int ncell) {
+    const int lane = (int)(threadIdx.x & 31u);
+    int sum = 0;
+    for (int u = 0; u < 8; ++u) {
+        const int c = __ldg(&cell[(int)((long long)n * (8 * lane + u) / 256)]);
+        if (c >= 0 && c < ncell) sum += __ldg(&off[c + 1]) - __ldg(&off[c]);
+    }
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    return (float)sum >= 256.0f * kShellOccupancy ? 2 : 3;
+}
+
+// One warp per system: its walk (cells and offsets in the batch's numbering).
+__global__ void __launch_bounds__(256) k_sys_walk(const SysDev* __restrict__ sys, int nsys, const int* __restrict__ cell,
+                                                  const int* __restrict__ off, int total_cells, int* __restrict__ walk) {
+    const int s = (int)(blockIdx.x * 8 + (threadIdx.x >> 5));
+    if (s >= nsys) return;
+    int w = sys[s].walk;
+    if (w == 4) w = sys[s].n > 0 ? sampled_walk(cell + sys[s].first, off, sys[s].n, total_cells) : 3;
+    if ((threadIdx.x & 31u) == 0) walk[s] = w;
+}
+
+// The same for one system in its own numbering.
+__global__ void __launch_bounds__(32) k_one_walk(const int* __restrict__ cell, const int* __restrict__ off, int n, int ncell,
+                                                 int* __restrict__ walk) {
+    const int w = sampled_walk(cell, off, n, ncell);
+    if (threadIdx.x == 0) *walk = w;
+}
+
 template <int BLOCK, int PPT, int MODE>
 __global__ void __launch_bounds__(BLOCK, MODE == 2 ? kCluWarpsPerSm * 32 / BLOCK : 1) k_pair_batched(const SysDev* __restrict__ sys, const float4* __restrict__ p,
                                                         const int* __restrict__ cs, const int* __restrict__ off,
+                                                        const int* __restrict__ walk,
                                                         const int4* __restrict__ tiles, int ntiles,
                                                         unsigned* tile_counter, float* __restrict__ energy,
                                                         float* __restrict__ force, float* __restrict__ te,
@@ -98,6 +135,10 @@ __global__ void __launch_bounds__(BLOCK, MODE == 2 ? kCluWarpsPerSm * 32 / BLOCK
         const int t = s_t;
         if (t >= ntiles) break;
         const int4 d = __ldg(&tiles[t]);
+        if (walk[d.x] != MODE) {
+            __syncthreads();  // s_t is reused by the next tile
+            continue;
+        }
         const SysDev S = sys[d.x];
         const int ncell = S.g.gx * S.g.gy * S.g.gz;
         const float4* ps = p + S.first;
@@ -310,7 +351,7 @@ struct lj_batch {
     int* d_firsts = nullptr;
     int4* d_tiles = nullptr;
     int ntiles = 0;
-    int ntiles1 = 0, ntiles2 = 0;  // tiles [0, ntiles1) use walk mode 1, [ntiles1, ntiles2) mode 2, the rest mode 3
+    int ntiles1 = 0, ntiles2 = 0;  // tiles [0, ntiles1) use walk mode 1, [ntiles1, ntiles2) mode 2, the rest 2 or 3
     size_t tiles_cap = 0;
     unsigned* d_counter = nullptr;
     int* counts = nullptr;
@@ -322,6 +363,7 @@ struct lj_batch {
     float* tw = nullptr;
     unsigned* tnp = nullptr;
     lj_totals* share = nullptr;  // [nsys * kMaxShares] shares of the systems' totals
+    int* walk = nullptr;         // [nsys] the systems' walks, written after the binning
     unsigned* done = nullptr;    // [nsys] blocks that have written theirs
     int persistent_blocks[3] = {0, 0, 0};  // grid of the persistent pair kernel per walk mode
     // graph replay
@@ -349,6 +391,7 @@ static void free_plan_buffers(lj_batch* b) {
     cudaFree(b->tnp);
     cudaFree(b->share);
     cudaFree(b->done);
+    cudaFree(b->walk);
     b->d_sys = nullptr;
     b->d_binsys = nullptr;
     b->d_firsts = nullptr;
@@ -361,6 +404,7 @@ static void free_plan_buffers(lj_batch* b) {
     b->tnp = nullptr;
     b->share = nullptr;
     b->done = nullptr;
+    b->walk = nullptr;
     b->tiles_cap = b->cells_cap = 0;
 }
 
@@ -395,7 +439,7 @@ static lj_status build_grids(lj_batch* b) {
         // the walk of the single-system default's kernel; kernel 6's where that is kernel 12 (the
         // persistent tile queue has no pair list)
         const int kernel = default_pair_kernel(y.n, g);
-        d.walk = kernel == 1 ? 2 : (kernel == 10 ? 3 : 1);
+        d.walk = kernel == 1 ? 2 : (kernel == 10 ? 4 : 1);
         base += (long long)g.dim[0] * g.dim[1] * g.dim[2];
         if (base > 2147483646LL) return LJ_EUNSUPPORTED;
     }
@@ -404,7 +448,8 @@ static lj_status build_grids(lj_batch* b) {
 }
 
 // Tiles of T = threads * per_thread consecutive targets per system (2T for systems on the cluster or
-// the two-target walk): first those of the systems walked with mode 1, then 2, then 3, each ordered by estimated
+// the two-target walk): first those of walk 1, then 2, then 4 (in which modes 2 and 3
+// take theirs), each ordered by estimated
 // cost (targets x expected candidates: n / box volume x cutoff^3), largest first.
 static std::vector<int4> build_tiles(const lj_batch* b) {
     const int T = b->cfg.threads * b->cfg.per_thread;
@@ -463,6 +508,7 @@ static lj_status build_plan(lj_ctx* ctx, lj_batch* b) {
             (st = dev_alloc(&b->d_binsys, (size_t)b->nsys)) != LJ_OK ||
             (st = dev_alloc(&b->d_counter, (size_t)64)) != LJ_OK ||
             (st = dev_alloc(&b->share, (size_t)b->nsys * kMaxShares)) != LJ_OK ||
+            (st = dev_alloc(&b->walk, (size_t)b->nsys)) != LJ_OK ||
             (st = dev_alloc(&b->done, (size_t)b->nsys)) != LJ_OK)
             return st;
         if (cudaMemset(b->done, 0, sizeof(unsigned) * (size_t)b->nsys) != cudaSuccess) return LJ_ECUDA;
@@ -537,13 +583,13 @@ static void launch_batched_mode(lj_ctx* ctx, lj_batch* b, const float* p4, float
     if (t1 <= t0) return;
     const int grid = std::min(b->persistent_blocks[MODE - 1], t1 - t0);
     k_pair_batched<BLOCK, PPT, MODE><<<grid, BLOCK, 0, ctx->stream>>>(
-        b->d_sys, reinterpret_cast<const float4*>(p4), b->cell, b->offsets, b->d_tiles + t0,
+        b->d_sys, reinterpret_cast<const float4*>(p4), b->cell, b->offsets, b->walk, b->d_tiles + t0,
         t1 - t0, b->d_counter + (MODE - 1), energy, force, b->te, b->tw, b->tnp, ctx->d_status);
 }
 
 template <int BLOCK, int PPT>
 static void launch_batched_pair(lj_ctx* ctx, lj_batch* b, const float* p4, float* energy, float* force) {
-    launch_batched_mode<BLOCK, PPT, 2>(ctx, b, p4, energy, force, b->ntiles1, b->ntiles2);
+    launch_batched_mode<BLOCK, PPT, 2>(ctx, b, p4, energy, force, b->ntiles1, b->ntiles);
     launch_batched_mode<BLOCK, PPT, 3>(ctx, b, p4, energy, force, b->ntiles2, b->ntiles);
     launch_batched_mode<BLOCK, PPT, 1>(ctx, b, p4, energy, force, 0, b->ntiles1);
 }
@@ -571,6 +617,9 @@ static lj_status batch_step(lj_ctx* ctx, lj_batch* b, const float* x, const floa
         LJ_OK)
         return st;
     if (cudaMemsetAsync(b->d_counter, 0, 3 * sizeof(unsigned), s) != cudaSuccess) return LJ_ECUDA;
+    k_sys_walk<<<(unsigned)((b->nsys + 7) / 8), 256, 0, s>>>(b->d_sys, b->nsys, b->cell, b->offsets, (int)b->total_cells,
+                                                             b->walk);
+    if ((st = last_launch_status()) != LJ_OK) return st;
     const int T = b->cfg.threads, P = b->cfg.per_thread;
     if (T == 64)
         P == 1 ? launch_batched_pair<64, 1>(ctx, b, xyzi, energy, force)
@@ -645,7 +694,7 @@ static lj_status batch_graph(lj_ctx* ctx, lj_batch* b, const float* x, const flo
 
 // One plain lj_bin + lj_compute per system (the path the batched step replaces), each with the
 // single-system kernel of the walk the batched kernel takes for it (6: one target per lane, 1: the
-// cluster walk, 10: two targets per lane), so per-particle results are equal bit for bit.
+// cluster walk; of walk 4 the one that the device picks), so per-particle results are equal bit for bit.
 static lj_status batch_separate_one(lj_ctx* ctx, lj_batch* b, int s, const float* x, const float* y, const float* z,
                                     float* energy, float* force, int* index, lj_totals* totals);
 
@@ -654,7 +703,7 @@ static lj_status batch_separate(lj_ctx* ctx, lj_batch* b, const float* x, const 
     const lj_tuning saved = ctx->tuning;
     lj_status st = LJ_OK;
     for (int s = 0; s < b->nsys && st == LJ_OK; ++s) {
-        ctx->tuning.pair_kernel = b->sd[s].walk == 3 ? 10 : (b->sd[s].walk == 2 ? 1 : 6);
+        ctx->tuning.pair_kernel = b->sd[s].walk == 2 ? 1 : 6;
         st = batch_separate_one(ctx, b, s, x, y, z, energy, force, index, totals);
     }
     ctx->tuning = saved;
@@ -678,9 +727,23 @@ static lj_status batch_separate_one(lj_ctx* ctx, lj_batch* b, int s, const float
             k_add_offset<<<(sy.n + 255) / 256, 256, 0, ctx->stream>>>(index + f, sy.n, f);
             if ((st = last_launch_status()) != LJ_OK) return st;
         }
-        st = lj_compute(ctx, &b->grids[s], &sy.params, sy.n, reinterpret_cast<const float*>(b->xyzi + f),
-                        b->cell + f, off_s, LJ_ORDER_X, energy ? energy + f : nullptr,
-                        force ? force + 3 * (size_t)f : nullptr, totals ? totals + s : nullptr);
+        float* e = energy ? energy + f : nullptr;
+        float* fo = force ? force + 3 * (size_t)f : nullptr;
+        lj_totals* t = totals ? totals + s : nullptr;
+        const float* r = reinterpret_cast<const float*>(b->xyzi + f);
+        if (d.walk == 4 && sy.n > 0) {  // the walk chosen on the device: both kernels launched, one has work
+            k_one_walk<<<1, 32, 0, ctx->stream>>>(b->cell + f, off_s, sy.n, d.g.gx * d.g.gy * d.g.gz, b->walk + s);
+            if ((st = last_launch_status()) != LJ_OK) return st;
+            PairParams pp = d.pp;
+            pp.gate = b->walk + s;
+            pp.want = 2;
+            st = launch_pair_cluster(ctx, &b->grids[s], pp, sy.n, r, b->cell + f, off_s, true, e, fo, t, 0, sy.n);
+            if (st != LJ_OK) return st;
+            pp.want = 3;
+            st = launch_pair_pass(ctx, &b->grids[s], pp, sy.n, r, b->cell + f, off_s, true, e, fo, t, 0, sy.n);
+        } else {
+            st = lj_compute(ctx, &b->grids[s], &sy.params, sy.n, r, b->cell + f, off_s, LJ_ORDER_X, e, fo, t);
+        }
         if (st != LJ_OK) return st;
     }
     return LJ_OK;

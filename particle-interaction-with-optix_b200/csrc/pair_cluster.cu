@@ -20,6 +20,7 @@ __global__ void __launch_bounds__(32 * kCluWarps, kCluWarpsPerSm / kCluWarps)
     __shared__ __align__(16) CluSmem sm[kCluWarps];
     chain_wait();
     chain_next();
+    if (pp.gate && *pp.gate != pp.want) return;
     const int w = (int)(threadIdx.x >> 5);
     const long long first = a0 + (long long)blockIdx.x * stretch;
     double te = 0.0, tw = 0.0;

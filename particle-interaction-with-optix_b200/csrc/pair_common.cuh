@@ -22,6 +22,8 @@ struct PairParams {
     float e24;     // 24 eps
     float fscale;  // -24 eps / sigma^2: converts the accumulated sum of t * s2 * d into a force
     float slack;   // absolute rounding slack for cell planes and window ends
+    const int* gate = nullptr;  // if set, the launch has work only when *gate == want
+    int want = 0;
     int by_index = 0;  // 1: target k's outputs go to its original index (its record's fourth word), not k
 };
 

@@ -51,6 +51,7 @@ __global__ void __launch_bounds__(BLOCK, 8) k_pair_pass2(GridDev g, PairParams p
                                                              float* __restrict__ force, Partial* part,
                                                              unsigned* counter, lj_totals* totals, unsigned* status) {
     chain_wait();
+    if (pp.gate && *pp.gate != pp.want) return;
     const int ka = kb + 2 * (blockIdx.x * BLOCK + threadIdx.x);
     const bool activeA = ka < ke, activeB = ka + 1 < ke;
     const int ncell = g.gx * g.gy * g.gz;

@@ -87,3 +87,41 @@ def test_mixed_cluster_walk_edges(torch_cuda, ctx, name):
     fe, ee = ref.force_errors(np_(f)[:n]), ref.energy_errors(np_(e)[:n])
     assert fe["max_scaled"] <= FORCE_SCALED_TOL and fe["normwise"] <= FORCE_NORMWISE_TOL
     assert ee["max_scaled"] <= ENERGY_SCALED_TOL
+
+
+def test_batch_walk_chosen_by_occupied_cells(torch_cuda, ctx):
+    """Batched systems of 2 to 6 particles per cell of their whole grid take the cluster walk or the
+    two-target walk by the occupancy of the cells that hold particles, decided on the device: uniform and
+    shell systems, an empty and a one-particle one; the batched step, its graph replay and the per-system
+    launches agree bit for bit, and every pair count with lj_compute's."""
+    import ljcell
+
+    torch = torch_cuda
+    unit, box = ((0, 0, 0), (1, 1, 1)), ((-0.5,) * 3, (1.5,) * 3)
+    systems = []
+    for i, (kind, n, rc) in enumerate([("uniform", 3000, 0.1), ("shell", 20000, 0.11), ("uniform", 0, 0.1),
+                                       ("uniform", 5001, 0.1), ("shell", 9000, 0.15), ("uniform", 1, 0.3)]):
+        lo, hi = unit if kind == "uniform" else box
+        systems.append({"kind": kind, "n": n, "cutoff": rc, "lo": lo, "hi": hi, "seed": 40 + i})
+    b = ljcell.Batch(ctx, systems)
+    per_cell = [d["n"] / b.grid(s).ncells for s, d in enumerate(systems)]
+    assert all(2 <= per_cell[s] < 6 for s in (0, 1, 3, 4))
+    xyz = b.generate()
+    outs = []
+    for mode in ("plain", "separate", "graph", "graph"):
+        e, f, idx, tot = b.alloc_outputs()
+        b.run(*xyz, e, f, idx, tot, mode=mode)
+        ctx.sync()
+        outs.append((np_(e), np_(f), np_(idx), ljcell.totals_from_array(tot)))
+    for o in outs[1:]:
+        for x, y in zip(outs[0][:3], o[:3]):
+            assert np.array_equal(x.view(np.uint8), y.view(np.uint8))
+        assert [t["pairs"] for t in o[3]] == [t["pairs"] for t in outs[0][3]]
+    for s, d in enumerate(systems):
+        sl = slice(d["first"], d["first"] + d["n"])
+        g = b.grid(s)
+        q = ctx.bin(g, *(t[sl].contiguous() for t in xyz))
+        _, _, tot = ctx.compute(g, b.params(s), q)
+        ctx.sync()
+        assert ljcell.totals_from_tensor(tot)["pairs"] == outs[0][3][s]["pairs"], s
+    b.close()
