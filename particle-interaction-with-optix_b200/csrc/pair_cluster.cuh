@@ -76,7 +76,7 @@ __device__ __forceinline__ float rcp_count(float r2, float rc2, unsigned& np) {
     float r;
     asm("{\n\t.reg .pred p;\n\tsetp.lt.f32 p, %2, %3;\n\tmov.f32 %0, 0f00000000;\n\t@p rcp.approx.ftz.f32 %0, %2;\n\t"
         "@p add.u32 %1, %1, 1;\n\t}"
-        : "=f"(r), "+r"(np)
+        : "=&f"(r), "+r"(np)
         : "f"(r2), "f"(rc2));
     return r;
 }
