@@ -82,6 +82,22 @@ __device__ __forceinline__ float rcp_hit(bool hit, float r2) {
     return rcp_approx(hit ? r2 : __int_as_float(0x7f800000));
 }
 
+// r^-2 of a candidate inside the cutoff where m holds (counted in np), an exact 0 otherwise: the reciprocal
+// and the count run under the test's predicate, with no select in front of them; the values are rcp_hit's.
+// The walks that use it are bound by their instructions (2M particles, with the select and with the
+// predicate): kernel 12 at 0.5 / 3 / 10 per cell 157 / 276 / 615 and 153 / 269 / 594 us, kernel 10
+// 240 / 315 / 514 and 238 / 313 / 504, kernel 11 at 0.5 / 10 / 30 162 / 687 / 1669 and 160 / 668 / 1618,
+// kernel 6 at 2 / 10 / 30 301 / 583 / 1140 and 299 / 578 / 1127, the mixed form at 2 / 12 / 35
+// 328 / 635 / 1295 and 324 / 622 / 1266.
+__device__ __forceinline__ float rcp_count_if(float r2, float rc2, bool m, unsigned& np) {
+    float r;
+    asm("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 q, %4, 0;\n\tsetp.lt.and.f32 p, %2, %3, q;\n\tmov.f32 %0, 0f00000000;\n\t"
+        "@p rcp.approx.ftz.f32 %0, %2;\n\t@p add.u32 %1, %1, 1;\n\t}"
+        : "=&f"(r), "+r"(np)
+        : "f"(r2), "f"(rc2), "r"((int)m));
+    return r;
+}
+
 // Warp sums.
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll

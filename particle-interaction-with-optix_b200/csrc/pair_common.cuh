@@ -221,8 +221,9 @@ __device__ __forceinline__ void pair_target(const GridDev& g, const PairParams& 
         const float2 dy = __fadd2_rn(make_float2(q0.y, q1.y), npy);
         const float2 dz = __fadd2_rn(make_float2(q0.z, q1.z), npz);
         const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-        const bool in0 = r2.x < rc2, in1 = two && r2.y < rc2;
-        const float2 ir2 = make_float2(rcp_hit(in0, r2.x), rcp_hit(in1, r2.y));
+        float2 ir2;
+        ir2.x = rcp_count_if(r2.x, rc2, true, np);
+        ir2.y = rcp_count_if(r2.y, rc2, two, np);
         const float2 s2 = __fmul2_rn(sig2, ir2);
         const float2 s4 = __fmul2_rn(s2, s2);
         const float2 s6 = __fmul2_rn(s4, s2);
@@ -234,7 +235,6 @@ __device__ __forceinline__ void pair_target(const GridDev& g, const PairParams& 
         FX = __ffma2_rn(fs, dx, FX);
         FY = __ffma2_rn(fs, dy, FY);
         FZ = __ffma2_rn(fs, dz, FZ);
-        np += (unsigned)in0 + (unsigned)in1;
     }
     const float s12t = S12.x + S12.y, s6t = S6.x + S6.y;
     ea += s12t - s6t;

@@ -363,8 +363,9 @@ __device__ __forceinline__ void mix_walk_pass(const float2* __restrict__ rec, in
         const float2 dy = __fadd2_rn(f2(u0.x, u1.x), f2(a0 ? ntyA : ntyB, a1 ? ntyA : ntyB));
         const float2 dz = __fadd2_rn(f2(u0.y, u1.y), f2(a0 ? ntzA : ntzB, a1 ? ntzA : ntzB));
         const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-        const bool in0 = m0 && r2.x < rc2, in1 = m1 && r2.y < rc2;
-        const float2 ir2 = f2(rcp_hit(in0, r2.x), rcp_hit(in1, r2.y));
+        float2 ir2;
+        ir2.x = rcp_count_if(r2.x, rc2, m0, a.np);
+        ir2.y = rcp_count_if(r2.y, rc2, m1, a.np);
         const float2 s2n = __fmul2_rn(nsig2, ir2);
         const float2 s4 = __fmul2_rn(s2n, s2n);
         const float2 ns6 = __fmul2_rn(s4, s2n);
@@ -376,7 +377,6 @@ __device__ __forceinline__ void mix_walk_pass(const float2* __restrict__ rec, in
         px = __ffma2_rn(fsn, dx, px);
         py = __ffma2_rn(fsn, dy, py);
         pz = __ffma2_rn(fsn, dz, pz);
-        a.np += (unsigned)in0 + (unsigned)in1;
     }
     two_sum_add(a.se, a.ce, pe.x);
     two_sum_add(a.se, a.ce, pe.y);
@@ -499,8 +499,9 @@ __device__ __forceinline__ void mix_walk_pass2(const float2* __restrict__ rec, i
         const float2 dy = __fadd2_rn(f2(u.x, u.x), inA ? ntyA : ntyB);
         const float2 dz = __fadd2_rn(f2(u.y, u.y), inA ? ntzA : ntzB);
         const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-        const bool ia = ma && r2.x < rc2, ib = mb && r2.y < rc2;
-        const float2 ir2 = f2(rcp_hit(ia, r2.x), rcp_hit(ib, r2.y));
+        float2 ir2;
+        ir2.x = rcp_count_if(r2.x, rc2, ma, a.np);
+        ir2.y = rcp_count_if(r2.y, rc2, mb, a.np);
         const float2 s2n = __fmul2_rn(nsig2, ir2);
         const float2 s4 = __fmul2_rn(s2n, s2n);
         const float2 ns6 = __fmul2_rn(s4, s2n);
@@ -512,7 +513,6 @@ __device__ __forceinline__ void mix_walk_pass2(const float2* __restrict__ rec, i
         px = __ffma2_rn(fsn, dx, px);
         py = __ffma2_rn(fsn, dy, py);
         pz = __ffma2_rn(fsn, dz, pz);
-        a.np += (unsigned)ia + (unsigned)ib;
     };
     // two candidates per step: both records are loaded before either is evaluated
     for (int v = 0; v < maxL; v += 2) {

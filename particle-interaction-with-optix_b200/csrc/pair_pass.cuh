@@ -65,8 +65,9 @@ __device__ __forceinline__ void walk_pass(const float4* __restrict__ p, int k, i
         const float2 dy = __fadd2_rn(make_float2(q0.y, q1.y), npy);
         const float2 dz = __fadd2_rn(make_float2(q0.z, q1.z), npz);
         const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-        const bool in0 = m0 && r2.x < rc2, in1 = m1 && r2.y < rc2;
-        const float2 ir2 = make_float2(rcp_hit(in0, r2.x), rcp_hit(in1, r2.y));
+        float2 ir2;
+        ir2.x = rcp_count_if(r2.x, rc2, m0, a.np);
+        ir2.y = rcp_count_if(r2.y, rc2, m1, a.np);
         const float2 s2n = __fmul2_rn(nsig2, ir2);  // -s2
         const float2 s4 = __fmul2_rn(s2n, s2n);     // s2 * s2
         const float2 ns6 = __fmul2_rn(s4, s2n);     // -s6
@@ -78,7 +79,6 @@ __device__ __forceinline__ void walk_pass(const float4* __restrict__ p, int k, i
         a.fx = __ffma2_rn(fsn, dx, a.fx);
         a.fy = __ffma2_rn(fsn, dy, a.fy);
         a.fz = __ffma2_rn(fsn, dz, a.fz);
-        a.np += (unsigned)in0 + (unsigned)in1;
     }
 
 }
@@ -170,20 +170,6 @@ struct Pass2Acc {
     float2 e, w, fx, fy, fz;  // .x target a, .y target b
     unsigned np;
 };
-
-// r^-2 of an interacting candidate of a target that takes part (counted in np), an exact 0 otherwise: the
-// reciprocal and the count run under the test's predicate, with no select in front of them.  The walk is
-// bound by its instructions, so the two selects and adds a step show (both sides measured, 2M particles:
-// kernel 12 at 0.5 / 3 / 10 per cell 157 / 276 / 615 -> 153 / 269 / 594 us, kernel 10 240 / 315 / 514 ->
-// 238 / 313 / 504 us); the values are rcp_hit's.
-__device__ __forceinline__ float rcp_count_if(float r2, float rc2, bool m, unsigned& np) {
-    float r;
-    asm("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 q, %4, 0;\n\tsetp.lt.and.f32 p, %2, %3, q;\n\tmov.f32 %0, 0f00000000;\n\t"
-        "@p rcp.approx.ftz.f32 %0, %2;\n\t@p add.u32 %1, %1, 1;\n\t}"
-        : "=&f"(r), "+r"(np)
-        : "f"(r2), "f"(rc2), "r"((int)m));
-    return r;
-}
 
 // One packed evaluation of candidate q (index j) against targets (a, b), minus coordinates in nx/ny/nz.
 template <bool OWN>
