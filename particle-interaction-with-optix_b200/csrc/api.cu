@@ -37,6 +37,17 @@ lj_status grow(void** p, size_t* cap, size_t need) {
     return LJ_OK;
 }
 
+unsigned long long next_scratch_id() {
+    static std::atomic<unsigned long long> last{0};
+    return ++last;
+}
+
+lj_status grow_build(lj_ctx* ctx, void** p, size_t* cap, size_t need) {
+    if (need <= *cap && *p) return LJ_OK;
+    ctx->scratch_id = next_scratch_id();
+    return grow(p, cap, need);
+}
+
 lj_status last_launch_status() {
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? LJ_OK : LJ_ECUDA;
@@ -101,6 +112,7 @@ extern "C" lj_status lj_create(lj_ctx** out, int device, void* stream) {
     std::memset(c, 0, sizeof(*c));
     c->device = device;
     c->stream = static_cast<cudaStream_t>(stream);
+    c->scratch_id = next_scratch_id();
     if (cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
         delete c;
         return LJ_ECUDA;

@@ -372,6 +372,7 @@ struct lj_batch {
     cudaGraphExec_t exec = nullptr;
     const void* gkey[7] = {};
     unsigned gversion = ~0u;
+    unsigned long long gscratch = 0;  // scratch_id of the context at the capture
 };
 
 namespace ljc {
@@ -651,7 +652,10 @@ static lj_status batch_graph(lj_ctx* ctx, lj_batch* b, const float* x, const flo
             cudaEventCreateWithFlags(&b->ev_out, cudaEventDisableTiming) != cudaSuccess)
             return LJ_ECUDA;
     }
-    if (!b->exec || b->gversion != b->version || std::memcmp(key, b->gkey, sizeof(key)) != 0) {
+    // the captured step holds addresses of the caller's arrays, of the plan and of the context's build scratch: it is
+    // replayed only while all three are those of the capture
+    if (!b->exec || b->gversion != b->version || b->gscratch != ctx->scratch_id ||
+        std::memcmp(key, b->gkey, sizeof(key)) != 0) {
         if (b->exec) {
             cudaGraphExecDestroy(b->exec);
             b->exec = nullptr;
@@ -683,6 +687,7 @@ static lj_status batch_graph(lj_ctx* ctx, lj_batch* b, const float* x, const flo
         }
         std::memcpy(b->gkey, key, sizeof(key));
         b->gversion = b->version;
+        b->gscratch = ctx->scratch_id;
     }
     if (cudaEventRecord(b->ev_in, ctx->stream) != cudaSuccess ||
         cudaStreamWaitEvent(b->gstream, b->ev_in, 0) != cudaSuccess ||

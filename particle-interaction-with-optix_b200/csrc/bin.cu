@@ -547,7 +547,7 @@ static lj_status check_grid(const lj_grid* g, long long* ncells) {
 lj_status scan_prepare(lj_ctx* ctx, long long ncells) {
     const long long ntiles = (ncells + kScanTile - 1) / kScanTile;
     const size_t need = 256 + (size_t)(ntiles > 0 ? ntiles : 1) * sizeof(unsigned long long);
-    const lj_status s = grow(&ctx->scan_state, &ctx->scan_state_bytes, need);
+    const lj_status s = grow_build(ctx, &ctx->scan_state, &ctx->scan_state_bytes, need);
     if (s != LJ_OK) return s;
     return cudaMemsetAsync(ctx->scan_state, 0, need, ctx->stream) == cudaSuccess ? LJ_OK : LJ_ECUDA;
 }
@@ -621,10 +621,10 @@ static lj_status bin_scratch(lj_ctx* ctx, int n) {
         size_t c1 = ctx->part_cap * sizeof(int2), c2 = ctx->part_cap * sizeof(float4);
         // a failed growth has freed its old buffer: record the null pointer and a zero capacity
         // so that no freed buffer is used or freed again
-        s = grow(&p1, &c1, need * sizeof(int2));
+        s = grow_build(ctx, &p1, &c1, need * sizeof(int2));
         ctx->cell_ticket = static_cast<int2*>(p1);
         if (s == LJ_OK) {
-            s = grow(&p2, &c2, need * sizeof(float4));
+            s = grow_build(ctx, &p2, &c2, need * sizeof(float4));
             ctx->tmp4 = static_cast<float4*>(p2);
         }
         if (s != LJ_OK) {
@@ -637,7 +637,7 @@ static lj_status bin_scratch(lj_ctx* ctx, int n) {
     if (!ctx->large_cells || ctx->large_cap < large_need) {
         void* p = ctx->large_cells;
         size_t cap = ctx->large_cells ? sizeof(int) * (1 + ctx->large_cap) : 0;
-        s = grow(&p, &cap, sizeof(int) * (1 + large_need));
+        s = grow_build(ctx, &p, &cap, sizeof(int) * (1 + large_need));
         ctx->large_cells = static_cast<int*>(p);
         ctx->large_cap = s == LJ_OK ? large_need : 0;
         if (s != LJ_OK) return s;
@@ -842,7 +842,7 @@ extern "C" lj_status lj_test_scan_withheld_tile(lj_ctx* ctx, const int* counts, 
     if (!ctx || !counts || !offsets || ncells <= kScanTile || ncells > (long long)INT_MAX - 1) return LJ_EINVAL;
     const long long ntiles = (ncells + kScanTile - 1) / kScanTile;
     const size_t need = 256 + (size_t)ntiles * sizeof(unsigned long long);
-    lj_status s = grow(&ctx->scan_state, &ctx->scan_state_bytes, need);
+    lj_status s = grow_build(ctx, &ctx->scan_state, &ctx->scan_state_bytes, need);
     if (s != LJ_OK) return s;
     if (cudaMemsetAsync(ctx->scan_state, 0, need, ctx->stream) != cudaSuccess) return LJ_ECUDA;
     unsigned* counter = reinterpret_cast<unsigned*>(ctx->scan_state);

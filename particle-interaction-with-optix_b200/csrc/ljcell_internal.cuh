@@ -124,6 +124,8 @@ struct lj_ctx {
     cudaStream_t stream;
     int sm_count;
     unsigned* d_status;          // device status word
+    unsigned long long scratch_id;  // of the cell-grid build's buffers as they are now (grow_build): no two states,
+                                    // of this or of another context, share one
     // scratch, grown on demand
     void* scan_state;            // tile counter + tile status words
     size_t scan_state_bytes;
@@ -208,6 +210,10 @@ inline int grid_for(const lj_ctx* ctx, long long items, int per_block, int waves
 namespace ljc {
 // Host helpers shared by the .cu files (defined in api.cu).
 lj_status grow(void** p, size_t* cap, size_t need);
+// grow for the buffers of the cell-grid build (scan state, tickets, unsorted records, large cells), whose
+// addresses a captured batched step holds: a buffer that is replaced gives the context a new scratch_id.
+lj_status grow_build(lj_ctx* ctx, void** p, size_t* cap, size_t need);
+unsigned long long next_scratch_id();
 lj_status last_launch_status();
 // Cell-grid build stages (bin.cu), shared by lj_bin and the batched step.
 lj_status bin_prepare(lj_ctx* ctx, int n, long long nc, int* counts);
