@@ -5,7 +5,7 @@
 #include <cstring>
 #include <new>
 
-#include "ljcell_internal.cuh"
+#include "bin_common.cuh"
 
 namespace ljc {
 
@@ -121,6 +121,12 @@ extern "C" lj_status lj_create(lj_ctx** out, int device, void* stream) {
         cudaGetLastError();
         delete c;
         return LJ_ENOMEM;
+    }
+    const lj_status limits = bin_shared_limits();
+    if (limits != LJ_OK) {
+        cudaFree(c->d_status);
+        delete c;
+        return limits;
     }
     c->d_cand = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(c->d_status) + 64);
     *out = c;

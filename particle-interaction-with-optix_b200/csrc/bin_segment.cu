@@ -409,6 +409,25 @@ __global__ void __launch_bounds__(kSegThreads) k_bin_small(GridDev g, int ncell,
     if (bad) atomicOr(status, kFlagNonFinite);
 }
 
+// The limits of the kernels' dynamic shared memory on the current device, at the most that any build asks
+// for.  The limit belongs to the kernel on the device, not to a context: set per call to what that call
+// needs, one thread's smaller grid would make another thread's launch fail.
+lj_status bin_shared_limits() {
+    const auto raise = [](auto kernel, size_t bytes) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+    };
+    const size_t hist = kSegMax * sizeof(int), cells = kSegCells * sizeof(int);
+    const bool ok = raise(k_bin_small<LJ_ORDER_X>, (size_t)kSmallParticles * 18 + cells) &&
+                    raise(k_bin_small<LJ_ORDER_INDEX>, (size_t)kSmallParticles * 18 + cells) &&
+                    raise(k_seg_sort<LJ_ORDER_X, 256, kSegSmall, true>, (size_t)kSegSmall * 18 + cells) &&
+                    raise(k_seg_sort<LJ_ORDER_INDEX, 256, kSegSmall, true>, (size_t)kSegSmall * 18 + cells) &&
+                    raise(k_seg_sort<LJ_ORDER_X, 1024, kSegLarge, false>, (size_t)kSegLarge * 18 + cells) &&
+                    raise(k_seg_sort<LJ_ORDER_INDEX, 1024, kSegLarge, false>, (size_t)kSegLarge * 18 + cells) &&
+                    raise(k_seg_count, hist) && raise(k_seg_scatter, hist);
+    if (!ok) cudaGetLastError();
+    return ok ? LJ_OK : LJ_ECUDA;
+}
+
 bool small_bin_takes(const lj_ctx* ctx, int n, long long nc) {
     return n >= 1 && n <= kSmallParticles && nc <= kSegCells && ctx->tuning.scatter_passes == 0;
 }
@@ -419,8 +438,6 @@ lj_status launch_small_bin(lj_ctx* ctx, long long nc, int n, const float* x, con
     const auto kernel = order == LJ_ORDER_X ? k_bin_small<LJ_ORDER_X> : k_bin_small<LJ_ORDER_INDEX>;
     const size_t bytes = (size_t)kSmallParticles * 18 + (((size_t)nc * sizeof(int) + 15) & ~(size_t)15);
     const int vec = ((reinterpret_cast<uintptr_t>(counts) | reinterpret_cast<uintptr_t>(offsets)) & 15) == 0;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
-        return LJ_ECUDA;
     kernel<<<1, kSegThreads, bytes, ctx->stream>>>(g, (int)nc, x, y, z, stride, n, counts, offsets, vec, cells, so,
                                                    ctx->d_status);
     return last_launch_status();
@@ -452,9 +469,6 @@ static lj_status launch_seg_sorts(lj_ctx* ctx, const SegPlan& plan, long long nc
     const size_t cnt = std::max((size_t)16, sizeof(int) << plan.shift);
     const int vec = ((reinterpret_cast<uintptr_t>(counts) | reinterpret_cast<uintptr_t>(offsets)) & 15) == 0;
     const size_t b_small = (size_t)kSegSmall * 18 + cnt, b_large = (size_t)kSegLarge * 18 + cnt;
-    if (cudaFuncSetAttribute(small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b_small) != cudaSuccess ||
-        cudaFuncSetAttribute(large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b_large) != cudaSuccess)
-        return LJ_ECUDA;
     chain_launch(small, plan.nseg, 256, b_small, ctx->stream, g, (int)nc, n, plan.shift, plan.nseg, sc, ctx->tmp4, counts, offsets,
                                                     vec, cells, so, x, stride);
     lj_status s;
@@ -483,9 +497,6 @@ lj_status launch_segment_bin(lj_ctx* ctx, const SegPlan& plan, long long nc, int
     cudaStream_t st = ctx->stream;
     if (cudaMemsetAsync(p, 0, 256 + seg, st) != cudaSuccess) return LJ_ECUDA;
     const size_t hist = (size_t)plan.nseg * sizeof(int);
-    if (cudaFuncSetAttribute(k_seg_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist) != cudaSuccess ||
-        cudaFuncSetAttribute(k_seg_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist) != cudaSuccess)
-        return LJ_ECUDA;
     k_seg_count<<<blocks, kSegThreads, hist, st>>>(g, x, y, z, stride, n, plan.shift, plan.nseg, sc, ctx->d_status);
     if ((s = last_launch_status()) != LJ_OK) return s;
     // In passes of at most kSegRegion bytes of records, so that a run's 16-byte writes meet in L2 before
