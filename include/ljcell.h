@@ -184,7 +184,9 @@ LJ_API lj_status lj_cell_descriptors(lj_ctx* ctx, const int* offsets, long long 
  * executeSimulation (cudaLJ.cu:614-634): count, scan, descriptors and the
  * scatter of MoveParticlesToNewCells (cudaLJ.cu:441-471), made deterministic
  * (`order`).  Device pointers:
- *   in            positions as for lj_count_cells (stride 1 or 3)
+ *   in            positions as for lj_count_cells (stride 1 or 3); they may lie
+ *                 in sorted's x, y, z or in sorted_xyzi (binning in place): the
+ *                 last read of an input comes before the first sorted output
  *   counts        [ncells]        per-cell occupancy                (required)
  *   offsets       [ncells + 1]    exclusive prefix of counts        (required)
  *   cells         [ncells]        CellDescriptor view               (may be NULL)

@@ -218,14 +218,18 @@ __global__ void __launch_bounds__(kSegThreads) k_seg_scatter(const float* __rest
     }
 }
 
-// A record in shared memory: (y, z, original index, x as an unsigned integer of the same order, -0 as +0),
-// so that its last two words are the sort key of LJ_ORDER_X as one 64-bit integer.
-__device__ __forceinline__ unsigned x_key(float x) {
-    const unsigned u = __float_as_uint(x + 0.0f);
-    return u ^ ((unsigned)((int)u >> 31) | 0x80000000u);
+// A record in shared memory: (y, z, twice the original index plus one where x is -0, x as an unsigned integer
+// of the same order, -0 as +0), so that its last two words are the sort key of LJ_ORDER_X as one 64-bit
+// integer and hold every bit of x and of the index.
+__device__ __forceinline__ uint4 pack_record(const float4& r) {
+    const unsigned bits = __float_as_uint(r.x), u = r.x == 0.0f ? 0u : bits;
+    return make_uint4(__float_as_uint(r.y), __float_as_uint(r.z),
+                      2u * __float_as_uint(r.w) + (bits == 0x80000000u ? 1u : 0u),
+                      u ^ ((unsigned)((int)u >> 31) | 0x80000000u));
 }
-__device__ __forceinline__ float x_of_key(unsigned k) {
-    return __uint_as_float(k ^ ((unsigned)((int)~k >> 31) | 0x80000000u));
+__device__ __forceinline__ float4 unpack_record(const uint4& k) {
+    const unsigned u = (k.w ^ ((unsigned)((int)~k.w >> 31) | 0x80000000u)) | (k.z << 31);  // k.z odd: u is 0
+    return make_float4(__uint_as_float(u), __uint_as_float(k.x), __uint_as_float(k.y), __uint_as_float(k.z >> 1));
 }
 
 // One segment: its m records (at most CAP), load(i) the i-th, sorted to s0 on; its W cells from c0 on.
@@ -234,9 +238,8 @@ __device__ __forceinline__ float x_of_key(unsigned k) {
 template <int ORDER, int THREADS, int CAP, class Load>
 __device__ __forceinline__ void seg_sort(const GridDev& g, int c0, int W, int s0, int m, Load load,
                                          int* __restrict__ counts, int* __restrict__ offsets, bool vec,
-                                         lj_cell_desc* __restrict__ cells, const SortOut& so, const float* __restrict__ x, int stride,
-                                         uint4* s_rec, int* s_cnt,
-                                         unsigned short* s_cell) {
+                                         lj_cell_desc* __restrict__ cells, const SortOut& so, uint4* s_rec,
+                                         int* s_cnt, unsigned short* s_cell) {
     constexpr int PER = (CAP + THREADS - 1) / THREADS;
     __shared__ int s_sum[THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -325,7 +328,7 @@ __device__ __forceinline__ void seg_sort(const GridDev& g, int c0, int W, int s0
         if (u * THREADS + tid < m) {
             const int c = where[u] >> 16, at = s_cnt[c] + (where[u] & 0xffff);
             const float4 r = load(u * THREADS + tid);
-            s_rec[at] = make_uint4(__float_as_uint(r.y), __float_as_uint(r.z), __float_as_uint(r.w), x_key(r.x));
+            s_rec[at] = pack_record(r);
             s_cell[at] = (unsigned short)c;
         }
     __syncthreads();
@@ -344,16 +347,14 @@ __device__ __forceinline__ void seg_sort(const GridDev& g, int c0, int W, int s0
 #pragma unroll 4
             for (int j = e0; j < e1; ++j) rank += s_rec[j].z < k.z ? 1 : 0;
         }
-        float4 q = make_float4(x_of_key(k.w), __uint_as_float(k.x), __uint_as_float(k.y), __uint_as_float(k.z));
-        const int iq = (int)k.z;
-        if (q.x == 0.0f) q.x = __ldg(&x[(long long)iq * stride]);  // +0 or -0
+        const float4 q = unpack_record(k);
         const int slot = s0 + e0 + rank;
         so.out4[slot] = q;
         so.out_cell[s0 + i] = c0 + c;  // every slot of a cell holds its id, whatever the order inside the cell
         if (so.sx) so.sx[slot] = q.x;
         if (so.sy) so.sy[slot] = q.y;
         if (so.sz) so.sz[slot] = q.z;
-        if (so.sidx) so.sidx[slot] = iq;
+        if (so.sidx) so.sidx[slot] = __float_as_int(q.w);
     }
 }
 
@@ -362,7 +363,7 @@ template <int ORDER, int THREADS, int CAP, bool SMALL>
 __global__ void __launch_bounds__(THREADS, SMALL ? 6 : 1) k_seg_sort(GridDev g, int ncell, int n, int shift, int nseg, SegScratch sc,
                                                       const float4* __restrict__ tmp, int* __restrict__ counts,
                                                       int* __restrict__ offsets, int vec, lj_cell_desc* __restrict__ cells,
-                                                      SortOut so, const float* __restrict__ x, int stride) {
+                                                      SortOut so) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     uint4* s_rec = reinterpret_cast<uint4*>(s_raw);
     int* s_cnt = reinterpret_cast<int*>(s_raw + (size_t)CAP * 18);
@@ -377,7 +378,9 @@ __global__ void __launch_bounds__(THREADS, SMALL ? 6 : 1) k_seg_sort(GridDev g, 
         const int s0 = sc.start[b], m = sc.start[b + 1] - s0;
         if (m < 0 || m > CAP || s0 < 0 || s0 + m > n) continue;
         const int c0 = b << shift, W = min(1 << shift, ncell - c0);
-        seg_sort<ORDER, THREADS, CAP>(g, c0, W, s0, m, [&](int i) { return __ldcg(&tmp[s0 + i]); }, counts, offsets, vec != 0, cells, so, x, stride, s_rec, s_cnt, s_cell);
+        seg_sort<ORDER, THREADS, CAP>(
+            g, c0, W, s0, m, [&](int i) { return __ldcg(&tmp[s0 + i]); }, counts, offsets, vec != 0, cells, so, s_rec,
+            s_cnt, s_cell);
         if (!SMALL) __syncthreads();
     }
 }
@@ -405,7 +408,7 @@ __global__ void __launch_bounds__(kSegThreads) k_bin_small(GridDev g, int ncell,
             bad |= !(isfinite(r.x) && isfinite(r.y) && isfinite(r.z));
             return r;
         },
-        counts, offsets, vec != 0, cells, so, x, stride, s_rec, s_cnt, s_cell);
+        counts, offsets, vec != 0, cells, so, s_rec, s_cnt, s_cell);
     if (bad) atomicOr(status, kFlagNonFinite);
 }
 
@@ -462,19 +465,19 @@ SegPlan segment_plan(const lj_ctx* ctx, int n, long long nc) {
 
 template <int ORDER>
 static lj_status launch_seg_sorts(lj_ctx* ctx, const SegPlan& plan, long long nc, int n, const SegScratch& sc,
-                                  int* counts, int* offsets, lj_cell_desc* cells, const SortOut& so, const GridDev& g,
-                                  const float* x, int stride) {
+                                  int* counts, int* offsets, lj_cell_desc* cells, const SortOut& so,
+                                  const GridDev& g) {
     const auto small = k_seg_sort<ORDER, 256, kSegSmall, true>;
     const auto large = k_seg_sort<ORDER, 1024, kSegLarge, false>;
     const size_t cnt = std::max((size_t)16, sizeof(int) << plan.shift);
     const int vec = ((reinterpret_cast<uintptr_t>(counts) | reinterpret_cast<uintptr_t>(offsets)) & 15) == 0;
     const size_t b_small = (size_t)kSegSmall * 18 + cnt, b_large = (size_t)kSegLarge * 18 + cnt;
-    chain_launch(small, plan.nseg, 256, b_small, ctx->stream, g, (int)nc, n, plan.shift, plan.nseg, sc, ctx->tmp4, counts, offsets,
-                                                    vec, cells, so, x, stride);
+    chain_launch(small, plan.nseg, 256, b_small, ctx->stream, g, (int)nc, n, plan.shift, plan.nseg, sc, ctx->tmp4,
+                 counts, offsets, vec, cells, so);
     lj_status s;
     if ((s = last_launch_status()) != LJ_OK) return s;
-    chain_launch(large, std::min(ctx->sm_count, plan.nseg), 1024, b_large, ctx->stream, g, (int)nc, n, plan.shift, plan.nseg, sc,
-                                                                             ctx->tmp4, counts, offsets, vec, cells, so, x, stride);
+    chain_launch(large, std::min(ctx->sm_count, plan.nseg), 1024, b_large, ctx->stream, g, (int)nc, n, plan.shift,
+                 plan.nseg, sc, ctx->tmp4, counts, offsets, vec, cells, so);
     return last_launch_status();
 }
 
@@ -508,9 +511,8 @@ lj_status launch_segment_bin(lj_ctx* ctx, const SegPlan& plan, long long nc, int
                      ctx->d_status, s_lo, s_hi);
         if ((s = last_launch_status()) != LJ_OK) return s;
     }
-    return order == LJ_ORDER_X
-               ? launch_seg_sorts<LJ_ORDER_X>(ctx, plan, nc, n, sc, counts, offsets, cells, so, g, x, stride)
-               : launch_seg_sorts<LJ_ORDER_INDEX>(ctx, plan, nc, n, sc, counts, offsets, cells, so, g, x, stride);
+    return order == LJ_ORDER_X ? launch_seg_sorts<LJ_ORDER_X>(ctx, plan, nc, n, sc, counts, offsets, cells, so, g)
+                               : launch_seg_sorts<LJ_ORDER_INDEX>(ctx, plan, nc, n, sc, counts, offsets, cells, so, g);
 }
 
 }  // namespace ljc
