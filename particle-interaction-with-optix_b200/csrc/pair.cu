@@ -30,9 +30,8 @@ constexpr double kPairCell = 2.0;     // ... and below that, two targets per lan
 // targets per lane.  Measured, 2M uniform particles, two targets per lane -> warp per cell: 485 -> 348 us
 // at 8 per cell, 764 -> 437 at 16, 2495 -> 1463 at 64, but 291 -> 494 at 4 (the warps of thin cells spend
 // their time on the stencil's offsets).  Grids whose cells all run at once take it at any density: 10,000
-// particles at 4 per cell 45 -> 10 us, 1,000 at 8 per cell 49 -> 9.
+// particles at 4 per cell 47 -> 4.5 us, 1,000 at 8 per cell 45 -> 4.5, 100,000 on 8 cells 35 -> 4.5 ms.
 constexpr double kCompatCell = 6.0;
-constexpr int kCompatWarpsPerSm = 32;
 
 // Default pair kernel (measured on B200, pair stage, 2M uniform particles): the cluster walk (1) from
 // 6 particles per cell up (484 against 514 us for kernel 10 at 10 per cell, 401 against 367 at 5), the
@@ -330,7 +329,7 @@ extern "C" lj_status lj_compute_compat(lj_ctx* ctx, const lj_grid* g, int n, con
     if (n == 0) return LJ_OK;
     const double nc = (double)g->dim[0] * g->dim[1] * g->dim[2];
     if (n >= kCompatCell * nc || nc <= (double)ctx->sm_count * kCompatWarpsPerSm)
-        return launch_compat_cells(ctx, g, n, sorted_xyzi, offsets, v);
+        return launch_compat_cells(ctx, g, n, sorted_xyzi, sorted_cell, offsets, v);
     chain_launch(k_pair_compat, (n + 2 * kPairThreads - 1) / (2 * kPairThreads), kPairThreads, 0, ctx->stream, to_dev(*g),
                  reinterpret_cast<const float4*>(sorted_xyzi), sorted_cell, offsets, n, v, ctx->d_status);
     return last_launch_status();

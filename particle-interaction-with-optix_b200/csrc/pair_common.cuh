@@ -258,7 +258,9 @@ lj_status launch_pair_cluster(lj_ctx* ctx, const lj_grid* g, const PairParams& p
                               const int* cs, const int* off, bool xwin, float* energy, float* force,
                               lj_totals* totals, int kb, int ke);
 // Reference law, one warp per cell (pair_compat.cu).
-lj_status launch_compat_cells(lj_ctx* ctx, const lj_grid* g, int n, const float* xyzi, const int* off, float* v);
+constexpr int kCompatWarpsPerSm = 32;
+lj_status launch_compat_cells(lj_ctx* ctx, const lj_grid* g, int n, const float* xyzi, const int* cell_id,
+                              const int* off, float* v);
 // Exclusive scan of counts[ncells] into offsets[0..ncells] on the context's stream (bin.cu).
 lj_status launch_scan(lj_ctx* ctx, const int* counts, long long ncells, int* offsets);
 // The same in two steps, for a caller that has kernels to launch between the scan's memset and the scan;

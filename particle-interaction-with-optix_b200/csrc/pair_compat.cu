@@ -8,12 +8,21 @@
 // coordinate, and what a step loads serves 16 targets.  The cell's own particles are evaluated apart,
 // where the mask j != k belongs.
 //
+// A warp takes at most a chunk of its cell's targets, 64 or, on few cells, 16; the rest of a crowded cell goes to
+// other warps, so that the time follows the number of targets and not the fullest cell.  Measured on B200, one
+// warp for all of a cell's targets -> chunks (two targets per lane, k_pair_compat): 10,000 particles in one cell
+// 155 ms -> 0.26 (1.22), 100,000 on 27 cells 216 -> 2.55 (15.7), 1,000,000 with 20,000 in one cell 634 -> 2.0
+// (2.9); and on evenly filled cells, where the search for crowded ones costs, 1M at 8 per cell 168 -> 171 us,
+// 4.2M at 16 902 -> 918.  In a launch of its own that search costs 6 us there, but the crowded cells' first
+// chunks then run alone (droplets up to twice as long).
+//
 // What bounds it: 11 paired operations and two reciprocal square roots per two evaluations, about 25
 // cycles per 64 evaluations by register reads and by the FMA pipe (22); at 16 per cell that is two
-// thirds of the 0.91 ms that 4.2M particles take on B200 (1.53 ms with two targets per lane; 0.96 at 6
-// blocks per SM and 76 registers instead of 8 and 64).  k_pair_compat (pair.cu), two
-// targets of possibly different cells per lane, masks every candidate against both targets' cells and
-// ranges and duplicates each coordinate for them.
+// thirds of the 0.92 ms that 4.2M particles take on B200 (1.52 ms with two targets per lane; 6 blocks per SM and
+// 76 registers instead of 8 and 64 take 6% longer).  k_pair_compat (pair.cu), two targets of possibly different cells
+// per lane, masks every candidate against both targets' cells and ranges and duplicates each coordinate
+// for them.
+#include <algorithm>
 #include <climits>
 
 #include "pair_common.cuh"
@@ -66,19 +75,12 @@ __device__ __forceinline__ void cell_walk(const CellSmem& sm, int cnt, int group
     }
 }
 
-__global__ void __launch_bounds__(32 * kCellWarps, 8) k_compat_cells(GridDev g, const float4* __restrict__ p,
-                                                                     const int* __restrict__ off, int n,
-                                                                     float* __restrict__ v) {
-    __shared__ __align__(16) CellSmem smem[kCellWarps];
-    chain_wait();
-    CellSmem& sm = smem[threadIdx.x >> 5];
+// Evaluates the targets [t0, t1) of cell c, which holds [cs, ce) (one warp, all lanes).
+__device__ __forceinline__ void cell_targets(const GridDev& g, const float4* __restrict__ p, const int* __restrict__ off,
+                                             int n, int c, int cs, int ce, int t0, int t1, CellSmem& sm,
+                                             float* __restrict__ v) {
     const int lane = (int)(threadIdx.x & 31u), t = lane % kCellLanes, group = lane / kCellLanes;
     const unsigned below = lanemask_lt();
-    const long long cell = (long long)blockIdx.x * kCellWarps + (threadIdx.x >> 5);
-    if (cell >= (long long)g.gx * g.gy * g.gz) return;
-    const int c = (int)cell;
-    const int cs = min(max(__ldg(&off[c]), 0), n), ce = min(max(__ldg(&off[c + 1]), cs), n);
-    if (cs == ce) return;
     // the stencil's ranges: lane r < 9 reads row r; the own row's parts before and after the cell
     int T, nr;
     {
@@ -113,8 +115,8 @@ __global__ void __launch_bounds__(32 * kCellWarps, 8) k_compat_cells(GridDev g, 
     }
     const int4 rng = lane < nr ? sm.range[lane] : make_int4(INT_MAX, 0, 0, 0);
     bool staged = false;  // the whole list is in shared memory already
-    for (int k0 = cs; k0 < ce; k0 += kCellLanes * kCellDeep) {
-        const int m = min(ce - k0, kCellLanes * kCellDeep), deep = (m + kCellLanes - 1) / kCellLanes;
+    for (int k0 = t0; k0 < t1; k0 += kCellLanes * kCellDeep) {
+        const int m = min(t1 - k0, kCellLanes * kCellDeep), deep = (m + kCellLanes - 1) / kCellLanes;
         float2 nx[kCellDeep], ny[kCellDeep], nz[kCellDeep], pot[kCellDeep];
 #pragma unroll
         for (int q = 0; q < kCellDeep; ++q) {
@@ -179,15 +181,72 @@ __global__ void __launch_bounds__(32 * kCellWarps, 8) k_compat_cells(GridDev g, 
 #pragma unroll
             for (int o = kCellLanes; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
             const int k = k0 + t + kCellLanes * q;
-            if (group == 0 && k < ce) v[k] = 4.0f * s;
+            if (group == 0 && k < t1) v[k] = 4.0f * s;
         }
     }
 }
 
-lj_status launch_compat_cells(lj_ctx* ctx, const lj_grid* g, int n, const float* xyzi, const int* off, float* v) {
+// Work items: the first `chunk` targets of every cell, one warp each, and the chunks beyond them of cells that
+// hold more, which the launch's first `finders` warps look for.  Window q of the sorted targets, [q chunk,
+// (q + 1) chunk), holds the start of at most one such chunk, and one of the cell that holds the window's first
+// target; a finder takes every finders-th window, so the chunks of one crowded cell go to different warps.  The
+// finders also look at every target's cell id: one outside the grid is reported.
+__global__ void __launch_bounds__(32 * kCellWarps, 8) k_compat_cells(GridDev g, const float4* __restrict__ p,
+                                                                     const int* __restrict__ cell_id,
+                                                                     const int* __restrict__ off, int n, int chunk,
+                                                                     int windows, int finders, float* __restrict__ v,
+                                                                     unsigned* status) {
+    __shared__ __align__(16) CellSmem smem[kCellWarps];
+    chain_wait();
+    const int lane = (int)(threadIdx.x & 31u);
+    const int ncell = g.gx * g.gy * g.gz;
+    const long long warp = (long long)blockIdx.x * kCellWarps + (threadIdx.x >> 5);
+    int c = 0, cs = 0, ce = 0, t0 = 0;
+    if (warp < finders) {
+        const long long q = warp + (long long)lane * finders;
+        if (q < windows) {
+            const int k = (int)(q * chunk);
+            c = __ldg(&cell_id[k]);
+            if (c >= 0 && c < ncell) {
+                cs = min(max(__ldg(&off[c]), 0), k);
+                ce = min(__ldg(&off[c + 1]), n);
+                const long long start = cs + (long long)(k - cs + chunk - 1) / chunk * chunk;
+                t0 = start > cs ? (int)min(start, (long long)INT_MAX) : ce;
+            }
+        }
+        const int hi = (int)((long long)n * (warp + 1) / finders);
+        bool bad = false;
+#pragma unroll 4
+        for (int k = (int)((long long)n * warp / finders) + lane; k < hi; k += 32) {
+            const int id = __ldg(&cell_id[k]);
+            bad |= id < 0 || id >= ncell;
+        }
+        if (bad) atomicOr(status, kFlagRange);
+    } else if (warp - finders < ncell && lane == 0) {
+        c = (int)(warp - finders);
+        t0 = cs = min(max(__ldg(&off[c]), 0), n);
+        ce = min(__ldg(&off[c + 1]), n);
+    }
+    for (unsigned todo = __ballot_sync(0xffffffffu, t0 < ce); todo; todo &= todo - 1) {
+        const int src = __ffs(todo) - 1, start = __shfl_sync(0xffffffffu, t0, src), end = __shfl_sync(0xffffffffu, ce, src);
+        cell_targets(g, p, off, n, __shfl_sync(0xffffffffu, c, src), __shfl_sync(0xffffffffu, cs, src), end, start,
+                     end - start < chunk ? end : start + chunk, smem[threadIdx.x >> 5], v);
+    }
+}
+
+lj_status launch_compat_cells(lj_ctx* ctx, const lj_grid* g, int n, const float* xyzi, const int* cell_id,
+                              const int* off, float* v) {
     const long long nc = (long long)g->dim[0] * g->dim[1] * g->dim[2];
-    chain_launch(k_compat_cells, (unsigned)((nc + kCellWarps - 1) / kCellWarps), 32 * kCellWarps, 0, ctx->stream,
-                 to_dev(*g), reinterpret_cast<const float4*>(xyzi), off, n, v);
+    // A chunk of four rounds where the cells alone fill the GPU, of one round where they do not; as many finders as
+    // run at once, each with at most a window per lane.
+    const long long warps = (long long)ctx->sm_count * kCompatWarpsPerSm;
+    const int chunk = kCellLanes * kCellDeep * (nc >= warps ? 4 : 1);
+    const long long windows = ((long long)n + chunk - 1) / chunk;
+    const long long per = std::min(32LL, std::max(1LL, windows / warps));
+    const long long finders = (windows + per - 1) / per;
+    chain_launch(k_compat_cells, (unsigned)((nc + finders + kCellWarps - 1) / kCellWarps), 32 * kCellWarps, 0,
+                 ctx->stream, to_dev(*g), reinterpret_cast<const float4*>(xyzi), cell_id, off, n, chunk, (int)windows,
+                 (int)finders, v, ctx->d_status);
     return last_launch_status();
 }
 
