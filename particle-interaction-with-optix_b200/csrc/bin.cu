@@ -273,7 +273,6 @@ __device__ __forceinline__ void emit(const SortOut& o, long long slot, float4 r,
 }
 
 constexpr long long kScatterRegion = 56LL << 20;  // bytes of tmp4 one scatter pass writes (L2 holds 126 MB)
-constexpr int kRankMax = 512;    // cells up to this size are ranked record by record
 constexpr int kLargeCapMin = 4096;
 
 // One thread per record of the scattered (cell-grouped, unordered within a cell) array.  The

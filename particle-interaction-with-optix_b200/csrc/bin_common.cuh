@@ -15,6 +15,8 @@ __device__ __forceinline__ bool key_less(float xa, int ia, float xb, int ib) {
     return ia < ib;
 }
 
+constexpr int kRankMax = 512;  // cells up to this size are ranked record by record, larger ones are sorted
+
 struct SortOut {
     float4* out4;
     int* out_cell;

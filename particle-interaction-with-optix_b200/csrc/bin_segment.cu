@@ -232,6 +232,37 @@ __device__ __forceinline__ float4 unpack_record(const uint4& k) {
     return make_float4(__uint_as_float(u), __uint_as_float(k.x), __uint_as_float(k.y), __uint_as_float(k.z >> 1));
 }
 
+// Sorts the m records of one crowded cell by key, the whole block: a bitonic network over any number of records.
+// Each run of k starts with the mirrored comparison, so every comparison is ascending and the places past the
+// end, which count as greater, are never exchanged with.
+template <int ORDER, int THREADS>
+__device__ __noinline__ void cell_sort(uint4* rec, int m) {
+    const auto exchange = [&](int lo, int hi) {
+        if (hi >= m) return;
+        const uint4 a = rec[lo], b = rec[hi];
+        const bool less = ORDER == LJ_ORDER_X ? (b.w < a.w || (b.w == a.w && b.z < a.z)) : b.z < a.z;
+        if (less) {
+            rec[lo] = b;
+            rec[hi] = a;
+        }
+    };
+    for (int lk = 1; (1 << (lk - 1)) < m; ++lk) {
+        const int pairs = ((m + (1 << lk) - 1) >> lk) << (lk - 1);
+        for (int q = threadIdx.x; q < pairs; q += THREADS) {
+            const int run = (q >> (lk - 1)) << lk, at = q & ((1 << (lk - 1)) - 1);
+            exchange(run + at, run + (1 << lk) - 1 - at);
+        }
+        __syncthreads();
+        for (int lj = lk - 2; lj >= 0; --lj) {
+            for (int q = threadIdx.x; q < pairs; q += THREADS) {
+                const int lo = ((q >> lj) << (lj + 1)) + (q & ((1 << lj) - 1));
+                exchange(lo, lo + (1 << lj));
+            }
+            __syncthreads();
+        }
+    }
+}
+
 // One segment: its m records (at most CAP), load(i) the i-th, sorted to s0 on; its W cells from c0 on.
 // The records are read twice (the second time from L2) rather than held in registers, which would halve
 // the blocks per SM.
@@ -242,6 +273,7 @@ __device__ __forceinline__ void seg_sort(const GridDev& g, int c0, int W, int s0
                                          int* s_cnt, unsigned short* s_cell) {
     constexpr int PER = (CAP + THREADS - 1) / THREADS;
     __shared__ int s_sum[THREADS / 32];
+    __shared__ int s_crowded, s_list[CAP / (kRankMax + 1)];  // cells of more than kRankMax records
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     vec = vec && (W & 3) == 0;
     if (m == 0) {
@@ -261,6 +293,7 @@ __device__ __forceinline__ void seg_sort(const GridDev& g, int c0, int W, int s0
         return;
     }
     for (int c = 4 * tid; c < W; c += 4 * THREADS) *reinterpret_cast<int4*>(s_cnt + c) = make_int4(0, 0, 0, 0);
+    if (tid == 0) s_crowded = 0;
     __syncthreads();
     int where[PER];  // cell << 16 | ticket
 #pragma unroll
@@ -268,7 +301,9 @@ __device__ __forceinline__ void seg_sort(const GridDev& g, int c0, int W, int s0
         if (u * THREADS + tid < m) {
             const float4 r = load(u * THREADS + tid);
             const int c = min(max(cell_of(g, r.x, r.y, r.z) - c0, 0), W - 1);
-            where[u] = (c << 16) | atomicAdd(&s_cnt[c], 1);
+            const int ticket = atomicAdd(&s_cnt[c], 1);
+            if (ticket == kRankMax) s_list[atomicAdd(&s_crowded, 1)] = c;
+            where[u] = (c << 16) | ticket;
         }
     __syncthreads();
     // exclusive prefix of the cell counts in place: each warp takes a run of cells, 128 at a time
@@ -332,13 +367,19 @@ __device__ __forceinline__ void seg_sort(const GridDev& g, int c0, int W, int s0
             s_cell[at] = (unsigned short)c;
         }
     __syncthreads();
-    // a record's rank is the number of its cell's records with a smaller key
+    for (int l = 0; l < s_crowded; ++l) {
+        const int c = s_list[l], e0 = s_cnt[c];
+        cell_sort<ORDER, THREADS>(s_rec + e0, (c + 1 < W ? s_cnt[c + 1] : m) - e0);
+    }
+    // a record's rank is the number of its cell's records with a smaller key, its place in a sorted cell
     for (int i = tid; i < m; i += THREADS) {
         const uint4 k = s_rec[i];
         const int c = s_cell[i];
         const int e0 = s_cnt[c], e1 = c + 1 < W ? s_cnt[c + 1] : m;
         int rank = 0;
-        if (ORDER == LJ_ORDER_X) {
+        if (e1 - e0 > kRankMax) {
+            rank = i - e0;
+        } else if (ORDER == LJ_ORDER_X) {
             const unsigned long long key = ((unsigned long long)k.w << 32) | k.z;
             const unsigned long long* kj = reinterpret_cast<const unsigned long long*>(s_rec + e0) + 1;
 #pragma unroll 4
