@@ -341,7 +341,9 @@ __global__ void __launch_bounds__(256) k_cell_rank(const float4* __restrict__ tm
 // Cells larger than kRankMax (rare: clustered or degenerate inputs): one
 // CTA per cell sorts 2048-record chunks in shared memory (bitonic network),
 // then merges runs pairwise, each record finding its place in the partner run
-// by binary search; ping-pong between the cell's tmp and out ranges.
+// by binary search; ping-pong between the cell's tmp and out ranges.  One block per SM, and chained behind
+// k_cell_rank, so it asks for kOneBlockPerSm (3M particles, a third of them in one corner: build 683 us with two
+// blocks on half of the SMs, 482 with one on each).
 template <int ORDER>
 __device__ __forceinline__ bool rec_less(const float4& a, const float4& b) {
     return key_less<ORDER>(a.x, __float_as_int(a.w), b.x, __float_as_int(b.w));
@@ -712,8 +714,16 @@ static lj_status ticket_finish(lj_ctx* ctx, long long nc, int n, const float* x,
                  ctx->large_cells, lcap, ctx->d_status, gate);
     if ((s = last_launch_status()) != LJ_OK) return s;
     const auto sort = order == LJ_ORDER_X ? k_large_sort<LJ_ORDER_X> : k_large_sort<LJ_ORDER_INDEX>;
-    chain_launch(sort, ctx->sm_count, 1024, 0, st, ctx->tmp4, offsets, n, so, ctx->large_cells, lcap);
+    chain_launch(sort, ctx->sm_count, 1024, kOneBlockPerSm, st, ctx->tmp4, offsets, n, so, ctx->large_cells, lcap);
     return last_launch_status();
+}
+
+bool large_sort_shared_limit() {
+    const auto raise = [](auto kernel) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOneBlockPerSm) ==
+               cudaSuccess;
+    };
+    return raise(k_large_sort<LJ_ORDER_X>) && raise(k_large_sort<LJ_ORDER_INDEX>);
 }
 
 static SortOut sort_out(float* sorted_xyzi, int* sorted_cell, const lj_particles* sorted) {

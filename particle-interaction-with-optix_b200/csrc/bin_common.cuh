@@ -38,8 +38,9 @@ lj_status launch_segment_bin(lj_ctx* ctx, const SegPlan& plan, long long nc, int
                              const float* z, int stride, lj_order order, int* counts, int* offsets,
                              lj_cell_desc* cells, const SortOut& so, const GridDev& g, const unsigned** gate);
 
-// Sets what the kernels of both need on the current device; lj_create calls it.
+// Sets what the build's kernels need on the current device; lj_create calls it.
 lj_status bin_shared_limits();
+bool large_sort_shared_limit();  // bin.cu's part of it
 
 // A small system binned by one block in one launch.
 bool small_bin_takes(const lj_ctx* ctx, int n, long long nc);

@@ -461,13 +461,14 @@ lj_status bin_shared_limits() {
         return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
     };
     const size_t hist = kSegMax * sizeof(int), cells = kSegCells * sizeof(int);
+    static_assert(kSegMax * sizeof(int) <= kOneBlockPerSm, "k_seg_scatter's slots");
     const bool ok = raise(k_bin_small<LJ_ORDER_X>, (size_t)kSmallParticles * 18 + cells) &&
                     raise(k_bin_small<LJ_ORDER_INDEX>, (size_t)kSmallParticles * 18 + cells) &&
                     raise(k_seg_sort<LJ_ORDER_X, 256, kSegSmall, true>, (size_t)kSegSmall * 18 + cells) &&
                     raise(k_seg_sort<LJ_ORDER_INDEX, 256, kSegSmall, true>, (size_t)kSegSmall * 18 + cells) &&
                     raise(k_seg_sort<LJ_ORDER_X, 1024, kSegLarge, false>, (size_t)kSegLarge * 18 + cells) &&
                     raise(k_seg_sort<LJ_ORDER_INDEX, 1024, kSegLarge, false>, (size_t)kSegLarge * 18 + cells) &&
-                    raise(k_seg_count, hist) && raise(k_seg_scatter, hist);
+                    raise(k_seg_count, hist) && raise(k_seg_scatter, kOneBlockPerSm) && large_sort_shared_limit();
     if (!ok) cudaGetLastError();
     return ok ? LJ_OK : LJ_ECUDA;
 }
@@ -548,7 +549,7 @@ lj_status launch_segment_bin(lj_ctx* ctx, const SegPlan& plan, long long nc, int
     const long long passes = std::max(1LL, std::min(8LL, ((long long)n * 16 + kSegRegion - 1) / kSegRegion));
     for (long long q = 0; q < passes; ++q) {
         const int s_lo = (int)(plan.nseg * q / passes), s_hi = (int)(plan.nseg * (q + 1) / passes);
-        chain_launch(k_seg_scatter, blocks, kSegThreads, hist, st, x, y, z, stride, n, plan.nseg, sc, ctx->tmp4,
+        chain_launch(k_seg_scatter, blocks, kSegThreads, kOneBlockPerSm, st, x, y, z, stride, n, plan.nseg, sc, ctx->tmp4,
                      ctx->d_status, s_lo, s_hi);
         if ((s = last_launch_status()) != LJ_OK) return s;
     }

@@ -197,6 +197,11 @@ inline void chain_launch(void (*kernel)(P...), unsigned grid, unsigned block, si
     cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
 
+// Dynamic shared memory of a chained kernel of one block per SM: more than half of an SM's, so that no SM takes
+// two.  Scheduled while its predecessor's blocks still run, such a kernel would otherwise put two blocks on the
+// SMs that come free first and none on others.
+constexpr size_t kOneBlockPerSm = 116 << 10;
+
 // Blocks for a grid-stride loop over `items`: enough for every item, at most `waves` per SM.
 inline int grid_for(const lj_ctx* ctx, long long items, int per_block, int waves = 8) {
     long long b = (items + per_block - 1) / per_block;
