@@ -21,7 +21,7 @@ namespace ljc {
 
 // A kernel of the ticket path behind the segment path's gate (bin_segment.cu): it has work only when
 // the gate is open (nonzero); without a gate it always has.
-__device__ __forceinline__ bool closed(const unsigned* gate) { return gate && __ldg(gate) == 0u; }
+__device__ __forceinline__ bool closed(const unsigned* gate) { return gate && *gate == 0u; }
 
 // ---------------------------------------------------------------- counting
 // One thread per particle, grid-stride by whole warps.  Lanes that share a
@@ -33,7 +33,7 @@ template <bool TICKETS>
 __global__ void __launch_bounds__(256) k_count(GridDev g, const float* __restrict__ x, const float* __restrict__ y,
                                                const float* __restrict__ z, int stride, int n,
                                                int* __restrict__ counts, int2* __restrict__ ct,
-                                               unsigned* status, const unsigned* __restrict__ gate) {
+                                               unsigned* status, const unsigned* gate) {
     chain_wait();
     chain_next();
     if (closed(gate)) return;
@@ -82,11 +82,11 @@ __device__ __forceinline__ void st_state(unsigned long long* p, unsigned long lo
     *reinterpret_cast<volatile unsigned long long*>(p) = v;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan(const int* __restrict__ counts, int* __restrict__ offsets,
+__global__ void __launch_bounds__(kScanThreads) k_scan(const int* counts, int* __restrict__ offsets,
                                                        long long n, long long ntiles,
                                                        unsigned long long* tile_state, unsigned* tile_counter,
                                                        int vec_ok, unsigned* status,
-                                                       const unsigned* __restrict__ gate = nullptr) {
+                                                       const unsigned* gate = nullptr) {
     chain_wait();
     chain_next();
     if (closed(gate)) return;
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const int* __restrict__ c
     if (full) {
 #pragma unroll
         for (int it = 0; it < kScanIters; ++it) {
-            const int4 q = __ldg(reinterpret_cast<const int4*>(counts + wbase + it * 128 + lane * 4));
+            const int4 q = *reinterpret_cast<const int4*>(counts + wbase + it * 128 + lane * 4);
             v[it][0] = q.x;
             v[it][1] = q.y;
             v[it][2] = q.z;
@@ -223,9 +223,9 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const int* __restrict__ c
 // leave L2 as whole lines instead of as partial sectors.
 __global__ void __launch_bounds__(256) k_scatter(const float* __restrict__ x, const float* __restrict__ y,
                                                  const float* __restrict__ z, int stride, int n,
-                                                 const int2* __restrict__ ct, const int* __restrict__ offsets,
+                                                 const int2* ct, const int* offsets,
                                                  float4* __restrict__ tmp, unsigned* status, int c_lo, int c_hi,
-                                                 const unsigned* __restrict__ gate = nullptr) {
+                                                 const unsigned* gate = nullptr) {
     chain_wait();
     chain_next();
     if (closed(gate)) return;
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(256) k_scatter(const float* __restrict__ x, co
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const long long i = i0 + u * step;
-            c[u] = i < n ? __ldg(&ct[i]) : make_int2(0, 0);
+            c[u] = i < n ? ct[i] : make_int2(0, 0);
         }
         long long slot[U];
         float px[U], py[U], pz[U];
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(256) k_scatter(const float* __restrict__ x, co
         for (int u = 0; u < U; ++u) {
             const long long i = i0 + u * step;
             mine[u] = i < n && c[u].x >= c_lo && c[u].x < c_hi;
-            slot[u] = mine[u] ? (long long)__ldg(&offsets[c[u].x]) + c[u].y : -1;
+            slot[u] = mine[u] ? (long long)offsets[c[u].x] + c[u].y : -1;
             px[u] = mine[u] ? __ldg(&x[i * stride]) : 0.f;
             py[u] = mine[u] ? __ldg(&y[i * stride]) : 0.f;
             pz[u] = mine[u] ? __ldg(&z[i * stride]) : 0.f;
@@ -283,11 +283,11 @@ constexpr int kLargeCapMin = 4096;
 // is written at offset + rank.  Every lane is busy whatever the cell sizes.  Cells above kRankMax
 // go to a list handled by k_large_sort (registered by the thread of the cell's first slot).
 template <int ORDER>
-__global__ void __launch_bounds__(256) k_cell_rank(const float4* __restrict__ tmp, const int* __restrict__ offsets,
+__global__ void __launch_bounds__(256) k_cell_rank(const float4* tmp, const int* offsets,
                                                    GridDev g, const BinSys* __restrict__ sys,
                                                    const int* __restrict__ firsts, int nsys, int n, SortOut so,
                                                    int* large, int large_cap, unsigned* status,
-                                                   const unsigned* __restrict__ gate) {
+                                                   const unsigned* gate) {
     chain_wait();
     chain_next();
     if (closed(gate)) return;
@@ -309,8 +309,8 @@ __global__ void __launch_bounds__(256) k_cell_rank(const float4* __restrict__ tm
             c = sys[lo].cell_base + cell_of(sys[lo].g, r.x, r.y, r.z);
         }
         so.out_cell[s] = c;  // every slot of a cell holds its id, whatever the order inside the cell
-        const int o0 = min(max(__ldg(&offsets[c]), 0), n);
-        const int o1 = min(max(__ldg(&offsets[c + 1]), o0), n);
+        const int o0 = min(max(offsets[c], 0), n);
+        const int o1 = min(max(offsets[c + 1], o0), n);
         const int m = o1 - o0;
         if (m > kRankMax) {
             if (s == o0) {
@@ -350,8 +350,8 @@ __device__ __forceinline__ bool rec_less(const float4& a, const float4& b) {
 }
 
 template <int ORDER>
-__global__ void __launch_bounds__(1024) k_large_sort(float4* __restrict__ tmp, const int* __restrict__ offsets,
-                                                     int n, SortOut so, const int* __restrict__ large,
+__global__ void __launch_bounds__(1024) k_large_sort(float4* __restrict__ tmp, const int* offsets,
+                                                     int n, SortOut so, const int* large,
                                                      int large_cap) {
     chain_wait();
     chain_next();
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(1024) k_large_sort(float4* __restrict__ tmp, c
 }
 
 // Zeroes counts behind the gate.
-__global__ void __launch_bounds__(256) k_zero(int* __restrict__ v, long long n, const unsigned* __restrict__ gate) {
+__global__ void __launch_bounds__(256) k_zero(int* __restrict__ v, long long n, const unsigned* gate) {
     chain_wait();
     chain_next();
     if (closed(gate)) return;
@@ -429,9 +429,9 @@ __global__ void __launch_bounds__(256) k_zero(int* __restrict__ v, long long n, 
 }
 
 // ---------------------------------------------------------------- descriptors / candidates
-__global__ void __launch_bounds__(256) k_descriptors(const int* __restrict__ offsets, long long ncells,
+__global__ void __launch_bounds__(256) k_descriptors(const int* offsets, long long ncells,
                                                      lj_cell_desc* __restrict__ cells,
-                                                     const unsigned* __restrict__ gate = nullptr) {
+                                                     const unsigned* gate = nullptr) {
     chain_wait();
     chain_next();
     if (closed(gate)) return;

@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kSegThreads) k_seg_scatter(const float* __rest
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const long long i = i0 + u * kSegThreads + threadIdx.x;
-            seg[u] = i < hi ? (int)__ldg(&sc.id[i]) - seg_lo : -1;
+            seg[u] = i < hi ? (int)sc.id[i] - seg_lo : -1;
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -402,7 +402,7 @@ __device__ __forceinline__ void seg_sort(const GridDev& g, int c0, int W, int s0
 // SMALL: one block per segment of at most CAP records; else the blocks take the larger ones from the list.
 template <int ORDER, int THREADS, int CAP, bool SMALL>
 __global__ void __launch_bounds__(THREADS, SMALL ? 6 : 1) k_seg_sort(GridDev g, int ncell, int n, int shift, int nseg, SegScratch sc,
-                                                      const float4* __restrict__ tmp, int* __restrict__ counts,
+                                                      const float4* tmp, int* __restrict__ counts,
                                                       int* __restrict__ offsets, int vec, lj_cell_desc* __restrict__ cells,
                                                       SortOut so) {
     extern __shared__ __align__(16) unsigned char s_raw[];

@@ -177,9 +177,21 @@ namespace ljc {
 // Launch chaining inside one call's kernel sequence: a kernel launched with chain_launch may be scheduled
 // while its predecessor's last blocks still run; it calls chain_wait before its first access to memory
 // (which returns when every earlier grid it depends on has completed and its writes are visible), and
-// chain_next lets its own successor be scheduled in turn.
+// chain_next lets its own successor be scheduled in turn.  What earlier kernels of the chain may write during
+// that time -- all but the caller's positions of a build, which a kernel launched without the attribute reads
+// first -- is read with ordinary loads: not with __ldg, nor through a const pointer marked __restrict__, since
+// the read-only path is for data that is constant for the kernel's whole life and its loads may be moved in
+// front of the wait.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// A record by one vector load that stays behind chain_wait (volatile) but leaves other accesses free to move: in the
+// cluster walk's scan 10M particles take 2.131 ms, by a plain float4 copy 2.140.
+__device__ __forceinline__ float4 chain_load(const float4* p) {
+    float4 r;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(p));
+    return r;
+}
 
 template <class... P, class... A>
 inline void chain_launch(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream,

@@ -45,9 +45,9 @@ int default_pair_kernel(int n, const lj_grid& g) {
     return per_cell >= kClusterCell ? 1 : (per_cell >= kPairCell ? 10 : 12);
 }
 
-__global__ void __launch_bounds__(kPairThreads) k_pair_config(GridDev g, PairParams pp, const float4* __restrict__ p,
-                                                              const int* __restrict__ cs,
-                                                              const int* __restrict__ off, int n, int kb, int ke,
+__global__ void __launch_bounds__(kPairThreads) k_pair_config(GridDev g, PairParams pp, const float4* p,
+                                                              const int* cs,
+                                                              const int* off, int n, int kb, int ke,
                                                               float* __restrict__ energy, float* __restrict__ force,
                                                               Partial* part, unsigned* counter, lj_totals* totals,
                                                               unsigned* status) {
@@ -124,18 +124,18 @@ struct CompatRow {
 
 // Row (dy, dz) of cell (cx, cy, cz) clamped to the grid: [s, e), the particles of cells cx-1..cx+1;
 // (0, 0) off the grid.
-__device__ __forceinline__ int2 compat_range(const GridDev& g, const int* __restrict__ off, int n, int cx, int cy,
+__device__ __forceinline__ int2 compat_range(const GridDev& g, const int* off, int n, int cx, int cy,
                                              int cz, int dy, int dz) {
     const int z = cz + dz, y = cy + dy;
     if (z < 0 || z >= g.gz || y < 0 || y >= g.gy) return make_int2(0, 0);
     const int rb = (z * g.gy + y) * g.gx;
-    const int s = min(max(__ldg(&off[rb + max(cx - 1, 0)]), 0), n);
-    const int e = min(max(__ldg(&off[rb + min(cx + 1, g.gx - 1) + 1]), s), n);
+    const int s = min(max(off[rb + max(cx - 1, 0)], 0), n);
+    const int e = min(max(off[rb + min(cx + 1, g.gx - 1) + 1], s), n);
     return make_int2(s, e);
 }
 
 // Row (dy, dz) for this round: useA / useB select the targets, same: b shares a's rows.
-__device__ __forceinline__ CompatRow compat_row(const GridDev& g, const int* __restrict__ off, int n, bool useA,
+__device__ __forceinline__ CompatRow compat_row(const GridDev& g, const int* off, int n, bool useA,
                                                 bool useB, bool same, int cxa, int cya, int cza, int cxb, int cyb,
                                                 int czb, int dy, int dz) {
     CompatRow r{0, 0, 0, INT_MAX};
@@ -160,7 +160,7 @@ __device__ __forceinline__ CompatRow compat_row(const GridDev& g, const int* __r
 }
 
 // One window, all lanes of the warp in lockstep, two candidates per step.
-__device__ __forceinline__ void compat_walk(const float4* __restrict__ p, int kl, const CompatRow& R, float2 nx,
+__device__ __forceinline__ void compat_walk(const float4* p, int kl, const CompatRow& R, float2 nx,
                                             float2 ny, float2 nz, float2& pot) {
     const int L = R.e - R.s;
     const int maxL = (int)__reduce_max_sync(0xffffffffu, (unsigned)L);
@@ -170,7 +170,7 @@ __device__ __forceinline__ void compat_walk(const float4* __restrict__ p, int kl
             const int w = v + u;
             const bool ok = w < L;
             const int j = R.s + w;
-            const float4 q = __ldg(&p[ok ? j : kl]);
+            const float4 q = p[ok ? j : kl];
             compat2(q, ok && j < R.ea, ok && j >= R.sb, nx, ny, nz, pot);
         }
     }
@@ -178,8 +178,8 @@ __device__ __forceinline__ void compat_walk(const float4* __restrict__ p, int kl
 
 // The 9 rows of this round: the own row in two windows around the targets ([s, lo_self) and
 // [hi_self, e)), then opposite rows (-y, +y), (-z, +z), (-y-z, +y+z), (+y-z, -y+z).
-__device__ __forceinline__ void compat_rows(const GridDev& g, const float4* __restrict__ p,
-                                            const int* __restrict__ off, int n, int kl, int lo_self, int hi_self,
+__device__ __forceinline__ void compat_rows(const GridDev& g, const float4* p,
+                                            const int* off, int n, int kl, int lo_self, int hi_self,
                                             bool useA, bool useB, bool same, int cxa, int cya, int cza, int cxb,
                                             int cyb, int czb, float2 nx, float2 ny, float2 nz, float2& pot) {
     {
@@ -201,9 +201,9 @@ __device__ __forceinline__ void compat_rows(const GridDev& g, const float4* __re
     }
 }
 
-__global__ void __launch_bounds__(kPairThreads) k_pair_compat(GridDev g, const float4* __restrict__ p,
-                                                              const int* __restrict__ cs,
-                                                              const int* __restrict__ off, int n,
+__global__ void __launch_bounds__(kPairThreads) k_pair_compat(GridDev g, const float4* p,
+                                                              const int* cs,
+                                                              const int* off, int n,
                                                               float* __restrict__ v, unsigned* status) {
     chain_wait();
     const int ka = 2 * (blockIdx.x * kPairThreads + (int)threadIdx.x), kb = ka + 1;
@@ -213,22 +213,22 @@ __global__ void __launch_bounds__(kPairThreads) k_pair_compat(GridDev g, const f
     float4 pa = make_float4(far, far, far, 0.f), pb = pa;
     int cxa = 0, cya = 0, cza = 0, cxb = 0, cyb = 0, czb = 0;
     if (activeA) {
-        int c = __ldg(&cs[ka]);
+        int c = cs[ka];
         if (c < 0 || c >= ncell) {
             atomicOr(status, kFlagRange);
             c = 0;
         }
         decode_cell(g, c, cxa, cya, cza);
-        pa = __ldg(&p[ka]);
+        pa = p[ka];
     }
     if (activeB) {
-        int c = __ldg(&cs[kb]);
+        int c = cs[kb];
         if (c < 0 || c >= ncell) {
             atomicOr(status, kFlagRange);
             c = 0;
         }
         decode_cell(g, c, cxb, cyb, czb);
-        pb = __ldg(&p[kb]);
+        pb = p[kb];
     }
     const bool same = activeA && activeB && cya == cyb && cza == czb && cxb >= cxa;
     const bool apart = activeB && !same;

@@ -13,8 +13,8 @@ constexpr int kCluWarps = 4;
 // its warps in turn; SPLIT: two warps to a group, one for each cluster.
 template <bool XWIN, bool SPLIT>
 __global__ void __launch_bounds__(32 * kCluWarps, kCluWarpsPerSm / kCluWarps)
-    k_pair_cluster(GridDev g, PairParams pp, const float4* __restrict__ p, const int* __restrict__ cs,
-                   const int* __restrict__ off, int n, int kb, int ke, int a0, int stretch,
+    k_pair_cluster(GridDev g, PairParams pp, const float4* p, const int* cs,
+                   const int* off, int n, int kb, int ke, int a0, int stretch,
                    float* __restrict__ energy, float* __restrict__ force, Partial* part, unsigned* counter,
                    lj_totals* totals, unsigned* status) {
     __shared__ __align__(16) CluSmem sm[kCluWarps];

@@ -137,8 +137,8 @@ inline int clu_groups_per_warp(double waves) { return std::max(1, (int)(std::sqr
 // group s = 0, minus its force sums' components x, y, z in groups 1-3; w, np: this lane's share of the
 // target's sum of 2 s^12 - s^6 and of its interacting pairs; id: the record's fourth word.
 template <bool XWIN, class Emit>
-__device__ __forceinline__ void cluster_stretch(const GridDev& g, const PairParams& pp, const float4* __restrict__ p,
-                                                const int* __restrict__ cs, int cbase, const int* __restrict__ off,
+__device__ __forceinline__ void cluster_stretch(const GridDev& g, const PairParams& pp, const float4* p,
+                                                const int* cs, int cbase, const int* off,
                                                 int obase, int n, int a, int b, int kb, int ke, int turn, int turns,
                                                 int only, CluSmem& sm, unsigned* status, Emit emit) {
     const int lane = (int)(threadIdx.x & 31u), t = lane & 7, s = lane >> 3;
@@ -150,7 +150,7 @@ __device__ __forceinline__ void cluster_stretch(const GridDev& g, const PairPara
     bool entered = false;
     while (gs < b) {
         if (gs >= se) {  // a new segment of cells
-            int c = __ldg(&cs[gs]) - cbase;
+            int c = cs[gs] - cbase;
             if (c < 0 || c >= ncell) {
                 if (lane == 0) atomicOr(status, kFlagRange);
                 c = 0;
@@ -160,8 +160,8 @@ __device__ __forceinline__ void cluster_stretch(const GridDev& g, const PairPara
             cy = row - cz * g.gy;
             row0 = row * g.gx;
             const int c0 = row0 + cx / kCluSegment * kCluSegment, c1 = min(c0 + kCluSegment, row0 + g.gx);
-            const int ss = min(max(__ldg(&off[c0]) - obase, 0), gs);
-            se = min(max(__ldg(&off[c1]) - obase, gs + 1), n);
+            const int ss = min(max(off[c0] - obase, 0), gs);
+            se = min(max(off[c1] - obase, gs + 1), n);
             if (!entered) {  // [a, b) may begin inside a group, which then is the previous stretch's
                 entered = true;
                 gs = min(ss + (gs - ss + kCluGroup - 1) / kCluGroup * kCluGroup, se);
@@ -180,8 +180,8 @@ __device__ __forceinline__ void cluster_stretch(const GridDev& g, const PairPara
         int T, nr;
         {
             const int k = min(gs + (lane & (kCluGroup - 1)), ge - 1);
-            const float4 pi = __ldg(&p[k]);
-            const int ck = __ldg(&cs[k]) - cbase - row0;
+            const float4 pi = chain_load(&p[k]);
+            const int ck = cs[k] - cbase - row0;
             const int cxa = min(max(__shfl_sync(0xffffffffu, ck, 0), 0), g.gx - 1);
             const int cxb = min(max(__shfl_sync(0xffffffffu, ck, kCluGroup - 1), cxa), g.gx - 1);
             const float bx0 = warp_min(pi.x), bx1 = warp_max(pi.x), by0 = warp_min(pi.y), by1 = warp_max(pi.y),
@@ -206,14 +206,14 @@ __device__ __forceinline__ void cluster_stretch(const GridDev& g, const PairPara
                     const float d2 = fmaf(dym, dym, dzm * dzm);
                     if (d2 < pp.rc2w) {
                         const int rb = (z * g.gy + y) * g.gx;
-                        int lo = min(max(__ldg(&off[rb + max(cxa - 1, 0)]) - obase, 0), n);
-                        int hi = min(max(__ldg(&off[rb + min(cxb + 1, g.gx - 1) + 1]) - obase, lo), n);
+                        int lo = min(max(off[rb + max(cxa - 1, 0)] - obase, 0), n);
+                        int hi = min(max(off[rb + min(cxb + 1, g.gx - 1) + 1] - obase, lo), n);
                         if (XWIN) {
                             const float h = sqrtf(pp.rc2w - d2) + slack;
                             const float v = second ? bx1 + h : bx0 - h;
                             while (lo < hi) {  // first x >= v (starts) or x > v (ends)
                                 const int mid = (lo + hi) >> 1;
-                                const float x = __ldg(&p[mid].x);
+                                const float x = p[mid].x;
                                 if (x < v || (second && x == v))
                                     lo = mid + 1;
                                 else
@@ -246,7 +246,7 @@ __device__ __forceinline__ void cluster_stretch(const GridDev& g, const PairPara
         for (int cl = only < 0 ? gs : gs + only * kCluTargets; cl < ge; cl += only < 0 ? kCluTargets : kCluGroup) {
             const int nt = min(kCluTargets, ge - cl);
             const int k = cl + min(t, nt - 1);  // lanes past the end repeat the last target
-            const float4 pi = __ldg(&p[k]);
+            const float4 pi = chain_load(&p[k]);
             const float bx0 = warp_min(pi.x), bx1 = warp_max(pi.x), by0 = warp_min(pi.y), by1 = warp_max(pi.y),
                         bz0 = warp_min(pi.z), bz1 = warp_max(pi.z);
             const float2 nx = make_float2(-pi.x, -pi.x), ny = make_float2(-pi.y, -pi.y), nz = make_float2(-pi.z, -pi.z);
@@ -280,8 +280,8 @@ __device__ __forceinline__ void cluster_stretch(const GridDev& g, const PairPara
                 const int j = 2 * (base + lane) + __shfl_sync(0xffffffffu, rng.y, ri);
                 const int je = __shfl_sync(0xffffffffu, rng.z, ri);
                 const bool ok0 = j < je, ok1 = j + 1 < je;
-                const float4 q0 = __ldg(&p[ok0 ? j : cl]);
-                const float4 q1 = __ldg(&p[ok1 ? j + 1 : cl]);
+                const float4 q0 = chain_load(&p[ok0 ? j : cl]);
+                const float4 q1 = chain_load(&p[ok1 ? j + 1 : cl]);
                 const float dx0 = fmaxf(fmaxf(bx0 - q0.x, q0.x - bx1), 0.f), dx1 = fmaxf(fmaxf(bx0 - q1.x, q1.x - bx1), 0.f);
                 const float dy0 = fmaxf(fmaxf(by0 - q0.y, q0.y - by1), 0.f), dy1 = fmaxf(fmaxf(by0 - q1.y, q1.y - by1), 0.f);
                 const float dz0 = fmaxf(fmaxf(bz0 - q0.z, q0.z - bz1), 0.f), dz1 = fmaxf(fmaxf(bz0 - q1.z, q1.z - bz1), 0.f);

@@ -29,10 +29,10 @@ struct PairParams {
 
 // Output slot of sorted target k: k, or with pp.by_index the original index stored in its record
 // (-1, and the range flag, if that index is outside [0, n)).
-__device__ __forceinline__ int out_slot(const PairParams& pp, const float4* __restrict__ p, int k, int n,
+__device__ __forceinline__ int out_slot(const PairParams& pp, const float4* p, int k, int n,
                                         unsigned* status) {
     if (!pp.by_index) return k;
-    const int o = __float_as_int(__ldg(&p[k].w));
+    const int o = __float_as_int(p[k].w);
     if (o < 0 || o >= n) {
         atomicOr(status, kFlagRange);
         return -1;
@@ -49,10 +49,10 @@ __device__ __forceinline__ void decode_cell(const GridDev& g, int c, int& cx, in
 }
 
 // first j in [lo, hi) with p[j].x >= v (x-sorted range)
-__device__ __forceinline__ int lower_x(const float4* __restrict__ p, int lo, int hi, float v) {
+__device__ __forceinline__ int lower_x(const float4* p, int lo, int hi, float v) {
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
-        if (__ldg(&p[mid].x) < v)
+        if (p[mid].x < v)
             lo = mid + 1;
         else
             hi = mid;
@@ -60,10 +60,10 @@ __device__ __forceinline__ int lower_x(const float4* __restrict__ p, int lo, int
     return lo;
 }
 // first j in [lo, hi) with p[j].x > v
-__device__ __forceinline__ int upper_x(const float4* __restrict__ p, int lo, int hi, float v) {
+__device__ __forceinline__ int upper_x(const float4* p, int lo, int hi, float v) {
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
-        if (__ldg(&p[mid].x) <= v)
+        if (p[mid].x <= v)
             lo = mid + 1;
         else
             hi = mid;
@@ -164,8 +164,8 @@ __device__ void reduce_totals(double e, double w, unsigned long long np, Partial
 // Per-target work of the truncated law over whole rows.  `c` is the target's cell in grid g, `off` the
 // offsets of that grid (values are indices into p), `n` bounds every index.
 template <int BLOCK>
-__device__ __forceinline__ void pair_target(const GridDev& g, const PairParams& pp, const float4* __restrict__ p,
-                                            const int* __restrict__ off, int n, int k, int c,
+__device__ __forceinline__ void pair_target(const GridDev& g, const PairParams& pp, const float4* p,
+                                            const int* off, int n, int k, int c,
                                             int2 (*s_win)[BLOCK], float& ea, float& fx, float& fy, float& fz,
                                             float& wa, unsigned& np) {
     const int tid = threadIdx.x;
@@ -183,8 +183,8 @@ __device__ __forceinline__ void pair_target(const GridDev& g, const PairParams& 
             const int y = cy + dy;
             if (y < 0 || y >= g.gy) continue;
             const int rb = (z * g.gy + y) * g.gx;
-            const int s = min(max(__ldg(&off[rb + xl]), 0), n);
-            const int e = min(max(__ldg(&off[rb + xh + 1]), s), n);
+            const int s = min(max(off[rb + xl], 0), n);
+            const int e = min(max(off[rb + xh + 1], s), n);
             if (dz == 0 && dy == 0) {
                 s_win[nw++][tid] = make_int2(s, k);
                 s_win[nw++][tid] = make_int2(k + 1, e);
@@ -215,8 +215,8 @@ __device__ __forceinline__ void pair_target(const GridDev& g, const PairParams& 
         const bool two = j0 + 1 < cur.y;
         const int j1 = two ? j0 + 1 : j0;
         cur.x = j1 + 1;
-        const float4 q0 = __ldg(&p[j0]);
-        const float4 q1 = __ldg(&p[j1]);
+        const float4 q0 = p[j0];
+        const float4 q1 = p[j1];
         const float2 dx = __fadd2_rn(make_float2(q0.x, q1.x), npx);
         const float2 dy = __fadd2_rn(make_float2(q0.y, q1.y), npy);
         const float2 dz = __fadd2_rn(make_float2(q0.z, q1.z), npz);

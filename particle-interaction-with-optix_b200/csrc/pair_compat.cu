@@ -76,7 +76,7 @@ __device__ __forceinline__ void cell_walk(const CellSmem& sm, int cnt, int group
 }
 
 // Evaluates the targets [t0, t1) of cell c, which holds [cs, ce) (one warp, all lanes).
-__device__ __forceinline__ void cell_targets(const GridDev& g, const float4* __restrict__ p, const int* __restrict__ off,
+__device__ __forceinline__ void cell_targets(const GridDev& g, const float4* p, const int* off,
                                              int n, int c, int cs, int ce, int t0, int t1, CellSmem& sm,
                                              float* __restrict__ v) {
     const int lane = (int)(threadIdx.x & 31u), t = lane % kCellLanes, group = lane / kCellLanes;
@@ -91,8 +91,8 @@ __device__ __forceinline__ void cell_targets(const GridDev& g, const float4* __r
             const int z = cz + lane / 3 - 1, y = cy + lane % 3 - 1;
             if (z >= 0 && z < g.gz && y >= 0 && y < g.gy) {
                 const int rb = (z * g.gy + y) * g.gx;
-                s = min(max(__ldg(&off[rb + max(cx - 1, 0)]), 0), n);
-                e = min(max(__ldg(&off[rb + min(cx + 1, g.gx - 1) + 1]), s), n);
+                s = min(max(off[rb + max(cx - 1, 0)], 0), n);
+                e = min(max(off[rb + min(cx + 1, g.gx - 1) + 1], s), n);
             }
         }
         const int src = lane == 9 ? 4 : min(lane, 8);
@@ -120,7 +120,7 @@ __device__ __forceinline__ void cell_targets(const GridDev& g, const float4* __r
         float2 nx[kCellDeep], ny[kCellDeep], nz[kCellDeep], pot[kCellDeep];
 #pragma unroll
         for (int q = 0; q < kCellDeep; ++q) {
-            const float4 r = __ldg(&p[k0 + min(t + kCellLanes * q, m - 1)]);
+            const float4 r = p[k0 + min(t + kCellLanes * q, m - 1)];
             nx[q] = make_float2(-r.x, -r.x);
             ny[q] = make_float2(-r.y, -r.y);
             nz[q] = make_float2(-r.z, -r.z);
@@ -129,7 +129,7 @@ __device__ __forceinline__ void cell_targets(const GridDev& g, const float4* __r
         // own cell: two particles per lane group and step, never a target itself
         for (int j0 = cs; j0 < ce; j0 += 16) {
             const int j = j0 + 2 * group;
-            const float4 a = __ldg(&p[min(j, ce - 1)]), b = __ldg(&p[min(j + 1, ce - 1)]);
+            const float4 a = p[min(j, ce - 1)], b = p[min(j + 1, ce - 1)];
             const float2 X = make_float2(a.x, b.x), Y = make_float2(a.y, b.y), Z = make_float2(a.z, b.z);
 #pragma unroll
             for (int q = 0; q < kCellDeep; ++q) {
@@ -156,8 +156,8 @@ __device__ __forceinline__ void cell_targets(const GridDev& g, const float4* __r
                     const int je = __shfl_sync(0xffffffffu, rng.z, ri);
                     const float far = 1e18f;  // finite: its term is an exact 0
                     float4 a = make_float4(far, far, far, 0.f), b = a;
-                    if (j < je) a = __ldg(&p[j]);
-                    if (j + 1 < je) b = __ldg(&p[j + 1]);
+                    if (j < je) a = p[j];
+                    if (j + 1 < je) b = p[j + 1];
                     const int w = cnt + 2 * lane;
                     *reinterpret_cast<float2*>(&sm.x[w]) = make_float2(a.x, b.x);
                     *reinterpret_cast<float2*>(&sm.y[w]) = make_float2(a.y, b.y);
@@ -191,9 +191,9 @@ __device__ __forceinline__ void cell_targets(const GridDev& g, const float4* __r
 // (q + 1) chunk), holds the start of at most one such chunk, and one of the cell that holds the window's first
 // target; a finder takes every finders-th window, so the chunks of one crowded cell go to different warps.  The
 // finders also look at every target's cell id: one outside the grid is reported.
-__global__ void __launch_bounds__(32 * kCellWarps, 8) k_compat_cells(GridDev g, const float4* __restrict__ p,
-                                                                     const int* __restrict__ cell_id,
-                                                                     const int* __restrict__ off, int n, int chunk,
+__global__ void __launch_bounds__(32 * kCellWarps, 8) k_compat_cells(GridDev g, const float4* p,
+                                                                     const int* cell_id,
+                                                                     const int* off, int n, int chunk,
                                                                      int windows, int finders, float* __restrict__ v,
                                                                      unsigned* status) {
     __shared__ __align__(16) CellSmem smem[kCellWarps];
@@ -206,10 +206,10 @@ __global__ void __launch_bounds__(32 * kCellWarps, 8) k_compat_cells(GridDev g, 
         const long long q = warp + (long long)lane * finders;
         if (q < windows) {
             const int k = (int)(q * chunk);
-            c = __ldg(&cell_id[k]);
+            c = cell_id[k];
             if (c >= 0 && c < ncell) {
-                cs = min(max(__ldg(&off[c]), 0), k);
-                ce = min(__ldg(&off[c + 1]), n);
+                cs = min(max(off[c], 0), k);
+                ce = min(off[c + 1], n);
                 const long long start = cs + (long long)(k - cs + chunk - 1) / chunk * chunk;
                 t0 = start > cs ? (int)min(start, (long long)INT_MAX) : ce;
             }
@@ -218,14 +218,14 @@ __global__ void __launch_bounds__(32 * kCellWarps, 8) k_compat_cells(GridDev g, 
         bool bad = false;
 #pragma unroll 4
         for (int k = (int)((long long)n * warp / finders) + lane; k < hi; k += 32) {
-            const int id = __ldg(&cell_id[k]);
+            const int id = cell_id[k];
             bad |= id < 0 || id >= ncell;
         }
         if (bad) atomicOr(status, kFlagRange);
     } else if (warp - finders < ncell && lane == 0) {
         c = (int)(warp - finders);
-        t0 = cs = min(max(__ldg(&off[c]), 0), n);
-        ce = min(__ldg(&off[c + 1]), n);
+        t0 = cs = min(max(off[c], 0), n);
+        ce = min(off[c + 1], n);
     }
     for (unsigned todo = __ballot_sync(0xffffffffu, t0 < ce); todo; todo &= todo - 1) {
         const int src = __ffs(todo) - 1, start = __shfl_sync(0xffffffffu, t0, src), end = __shfl_sync(0xffffffffu, ce, src);

@@ -9,8 +9,8 @@ constexpr int kPassThreads = 128;
 }  // namespace
 
 // One thread per target of [kb, ke) (pass_target).
-__global__ void __launch_bounds__(kPassThreads) k_pair_pass(GridDev g, PairParams pp, const float4* __restrict__ p,
-                                                            const int* __restrict__ cs, const int* __restrict__ off,
+__global__ void __launch_bounds__(kPassThreads) k_pair_pass(GridDev g, PairParams pp, const float4* p,
+                                                            const int* cs, const int* off,
                                                             int n, int kb, int ke, float* __restrict__ energy,
                                                             float* __restrict__ force, Partial* part,
                                                             unsigned* counter, lj_totals* totals, unsigned* status) {
@@ -19,7 +19,7 @@ __global__ void __launch_bounds__(kPassThreads) k_pair_pass(GridDev g, PairParam
     const bool active = k < ke;
     int c = 0;
     if (active) {
-        c = __ldg(&cs[k]);
+        c = cs[k];
         if (c < 0 || c >= g.gx * g.gy * g.gz) {
             atomicOr(status, kFlagRange);
             c = 0;
@@ -45,8 +45,8 @@ __global__ void __launch_bounds__(kPassThreads) k_pair_pass(GridDev g, PairParam
 // Two targets per thread (pass_target2): thread t of the launch takes targets kb + 2t and kb + 2t + 1;
 // registers capped for 8 blocks per SM, the windows parked in shared memory during the walk.
 template <int BLOCK = kPassThreads>
-__global__ void __launch_bounds__(BLOCK, 8) k_pair_pass2(GridDev g, PairParams pp, const float4* __restrict__ p,
-                                                             const int* __restrict__ cs, const int* __restrict__ off,
+__global__ void __launch_bounds__(BLOCK, 8) k_pair_pass2(GridDev g, PairParams pp, const float4* p,
+                                                             const int* cs, const int* off,
                                                              int n, int kb, int ke, float* __restrict__ energy,
                                                              float* __restrict__ force, Partial* part,
                                                              unsigned* counter, lj_totals* totals, unsigned* status) {
@@ -57,14 +57,14 @@ __global__ void __launch_bounds__(BLOCK, 8) k_pair_pass2(GridDev g, PairParams p
     const int ncell = g.gx * g.gy * g.gz;
     int ca = 0, cb = 0;
     if (activeA) {
-        ca = __ldg(&cs[ka]);
+        ca = cs[ka];
         if (ca < 0 || ca >= ncell) {
             atomicOr(status, kFlagRange);
             ca = 0;
         }
     }
     if (activeB) {
-        cb = __ldg(&cs[ka + 1]);
+        cb = cs[ka + 1];
         if (cb < 0 || cb >= ncell) {
             atomicOr(status, kFlagRange);
             cb = 0;
@@ -117,18 +117,18 @@ __global__ void __launch_bounds__(BLOCK, 8) k_pair_pass2(GridDev g, PairParams p
 // against 88% for one pass).
 
 // Flag of target k: 1 when it opens a pair (even rank among the range's targets of its cell).
-__global__ void __launch_bounds__(256) k_cellpair_flags(const int* __restrict__ cs, const int* __restrict__ off,
+__global__ void __launch_bounds__(256) k_cellpair_flags(const int* cs, const int* off,
                                                         int ncell, int kb, int ke, int* __restrict__ flag,
                                                         unsigned* status) {
     chain_wait();
     chain_next();
     for (int k = kb + blockIdx.x * blockDim.x + threadIdx.x; k < ke; k += gridDim.x * blockDim.x) {
-        const int c = __ldg(&cs[k]);
+        const int c = cs[k];
         int f = 1;  // a target whose cell id is out of range stays alone (and is reported)
         if (c < 0 || c >= ncell) {
             atomicOr(status, kFlagRange);
         } else {
-            const int s = min(max(__ldg(&off[c]), kb), k);
+            const int s = min(max(off[c], kb), k);
             f = ((k - s) & 1) == 0 ? 1 : 0;
         }
         flag[k - kb] = f;
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256) k_cellpair_flags(const int* __restrict__ 
 }
 
 // list[pos[i]] = kb + i for every flagged i: the pairs' first targets in sorted order.
-__global__ void __launch_bounds__(256) k_cellpair_list(const int* __restrict__ flag, const int* __restrict__ pos,
+__global__ void __launch_bounds__(256) k_cellpair_list(const int* flag, const int* pos,
                                                        int nk, int kb, int* __restrict__ list) {
     chain_wait();
     chain_next();
@@ -149,10 +149,10 @@ __global__ void __launch_bounds__(256) k_cellpair_list(const int* __restrict__ f
 // One lane per pair: list[t] = a, b = a + 1 when in a's cell.  npairs is read on the device (pos[nk],
 // at most nk); the grid covers nk lanes, the most pairs there can be.
 template <int BLOCK = kPassThreads>
-__global__ void __launch_bounds__(BLOCK, 8) k_pair_cellpair(GridDev g, PairParams pp, const float4* __restrict__ p,
-                                                            const int* __restrict__ cs, const int* __restrict__ off,
-                                                            int n, int nk, int ke, const int* __restrict__ list,
-                                                            const int* __restrict__ npairs_p,
+__global__ void __launch_bounds__(BLOCK, 8) k_pair_cellpair(GridDev g, PairParams pp, const float4* p,
+                                                            const int* cs, const int* off,
+                                                            int n, int nk, int ke, const int* list,
+                                                            const int* npairs_p,
                                                             float* __restrict__ energy, float* __restrict__ force,
                                                             Partial* part, unsigned* counter, lj_totals* totals,
                                                             unsigned* status) {
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(BLOCK, 8) k_pair_cellpair(GridDev g, PairParam
     chain_wait();
     const int t = blockIdx.x * BLOCK + threadIdx.x;
     const int ncell = g.gx * g.gy * g.gz;
-    const bool activeA = t < min(__ldg(npairs_p), nk);
+    const bool activeA = t < min(*npairs_p, nk);
     bool activeB = false;
     int ka = 0;
     float4 pa = make_float4(0.f, 0.f, 0.f, 0.f), pb = pa;
@@ -168,15 +168,15 @@ __global__ void __launch_bounds__(BLOCK, 8) k_pair_cellpair(GridDev g, PairParam
 #pragma unroll
     for (int r = 0; r < 9; ++r) ws[r] = wl[r] = 0;
     if (activeA) {
-        ka = min(max(__ldg(&list[t]), 0), n - 1);
-        int c = __ldg(&cs[ka]);
+        ka = min(max(list[t], 0), n - 1);
+        int c = cs[ka];
         if (c < 0 || c >= ncell) {
             atomicOr(status, kFlagRange);
             c = 0;
         }
-        activeB = ka + 1 < ke && __ldg(&cs[ka + 1]) == c;
-        pa = __ldg(&p[ka]);
-        if (activeB) pb = __ldg(&p[ka + 1]);
+        activeB = ka + 1 < ke && cs[ka + 1] == c;
+        pa = p[ka];
+        if (activeB) pb = p[ka + 1];
         int cx, cy, cz;
         decode_cell(g, c, cx, cy, cz);
         const int xl = max(cx - 1, 0), xh = min(cx + 1, g.gx - 1);
@@ -185,8 +185,8 @@ __global__ void __launch_bounds__(BLOCK, 8) k_pair_cellpair(GridDev g, PairParam
             const int z = cz + r / 3 - 1, y = cy + r % 3 - 1;
             if (z < 0 || z >= g.gz || y < 0 || y >= g.gy) continue;
             const int rb = (z * g.gy + y) * g.gx;
-            const int s = min(max(__ldg(&off[rb + xl]), 0), n);
-            const int e = min(max(__ldg(&off[rb + xh + 1]), s), n);
+            const int s = min(max(off[rb + xl], 0), n);
+            const int e = min(max(off[rb + xh + 1], s), n);
             ws[r] = s;
             wl[r] = e - s;
         }

@@ -43,7 +43,7 @@ struct PassAcc {
 // or the last record for a lane without a target) instead of skipping the load, so no default value
 // has to be kept in registers; the masks discard it.
 template <bool OWN>
-__device__ __forceinline__ void walk_pass(const float4* __restrict__ p, int k, int kl, const float4& pi, int sA,
+__device__ __forceinline__ void walk_pass(const float4* p, int k, int kl, const float4& pi, int sA,
                                           int LA, int offB, int L, float rc2, float sig2, PassAcc& a) {
     const int maxL = (int)__reduce_max_sync(0xffffffffu, (unsigned)L);
     const float2 npx = make_float2(-pi.x, -pi.x), npy = make_float2(-pi.y, -pi.y),
@@ -54,8 +54,8 @@ __device__ __forceinline__ void walk_pass(const float4* __restrict__ p, int k, i
         const bool ok0 = v < L, ok1 = v1 < L;
         const int j0 = v + (v < LA ? sA : offB);
         const int j1 = v1 + (v1 < LA ? sA : offB);
-        const float4 q0 = __ldg(&p[ok0 ? j0 : kl]);
-        const float4 q1 = __ldg(&p[ok1 ? j1 : kl]);
+        const float4 q0 = p[ok0 ? j0 : kl];
+        const float4 q1 = p[ok1 ? j1 : kl];
         bool m0 = ok0, m1 = ok1;
         if (OWN) {
             m0 = m0 && j0 != k;
@@ -88,8 +88,8 @@ __device__ __forceinline__ void walk_pass(const float4* __restrict__ p, int k, i
 // cutoff.  `off` holds the offsets of the target's grid; obase is subtracted from them (the index of
 // the system's first particle when the offsets count from a larger array).  The
 // windows are a superset of the interacting partners.
-__device__ __forceinline__ void pass_windows(const GridDev& g, const PairParams& pp, const float4* __restrict__ p,
-                                             const int* __restrict__ off, int obase, int n, const float4& pi, int c,
+__device__ __forceinline__ void pass_windows(const GridDev& g, const PairParams& pp, const float4* p,
+                                             const int* off, int obase, int n, const float4& pi, int c,
                                              int (&ws)[9], int (&wl)[9]) {
     int cx, cy, cz;
     decode_cell(g, c, cx, cy, cz);
@@ -110,8 +110,8 @@ __device__ __forceinline__ void pass_windows(const GridDev& g, const PairParams&
         const float d2 = fmaf(dym, dym, dzm * dzm);
         if (d2 >= pp.rc2w) continue;
         const int rb = (z * g.gy + y) * g.gx;
-        int s = min(max(__ldg(&off[rb + xl]) - obase, 0), n);
-        int e = min(max(__ldg(&off[rb + xh + 1]) - obase, s), n);
+        int s = min(max(off[rb + xl] - obase, 0), n);
+        int e = min(max(off[rb + xh + 1] - obase, s), n);
         const float h = sqrtf(pp.rc2w - d2) + slack;
         s = lower_x(p, s, e, pi.x - h);
         e = upper_x(p, s, e, pi.x + h);
@@ -123,15 +123,15 @@ __device__ __forceinline__ void pass_windows(const GridDev& g, const PairParams&
 // Per-target pass walk, two candidates per step in paired FP32.  Every lane of the warp must call it
 // (inactive lanes with active = false): the passes' loop bounds are warp maxima.  Indices k, and
 // those of p, are local: [0, n).
-__device__ __forceinline__ void pass_target(const GridDev& g, const PairParams& pp, const float4* __restrict__ p,
-                                            const int* __restrict__ off, int obase, int n, int k, int c, bool active,
+__device__ __forceinline__ void pass_target(const GridDev& g, const PairParams& pp, const float4* p,
+                                            const int* off, int obase, int n, int k, int c, bool active,
                                             PassAcc& a) {
     int ws[9], wl[9];
 #pragma unroll
     for (int r = 0; r < 9; ++r) ws[r] = wl[r] = 0;
     float4 pi = make_float4(0.f, 0.f, 0.f, 0.f);
     if (active) {
-        pi = __ldg(&p[k]);
+        pi = p[k];
         pass_windows(g, pp, p, off, obase, n, pi, c, ws, wl);
     }
     a.e = a.w = a.fx = a.fy = a.fz = make_float2(0.f, 0.f);
@@ -203,7 +203,7 @@ __device__ __forceinline__ void eval2(const float4& q, int j, bool ok, bool useA
 // One pass of two windows (A = [sA, sA + LA), then B = [offB + LA, offB + L)), two candidates per step.
 // kl: index loaded by a lane past the end of its windows (valid, masked).
 template <bool OWN>
-__device__ __forceinline__ void walk_pass2(const float4* __restrict__ p, int ka, int kb, int kl, bool useA, bool useB,
+__device__ __forceinline__ void walk_pass2(const float4* p, int ka, int kb, int kl, bool useA, bool useB,
                                            float2 nx, float2 ny, float2 nz, int sA, int LA, int offB, int L,
                                            float rc2, float sig2, Pass2Acc& a) {
     const int maxL = (int)__reduce_max_sync(0xffffffffu, (unsigned)L);
@@ -213,8 +213,8 @@ __device__ __forceinline__ void walk_pass2(const float4* __restrict__ p, int ka,
         const bool ok0 = v < L, ok1 = v1 < L;
         const int j0 = v + (v < LA ? sA : offB);
         const int j1 = v1 + (v1 < LA ? sA : offB);
-        const float4 q0 = __ldg(&p[ok0 ? j0 : kl]);
-        const float4 q1 = __ldg(&p[ok1 ? j1 : kl]);
+        const float4 q0 = p[ok0 ? j0 : kl];
+        const float4 q1 = p[ok1 ? j1 : kl];
         eval2<OWN>(q0, j0, ok0, useA, useB, ka, kb, nx, ny, nz, rc2, nsig2, a);
         eval2<OWN>(q1, j1, ok1, useA, useB, ka, kb, nx, ny, nz, rc2, nsig2, a);
     }
@@ -226,7 +226,7 @@ __device__ __forceinline__ void walk_pass2(const float4* __restrict__ p, int ka,
 // lane to lane, so five lockstep passes would each wait for their own longest lane.  Every candidate
 // is masked against both targets' own indices (the own row is one of the windows).
 template <int BLOCK>
-__device__ __forceinline__ void walk_flat2(const float4* __restrict__ p, int ka, int kb, int kl, bool useA, bool useB,
+__device__ __forceinline__ void walk_flat2(const float4* p, int ka, int kb, int kl, bool useA, bool useB,
                                            float2 nx, float2 ny, float2 nz, const int2 (*sw)[BLOCK], int nw, int L,
                                            float rc2, float sig2, Pass2Acc& a) {
     const int maxL = (int)__reduce_max_sync(0xffffffffu, (unsigned)L);
@@ -240,8 +240,8 @@ __device__ __forceinline__ void walk_flat2(const float4* __restrict__ p, int ka,
         if (cur.x == cur.y && w + 1 < nw) cur = sw[++w][t];
         const int j1 = cur.x++;
         if (cur.x == cur.y && w + 1 < nw) cur = sw[++w][t];
-        const float4 q0 = __ldg(&p[ok0 ? j0 : kl]);
-        const float4 q1 = __ldg(&p[ok1 ? j1 : kl]);
+        const float4 q0 = p[ok0 ? j0 : kl];
+        const float4 q1 = p[ok1 ? j1 : kl];
         eval2<true>(q0, j0, ok0, useA, useB, ka, kb, nx, ny, nz, rc2, nsig2, a);
         eval2<true>(q1, j1, ok1, useA, useB, ka, kb, nx, ny, nz, rc2, nsig2, a);
     }
@@ -264,8 +264,8 @@ __device__ __forceinline__ float row_d2(const GridDev& g, int cy, int cz, int dy
 // Merged windows of targets a (cell (cxa, cy, cz)) and, when useB, b (cell (cxb, cy, cz), cxb >= cxa):
 // per row the candidates of both targets' windows (a superset of each), empty when the row is culled
 // for both.  Without useB, a's own windows.
-__device__ __forceinline__ void pass_windows2(const GridDev& g, const PairParams& pp, const float4* __restrict__ p,
-                                              const int* __restrict__ off, int obase, int n, const float4& pa,
+__device__ __forceinline__ void pass_windows2(const GridDev& g, const PairParams& pp, const float4* p,
+                                              const int* off, int obase, int n, const float4& pa,
                                               const float4& pb, bool useB, int cxa, int cxb, int cy, int cz,
                                               int (&ws)[9], int (&wl)[9]) {
     const int xl = max(cxa - 1, 0), xh = min((useB ? cxb : cxa) + 1, g.gx - 1);
@@ -294,8 +294,8 @@ __device__ __forceinline__ void pass_windows2(const GridDev& g, const PairParams
             hi = fmaxf(hi, pb.x + h);
         }
         const int rb = (z * g.gy + y) * g.gx;
-        int s = min(max(__ldg(&off[rb + xl]) - obase, 0), n);
-        int e = min(max(__ldg(&off[rb + xh + 1]) - obase, s), n);
+        int s = min(max(off[rb + xl] - obase, 0), n);
+        int e = min(max(off[rb + xh + 1] - obase, s), n);
         s = lower_x(p, s, e, lo);
         e = upper_x(p, s, e, hi);
         ws[r] = s;
@@ -306,7 +306,7 @@ __device__ __forceinline__ void pass_windows2(const GridDev& g, const PairParams
 // The 5 passes of both targets, the windows read from shared memory (sw[r][threadIdx.x] = (start,
 // length) of row r) at the start of each pass, so they hold no registers during the walk.
 template <int BLOCK>
-__device__ __forceinline__ void passes2_smem(const float4* __restrict__ p, int ka, int kb, int kl, bool useA,
+__device__ __forceinline__ void passes2_smem(const float4* p, int ka, int kb, int kl, bool useA,
                                              bool useB, float2 nx, float2 ny, float2 nz, const int2 (*sw)[BLOCK],
                                              float rc2, float sig2, Pass2Acc& a) {
     const int t = threadIdx.x;
@@ -328,19 +328,19 @@ __device__ __forceinline__ void passes2_smem(const float4* __restrict__ p, int k
 // ids).  Results: a.x for target a, a.y for target b.
 // sw: shared memory, BLOCK entries per row, where the windows are parked during the walk.
 template <int BLOCK = 128>
-__device__ __forceinline__ void pass_target2(const GridDev& g, const PairParams& pp, const float4* __restrict__ p,
-                                             const int* __restrict__ off, int obase, int n, int ka, int ca, int cb,
+__device__ __forceinline__ void pass_target2(const GridDev& g, const PairParams& pp, const float4* p,
+                                             const int* off, int obase, int n, int ka, int ca, int cb,
                                              bool activeA, bool activeB, Pass2Acc& a, int2 (*sw)[BLOCK]) {
     const int kb = ka + 1;
     float4 pa = make_float4(0.f, 0.f, 0.f, 0.f), pb = pa;
     int ws[9], wl[9];
     int cxa = 0, cya = 0, cza = 0, cxb = 0, cyb = 0, czb = 0;
     if (activeA) {
-        pa = __ldg(&p[ka]);
+        pa = p[ka];
         decode_cell(g, ca, cxa, cya, cza);
     }
     if (activeB) {
-        pb = __ldg(&p[kb]);
+        pb = p[kb];
         decode_cell(g, cb, cxb, cyb, czb);
     }
     const bool same = activeA && activeB && cya == cyb && cza == czb && cxb >= cxa;

@@ -44,7 +44,8 @@ __global__ void __launch_bounds__(256) k_verlet_drift(const float4* __restrict__
     }
 }
 
-// After the rebinning, record s' holds in .w the slot o it came from: carry vh[o] and ids[o] over.
+// After the rebinning, record s' holds in .w the slot o it came from: carry vh[o] and ids[o] over (both written
+// before the rebinning's first kernel, which is launched without chaining, so they are constant here).
 __global__ void __launch_bounds__(256) k_verlet_carry(float4* __restrict__ rec, const float* __restrict__ vh,
                                                       const int* __restrict__ ids, int n, float* __restrict__ vel,
                                                       unsigned* status) {
@@ -67,8 +68,7 @@ __global__ void __launch_bounds__(256) k_verlet_carry(float4* __restrict__ rec, 
 }
 
 // Second half kick with the new forces.
-__global__ void __launch_bounds__(256) k_verlet_kick(const float* __restrict__ force, int n3, float h,
-                                                     float* __restrict__ vel) {
+__global__ void __launch_bounds__(256) k_verlet_kick(const float* force, int n3, float h, float* __restrict__ vel) {
     chain_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += gridDim.x * blockDim.x)
         vel[i] = __fadd_rn(vel[i], __fmul_rn(h, force[i]));
