@@ -318,8 +318,8 @@ __device__ __forceinline__ void cluster_stretch(const GridDev& g, const PairPara
                     cnt = rest;
                 }
             }
-            // fill the last run with candidates beyond any cutoff (finite: a miss adds 0 times its difference)
-            if (lane < ((16 - cnt) & 15)) sm.x[cnt + lane] = sm.y[cnt + lane] = sm.z[cnt + lane] = 1e18f;
+            // fill the last run with candidates that no target accepts (kFarPlace)
+            if (lane < ((16 - cnt) & 15)) sm.x[cnt + lane] = sm.y[cnt + lane] = sm.z[cnt + lane] = kFarPlace;
             __syncwarp();
             clu_walk(sm, (cnt + 15) & ~15, s, nx, ny, nz, rc2, nsig2, acc);
             __syncwarp();

@@ -71,6 +71,12 @@ __device__ __forceinline__ int upper_x(const float4* p, int lo, int hi, float v)
     return lo;
 }
 
+// A coordinate that fills up a list of candidates: about 1.49e30, far above every coordinate between which floats
+// resolve a distance whose square they can hold (under 2e19), so its squared distance overflows and it is no
+// one's partner, and below the largest float by enough that its differences stay finite (a candidate that is no
+// partner adds 0 times its difference).
+constexpr float kFarPlace = 0x1.2d5a3p100f;
+
 constexpr int kPairThreads = 128;
 constexpr int kMaxWin = 10;
 

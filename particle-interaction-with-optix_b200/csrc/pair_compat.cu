@@ -154,8 +154,7 @@ __device__ __forceinline__ void cell_targets(const GridDev& g, const float4* p, 
                     before += __popc(starts);
                     const int j = 2 * (base + lane) + __shfl_sync(0xffffffffu, rng.y, ri);
                     const int je = __shfl_sync(0xffffffffu, rng.z, ri);
-                    const float far = 1e18f;  // finite: its term is an exact 0
-                    float4 a = make_float4(far, far, far, 0.f), b = a;
+                    float4 a = make_float4(kFarPlace, kFarPlace, kFarPlace, 0.f), b = a;  // its term is an exact 0
                     if (j < je) a = p[j];
                     if (j + 1 < je) b = p[j + 1];
                     const int w = cnt + 2 * lane;
