@@ -813,7 +813,7 @@ extern "C" lj_status lj_bin(lj_ctx* ctx, const lj_grid* g, int n, const float* x
         return s;
     }
     const SegPlan plan = segment_plan(ctx, n, nc);
-    if (plan.nseg)
+    if (plan.nseg && segment_scratch(ctx, plan))
         return bin_segments(ctx, plan, nc, n, x, y, z, stride, order, counts, offsets, cells, sorted, sorted_xyzi,
                             sorted_cell, to_dev(*g));
     if ((s = bin_prepare(ctx, n, nc, counts)) != LJ_OK) return s;

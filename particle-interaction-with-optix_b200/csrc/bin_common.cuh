@@ -32,7 +32,8 @@ struct SegPlan {
     int nseg;   // 0: the path does not take this grid
 };
 SegPlan segment_plan(const lj_ctx* ctx, int n, long long nc);
-// Enqueues the build; *gate (device) is nonzero afterwards when a segment was too large for it and the
+bool segment_scratch(lj_ctx* ctx, const SegPlan& plan);
+// Enqueues the build in the plan's scratch; *gate (device) is nonzero afterwards when a segment was too large for it and the
 // ticket kernels have to run instead.
 lj_status launch_segment_bin(lj_ctx* ctx, const SegPlan& plan, long long nc, int n, const float* x, const float* y,
                              const float* z, int stride, lj_order order, int* counts, int* offsets,

@@ -523,13 +523,29 @@ static lj_status launch_seg_sorts(lj_ctx* ctx, const SegPlan& plan, long long nc
     return last_launch_status();
 }
 
+// Bytes of an array of one word per segment.
+static size_t seg_array(const SegPlan& plan) { return ((size_t)plan.nseg * sizeof(int) + 255) & ~(size_t)255; }
+
+// Makes room for the plan's scratch; false where there is none (no memory, or the stream is being captured, when
+// nothing may be allocated): the caller takes the ticket path, which needs less and which an earlier, larger
+// build of any grid has made room for.
+bool segment_scratch(lj_ctx* ctx, const SegPlan& plan) {
+    const size_t need = 256 + 3 * seg_array(plan) + 256 + (size_t)ctx->sm_count * plan.nseg * sizeof(int);
+    if (ctx->seg && need <= ctx->seg_bytes) return true;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &capturing) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return capturing == cudaStreamCaptureStatusNone && grow(&ctx->seg, &ctx->seg_bytes, need) == LJ_OK;
+}
+
 lj_status launch_segment_bin(lj_ctx* ctx, const SegPlan& plan, long long nc, int n, const float* x, const float* y,
                              const float* z, int stride, lj_order order, int* counts, int* offsets,
                              lj_cell_desc* cells, const SortOut& so, const GridDev& g, const unsigned** gate) {
     const int blocks = ctx->sm_count;
-    const size_t seg = ((size_t)plan.nseg * sizeof(int) + 255) & ~(size_t)255;
-    lj_status s = grow(&ctx->seg, &ctx->seg_bytes, 256 + 3 * seg + 256 + (size_t)blocks * plan.nseg * sizeof(int));
-    if (s != LJ_OK) return s;
+    const size_t seg = seg_array(plan);
+    lj_status s;
     char* p = static_cast<char*>(ctx->seg);
     SegScratch sc;
     sc.gate = reinterpret_cast<unsigned*>(p);
