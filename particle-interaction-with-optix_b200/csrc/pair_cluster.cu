@@ -66,7 +66,7 @@ lj_status launch_pair_cluster(lj_ctx* ctx, const lj_grid* g, const PairParams& p
     const int stretch = split ? kCluWarps / 2 * kCluGroup
                               : kCluWarps * kCluGroup * clu_groups_per_warp((double)nk / (double)wave);
     const int blocks = (int)((nk + stretch - 1) / stretch);
-    const size_t need = 256 + (size_t)blocks * sizeof(Partial);
+    const size_t need = 256 + clu_most_blocks(nk, (double)nk / (double)wave, (double)wave / (kCluWarps * kCluGroup)) * sizeof(Partial);
     if (need > ctx->red_bytes) {
         lj_status s = grow(&ctx->red, &ctx->red_bytes, need);
         if (s != LJ_OK) return s;

@@ -128,6 +128,14 @@ __device__ __forceinline__ void clu_walk(const CluSmem& sm, int cnt, int s, floa
 // at 45, 8 at 90; 10M (150 waves) 2.17 ms at 4 groups, 2.04 at 16.
 inline int clu_groups_per_warp(double waves) { return std::max(1, (int)(std::sqrt(waves) + 0.5)); }
 
+// Blocks to make room for in a launch over nk targets of `waves` waves, of which each is one_wave blocks without
+// grouping: the most that any smaller launch has (the number itself falls where a warp takes a group more), and
+// those of the other walks, so that a smaller launch, or one on a sparser grid, finds its room made.
+inline size_t clu_most_blocks(long long nk, double waves, double one_wave) {
+    const double most = one_wave * std::max(std::min(2.0 * waves, 1.0), waves / std::max(1.0, std::sqrt(waves) - 0.5));
+    return std::max((size_t)most + 2, (size_t)(nk / kPairThreads + 1));
+}
+
 // Evaluates the groups that start in [a, b), one warp (all 32 lanes must call): of consecutive groups
 // every turns-th from the turn-th on, so that a block's warps share their candidates in L1; of a group
 // both clusters, or (only >= 0) the only-th.  p, cs, off:

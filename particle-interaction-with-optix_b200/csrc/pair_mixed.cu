@@ -1012,7 +1012,8 @@ extern "C" lj_status lj_compute_mixed(lj_ctx* ctx, const lj_grid* g, const lj_pa
     const double waves = (double)n / ((double)ctx->sm_count * kMixCluWarpsPerSm * kCluGroup);
     const int per_block = cluster ? kMixCluWarps * kCluGroup * clu_groups_per_warp(waves) : (two ? 2 * kMixThreads : kMixThreads);
     const int blocks = (n + per_block - 1) / per_block;
-    const size_t need = 256 + (size_t)blocks * sizeof(Partial);
+    const size_t most = cluster ? clu_most_blocks(n, waves, (double)ctx->sm_count * kMixCluWarpsPerSm / kMixCluWarps) : (size_t)blocks;
+    const size_t need = 256 + most * sizeof(Partial);
     if (need > ctx->red_bytes) {
         lj_status s = grow(&ctx->red, &ctx->red_bytes, need);
         if (s != LJ_OK) return s;
