@@ -544,10 +544,15 @@ static lj_status check_grid(const lj_grid* g, long long* ncells) {
     return LJ_OK;
 }
 
-// The scan's look-back state for ncells counts, zeroed.
-lj_status scan_prepare(lj_ctx* ctx, long long ncells) {
+// Bytes of the scan's look-back state for ncells counts.
+static size_t scan_bytes(long long ncells) {
     const long long ntiles = (ncells + kScanTile - 1) / kScanTile;
-    const size_t need = 256 + (size_t)(ntiles > 0 ? ntiles : 1) * sizeof(unsigned long long);
+    return 256 + (size_t)(ntiles > 0 ? ntiles : 1) * sizeof(unsigned long long);
+}
+
+// The state for ncells counts, zeroed.
+lj_status scan_prepare(lj_ctx* ctx, long long ncells) {
+    const size_t need = scan_bytes(ncells);
     const lj_status s = grow_build(ctx, &ctx->scan_state, &ctx->scan_state_bytes, need);
     if (s != LJ_OK) return s;
     return cudaMemsetAsync(ctx->scan_state, 0, need, ctx->stream) == cudaSuccess ? LJ_OK : LJ_ECUDA;
@@ -644,6 +649,20 @@ static lj_status bin_scratch(lj_ctx* ctx, int n) {
         if (s != LJ_OK) return s;
     }
     return LJ_OK;
+}
+
+// Room for the ticket build of n particles on nc cells beside a build that does without it: a program that then
+// captures a smaller system which takes tickets finds it made, as with any build.  No room is no error here.
+static void reserve_ticket_scratch(lj_ctx* ctx, int n, long long nc) {
+    if ((size_t)n <= ctx->part_cap && ctx->large_cells && ctx->scan_state && scan_bytes(nc) <= ctx->scan_state_bytes)
+        return;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &capturing) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    if (capturing != cudaStreamCaptureStatusNone || bin_scratch(ctx, n) != LJ_OK) return;
+    grow_build(ctx, &ctx->scan_state, &ctx->scan_state_bytes, scan_bytes(nc));
 }
 
 // Stage 1 of a cell-grid build: scratch for n particles, the scan's state, counts zeroed.  All memsets
@@ -802,6 +821,7 @@ extern "C" lj_status lj_bin(lj_ctx* ctx, const lj_grid* g, int n, const float* x
     if (n > 0 && (!x || !y || !z || !sorted_xyzi || !sorted_cell)) return LJ_EINVAL;
     if (reinterpret_cast<uintptr_t>(sorted_xyzi) & 15) return LJ_EINVAL;
     if (small_bin_takes(ctx, n, nc)) {
+        reserve_ticket_scratch(ctx, n, nc);
         s = launch_small_bin(ctx, nc, n, x, y, z, stride, order, counts, offsets, cells,
                              sort_out(sorted_xyzi, sorted_cell, sorted), to_dev(*g));
 #ifdef LJ_CHECKS

@@ -53,3 +53,31 @@ def test_smaller_pair_stage_under_capture(torch_cuda, form, large, small):
     for got, want in zip(out, systems[1][4]):
         assert torch.equal(got.view(torch.int32), want.view(torch.int32))
     ctx.close()
+
+
+def test_ticket_build_under_capture_after_one_launch_builds(torch_cuda):
+    """Warmed up with small systems, which one launch builds without any scratch; captured: fewer particles on
+    more cells than that launch takes, and the same particles with a set number of scatter passes."""
+    import ljcell
+
+    torch = torch_cuda
+    stream = torch.cuda.Stream()
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    xyz = [torch.rand(4096, device="cuda", generator=gen) for _ in range(3)]
+    for n, rc, passes in ((3000, 0.0476, 0), (4096, 0.05001, 2)):
+        with torch.cuda.stream(stream):
+            ctx = ljcell.Context(0, stream)
+            ctx.bin(ljcell.grid_from_box((0, 0, 0), (1, 1, 1), 0.0501), *xyz)
+            ctx.sync()
+        g = ljcell.grid_from_box((0, 0, 0), (1, 1, 1), rc)
+        part = [v[:n].contiguous() for v in xyz]
+        out, want = ctx.alloc_binned(g, n), ctx.alloc_binned(g, n)
+        ctx.set_tuning(0, passes)
+        capture(torch, stream, lambda: ctx.bin(g, *part, out=out))
+        with torch.cuda.stream(stream):
+            ctx.bin(g, *part, out=want)
+            ctx.sync()
+        for k in ("counts", "offsets", "cell"):
+            assert torch.equal(getattr(out, k), getattr(want, k))
+        assert torch.equal(out.xyzi.view(torch.int32), want.xyzi.view(torch.int32))
+        ctx.close()
