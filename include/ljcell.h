@@ -261,8 +261,8 @@ LJ_API lj_status lj_compute_half(lj_ctx* ctx, const lj_grid* g, const lj_params*
  * whose launch shape is fixed at 128 threads per particle, cudaLJ.cu:519-520).
  * Results do not depend on them except in the last bits of floating-point
  * sums.  pair_kernel, for particles binned with LJ_ORDER_X:
- *   0 = default: 1 when the grid averages 6 or more particles per cell, 10 from
- *       2, else 12,
+ *   0 = default: 1 when the grid averages 6 or more particles per cell (and, above
+ *       30,000 particles, 8 per row of cells along x), 10 from 2, else 12,
  *   1 = cluster walk: a warp takes 8 consecutive targets of a row of cells,
  *       keeps the candidates within the cutoff of their bounding box in shared
  *       memory and evaluates that list, two candidates per step in paired FP32
@@ -288,7 +288,8 @@ LJ_API lj_status lj_compute_half(lj_ctx* ctx, const lj_grid* g, const lj_params*
  *       cell).  A target's results do not depend on its partner, so
  *       lj_compute_range gives the bits of lj_compute.
  * Particles binned with LJ_ORDER_INDEX take the cluster walk (with whole cells
- * for windows) where the value is 1 or the default rule gives 1, else the walk of 11.
+ * for windows) where the value is 1 or, by default, from 6 particles per cell and,
+ * above 30,000 particles, 18 per row of cells; else the walk of 11.
  * The values 2-5 and 7-9 named variants that never won on any benchmark
  * workload (per-lane queues, register windows, cell-block tiles staged by TMA
  * bulk copies, scalar passes, SoA pairs); they are kept as aliases of the kernel

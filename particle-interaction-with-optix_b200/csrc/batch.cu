@@ -439,7 +439,7 @@ static lj_status build_grids(lj_batch* b) {
         d.n = y.n;
         // the walk of the single-system default's kernel; kernel 6's where that is kernel 12 (the
         // persistent tile queue has no pair list)
-        const int kernel = default_pair_kernel(y.n, g);
+        const int kernel = default_pair_kernel(y.n, g, LJ_ORDER_X);
         d.walk = kernel == 1 ? 2 : (kernel == 10 ? 4 : 1);
         base += (long long)g.dim[0] * g.dim[1] * g.dim[2];
         if (base > 2147483646LL) return LJ_EUNSUPPORTED;

@@ -25,6 +25,10 @@ namespace ljc {
 
 constexpr double kClusterCell = 6.0;  // particles per cell from which the default takes the cluster walk
 constexpr double kPairCell = 2.0;     // ... and below that, two targets per lane
+constexpr double kClusterRow = 8.0;         // particles of a row of cells from which it takes the cluster walk ...
+constexpr double kClusterRowIndex = 18.0;   // ... for LJ_ORDER_INDEX, whose other walk has no windows to search ...
+constexpr int kClusterFew = 30000;          // ... on more particles than this
+constexpr int kClusterRowCells = 64;        // a row of more cells counts as several (the walk's segments)
 
 // Particles per cell from which the reference law takes a warp per cell (pair_compat.cu) instead of two
 // targets per lane.  Measured, 2M uniform particles, two targets per lane -> warp per cell: 485 -> 348 us
@@ -40,9 +44,19 @@ constexpr double kCompatCell = 6.0;
 // 0.517 ms against 0.597 for kernel 11 and 0.75 for kernel 6; 0.5M uniform on 100^3 cells 0.055 ms
 // against 0.060 for kernel 6), where windows merged across cells add more candidates than the shared
 // loads save.
-int default_pair_kernel(int n, const lj_grid& g) {
+//
+// A cluster ends with its row of cells, so rows of few particles (grids of one or two cells along x) leave its
+// lanes empty: 2M particles on grids one cell long take 499 us against 400 for kernel 10 at 6 per row, 458 against
+// 449 at 8 and 442 against 471 at 9; in the LJ_ORDER_INDEX form 425 against 257 for kernel 11 at 8, 408 against
+// 395 at 16 and 418 against 431 at 18.  Up to 30,000 particles the cluster walk is the fastest at any of these.
+int default_pair_kernel(int n, const lj_grid& g, lj_order order) {
     const double per_cell = (double)n / ((double)g.dim[0] * g.dim[1] * g.dim[2]);
-    return per_cell >= kClusterCell ? 1 : (per_cell >= kPairCell ? 10 : 12);
+    const double per_row = per_cell * (g.dim[0] < kClusterRowCells ? g.dim[0] : kClusterRowCells);
+    if (per_cell >= kClusterCell &&
+        (n <= kClusterFew || per_row >= (order == LJ_ORDER_X ? kClusterRow : kClusterRowIndex)))
+        return 1;
+    if (order != LJ_ORDER_X) return 11;
+    return per_cell >= kPairCell ? 10 : 12;
 }
 
 __global__ void __launch_bounds__(kPairThreads) k_pair_config(GridDev g, PairParams pp, const float4* p,
@@ -283,7 +297,7 @@ lj_status launch_pair_config(lj_ctx* ctx, const lj_grid* g, const lj_params* prm
     pp.slack = grid_slack(*g);
     pp.by_index = by_index ? 1 : 0;
     int kernel = ctx->tuning.pair_kernel;
-    if (kernel == 0) kernel = default_pair_kernel(n, *g);
+    if (kernel == 0) kernel = default_pair_kernel(n, *g, order);
     // retired variants run the surviving kernel of their family: 2, 3, 4 -> 1; 5, 7 -> 6; 8, 9 -> 10
     const bool cluster = kernel >= 1 && kernel <= 4;
     if (cluster)

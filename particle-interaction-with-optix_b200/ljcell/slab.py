@@ -147,15 +147,20 @@ class SlabResult:
 
 # Particles per cell from which the library's default pair kernel is the cluster walk (kernel 1), and
 # from which it takes two consecutive targets per lane with x-windows (kernel 10) instead of targets
-# paired inside their cell over whole rows (kernel 12).  The library applies them to n / ncells of the
-# whole grid; a slab fills only its own layers, so `step` applies them to the occupancy of those.
+# paired inside their cell over whole rows (kernel 12); above CLUSTER_FEW particles the cluster walk also
+# wants that many particles per row of (up to 64) cells, by the order the particles are binned in.  The
+# library applies them to n / ncells of the whole grid; a slab fills only its own layers, so `step` applies
+# them to the occupancy of those.
 CLUSTER_CELL = 6.0
+CLUSTER_ROW = {1: 8.0, 0: 18.0}
+CLUSTER_FEW = 30_000
 PAIR_CELL = 2.0
 
 
-def pair_kernel_for(dom: SlabDomain, targets: int) -> int:
+def pair_kernel_for(dom: SlabDomain, targets: int, order: int = 1) -> int:
     cells = (dom.z1 - dom.z0) * dom.gx * dom.gy
-    if targets >= CLUSTER_CELL * cells:
+    if targets >= CLUSTER_CELL * cells and (targets <= CLUSTER_FEW or
+                                            targets * min(dom.gx, 64) >= CLUSTER_ROW[order] * cells):
         return 1
     return 10 if targets >= PAIR_CELL * cells else 12
 
@@ -182,7 +187,7 @@ def step(ctx, g, p, dom: SlabDomain, own_xyz, exchange=None, order=1) -> SlabRes
     ke = kb + int(own_xyz.shape[0])
     tuning = ctx.get_tuning()
     if tuning["pair_kernel"] == 0:
-        ctx.set_tuning(pair_kernel_for(dom, ke - kb), tuning["scatter_passes"])
+        ctx.set_tuning(pair_kernel_for(dom, ke - kb, order), tuning["scatter_passes"])
     try:
         e, f, tot = ctx.compute_range(g, p, b, kb, ke)
     finally:
