@@ -1,6 +1,6 @@
 """Crowded cells in the one-launch and the segment builds, against the oracle bit for bit: cells on both sides
 of the size from which they are sorted instead of ranked, of the small and the large sort kernel's capacity
-and of the gate, several in one segment, equal keys and zeros of both signs; both orders."""
+and of any block's, several in one segment, equal keys and zeros of both signs; both orders."""
 import numpy as np
 import pytest
 
@@ -59,16 +59,32 @@ def test_one_launch_build(torch_cuda, ctx, counts, levels, order):
 
 @pytest.mark.parametrize("order", [0, 1])
 @pytest.mark.parametrize("levels", [0, 9])
-@pytest.mark.parametrize("name", ["below_the_gate", "through_the_gate"])
+@pytest.mark.parametrize("name", ["as_large_as_a_block", "too_large_for_a_block"])
 def test_segment_build(torch_cuda, ctx, name, levels, order):
     """4 million uniform particles in the lower half of 74^3 cells (segments of 128 cells) and crowded cells in
     the upper half, each in a segment of its own, and three that share one."""
     rng = np.random.default_rng(7 + order)
     width = 0.0135
     p = rng.random((4_000_000, 3), dtype=np.float32) * np.array([1, 1, 0.5], np.float32)
-    counts = [511, 512, 513, 1024, 2047, 2048, 2049, 5000, 10239, 10240 if name == "below_the_gate" else 10241]
+    counts = [511, 512, 513, 1024, 2047, 2048, 2049, 5000, 10239, 10240 if name == "as_large_as_a_block" else 10241]
     cells = [(0 if i % 2 else 40, 5 * i, 50) for i in range(len(counts))]
     cells += [(3, 7, 60), (4, 7, 60), (9, 7, 60)]
     q = in_cells(rng, cells, counts + [600, 700, 1400], width, levels)
     p = np.concatenate([p, q])
+    check(torch_cuda, ctx, p[rng.permutation(len(p))], width, order)
+
+
+@pytest.mark.parametrize("order", [0, 1])
+@pytest.mark.parametrize("levels", [0, 5])
+def test_segments_too_large_for_a_block(torch_cuda, ctx, levels, order):
+    """Segments of 13,000 to 60,000 records whose cells are ranked (a block of 20^3 cells at 400 each, reaching to
+    x = 0), others whose cells are sorted, and one that holds both, among 800,000 uniform particles."""
+    rng = np.random.default_rng(17 + order)
+    width = 0.0125
+    cells = [(i, j, k) for k in range(30, 50) for j in range(30, 50) for i in range(20)]
+    counts = list(rng.integers(380, 420, len(cells)))
+    cells += [(40, 10, 5), (41, 10, 5), (42, 10, 5), (60, 70, 70), (3, 2, 1), (4, 2, 1), (5, 2, 1)]
+    counts += [15_000, 600, 40, 25_000, 511, 9000, 2000]
+    p = np.concatenate([in_cells(rng, cells, counts, width, levels), rng.random((800_000, 3), dtype=np.float32)])
+    assert len(p) >= 4_000_000
     check(torch_cuda, ctx, p[rng.permutation(len(p))], width, order)
