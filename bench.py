@@ -52,23 +52,38 @@ KERNEL_NAMES = {1: "k_pair_cluster", 6: "k_pair_pass", 10: "k_pair_pass2", 11: "
 RETIRED = {2: 1, 3: 1, 4: 1, 5: 6, 7: 6, 8: 10, 9: 10}   # tuning values of retired variants -> the kernel they run
 
 
+SMS = 148          # streaming multiprocessors of a B200, for the library's choices on small systems
+
+
 def kernel_name(k: int) -> str:
     return KERNEL_NAMES[RETIRED.get(k, k)]
+
+
 SCATTER_REGION = 56 << 20   # bytes of scattered records per binning scatter pass (the library's default)
 
 
 def bin_launches(n: int, ncells: int) -> int:
-    """Kernels one lj_bin launches: count, scan, the scatter passes, rank, large-cell sort; or, by segments
-    of cells (4 million particles and more, up to 256 per cell): count, the scatter passes, two sorts, and
-    the six ticket kernels behind the gate (a grid beyond 16384 x 8192 cells takes tickets)."""
+    """Kernels one lj_bin launches: one for a small system (up to 4096 particles and 8192 cells); by segments
+    of cells (4 million particles and more, up to 256 per cell, up to 16384 x 8192 cells) count, the scatter
+    passes, two sorts, and the four for huge segments and the large-cell sort, which mostly find no work; by
+    tickets count, scan, the scatter passes, rank, large-cell sort."""
     passes = max(1, min(8, -(-16 * n // SCATTER_REGION)))
+    if 1 <= n <= 4096 and ncells <= 8192:
+        return 1
     if n >= 4_000_000 and n <= 256 * ncells and ncells <= 16384 * 8192:
-        return 3 + passes + 6
+        return 3 + passes + 5
     return 4 + min(passes, ncells)
 
+
 def compat_kernel(n: int, ncells: int) -> str:
-    """The reference law's kernel: a warp per cell from 6 particles per cell (or on few cells)."""
-    return "k_compat_cells" if n >= 6 * ncells else "k_pair_compat"
+    """The reference law's kernel: a warp per cell from 6 particles per cell, or where all cells run at once."""
+    return "k_compat_cells" if n >= 6 * ncells or ncells <= 32 * SMS else "k_pair_compat"
+
+
+def mixed_kernel(n: int, ncells: int) -> str:
+    """The mixed form's default kernel: the cluster walk from 40 particles per cell, from 8 on small systems."""
+    cluster = n >= 40 * ncells or (n >= 8 * ncells and n <= 24 * 16 * SMS)
+    return "k_pair_mixed_cluster" if cluster else "k_pair_mixed_pass2"
 
 
 CONFIGS = {
@@ -398,7 +413,7 @@ def run_ours(args, cfg):
     achieved = algo_flops / (pair_ms * 1e-3) / 1e12
     useful = (algo_flops if mode == "compat" else FLOP_INTERACTING * pairs) / (pair_ms * 1e-3) / 1e12
     kname = {"config": kernel_name(pair_kernel) if pair_kernel else "",
-             "mixed": "k_pair_mixed_cluster" if n >= 40 * g.ncells else "k_pair_mixed_pass2",
+             "mixed": mixed_kernel(n, g.ncells),
              "compat": compat_kernel(n, g.ncells)}[mode]
     traffic = read_traffic(kname, cfg["workload"])
 
@@ -715,7 +730,7 @@ def mixed_workload(ctx, cfg, seed, flush, reps=10):
     err_plain = error_stats(*ref_caller, e[:n], f[:n])
     out = {"workload": cfg["workload"] + ", mixed precision", "ms_pair_plain": t_plain,
            "plain_kernel": kernel_name(kern), "ms_pack_mixed": t_pack, "ms_pack_and_pair_mixed": t_mixed,
-           "mixed_kernel": {0: "k_pair_mixed_cluster" if n >= 40 * g.ncells else "k_pair_mixed_pass2", 1: "k_pair_mixed", 2: "k_pair_mixed_reg"}[mk],
+           "mixed_kernel": {0: mixed_kernel(n, g.ncells), 1: "k_pair_mixed", 2: "k_pair_mixed_reg"}[mk],
            "speedup_vs_plain": t_plain / t_mixed, "pairs_plain": plain_pairs, "pairs_mixed": mixed_pairs,
            "errors_vs_fp64": {
                "mixed_vs_caller_positions": err_mixed_caller,

@@ -957,6 +957,7 @@ __global__ void __launch_bounds__(32 * kMixCluWarps, kMixCluWarpsPerSm / kMixClu
             }
         }
         gs = ge;
+        __syncwarp();  // the ranges have been read: the next group writes them
     }
     __syncwarp();
     reduce_totals<32 * kMixCluWarps>(0.5 * (double)mp.e4 * te, 0.5 * (double)mp.e24 * tw, tp, part, counter, totals);
