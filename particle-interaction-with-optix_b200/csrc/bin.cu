@@ -19,6 +19,10 @@
 
 namespace ljc {
 
+// A kernel of the ticket path behind the segment path's gate (bin_segment.cu): it has work only when
+// the gate is open (nonzero); without a gate it always has.
+__device__ __forceinline__ bool closed(const unsigned* gate) { return gate && *gate == 0u; }
+
 // ---------------------------------------------------------------- counting
 // One thread per particle, grid-stride by whole warps.  Lanes that share a
 // cell elect a leader (__match_any_sync) which adds the group's size with one
@@ -29,9 +33,10 @@ template <bool TICKETS>
 __global__ void __launch_bounds__(256) k_count(GridDev g, const float* __restrict__ x, const float* __restrict__ y,
                                                const float* __restrict__ z, int stride, int n,
                                                int* __restrict__ counts, int2* __restrict__ ct,
-                                               unsigned* status) {
+                                               unsigned* status, const unsigned* gate) {
     chain_wait();
     chain_next();
+    if (closed(gate)) return;
     const int lane = threadIdx.x & 31;
     const long long gwarp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -80,9 +85,11 @@ __device__ __forceinline__ void st_state(unsigned long long* p, unsigned long lo
 __global__ void __launch_bounds__(kScanThreads) k_scan(const int* counts, int* __restrict__ offsets,
                                                        long long n, long long ntiles,
                                                        unsigned long long* tile_state, unsigned* tile_counter,
-                                                       int vec_ok, unsigned* status) {
+                                                       int vec_ok, unsigned* status,
+                                                       const unsigned* gate = nullptr) {
     chain_wait();
     chain_next();
+    if (closed(gate)) return;
     __shared__ unsigned s_tile;
     __shared__ long long s_warp[8];
     __shared__ long long s_prefix;
@@ -217,9 +224,11 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const int* counts, int* _
 __global__ void __launch_bounds__(256) k_scatter(const float* __restrict__ x, const float* __restrict__ y,
                                                  const float* __restrict__ z, int stride, int n,
                                                  const int2* ct, const int* offsets,
-                                                 float4* __restrict__ tmp, unsigned* status, int c_lo, int c_hi) {
+                                                 float4* __restrict__ tmp, unsigned* status, int c_lo, int c_hi,
+                                                 const unsigned* gate = nullptr) {
     chain_wait();
     chain_next();
+    if (closed(gate)) return;
     constexpr int U = 4;
     const long long step = (long long)gridDim.x * blockDim.x;
     for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += U * step) {
@@ -277,9 +286,11 @@ template <int ORDER>
 __global__ void __launch_bounds__(256) k_cell_rank(const float4* tmp, const int* offsets,
                                                    GridDev g, const BinSys* __restrict__ sys,
                                                    const int* __restrict__ firsts, int nsys, int n, SortOut so,
-                                                   int* large, int large_cap, unsigned* status) {
+                                                   int* large, int large_cap, unsigned* status,
+                                                   const unsigned* gate) {
     chain_wait();
     chain_next();
+    if (closed(gate)) return;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
         const float4 r = tmp[s];
         int c;
@@ -330,7 +341,7 @@ __global__ void __launch_bounds__(256) k_cell_rank(const float4* tmp, const int*
 // Cells larger than kRankMax (rare: clustered or degenerate inputs): one
 // CTA per cell sorts 2048-record chunks in shared memory (bitonic network),
 // then merges runs pairwise, each record finding its place in the partner run
-// by binary search; ping-pong between the cell's places in the two arrays.  One block per SM, and chained behind
+// by binary search; ping-pong between the cell's tmp and out ranges.  One block per SM, and chained behind
 // k_cell_rank, so it asks for kOneBlockPerSm (3M particles, a third of them in one corner: build 683 us with two
 // blocks on half of the SMs, 482 with one on each).
 template <int ORDER>
@@ -339,8 +350,9 @@ __device__ __forceinline__ bool rec_less(const float4& a, const float4& b) {
 }
 
 template <int ORDER>
-__global__ void __launch_bounds__(1024) k_large_sort(float4* from, float4* spare, const int* offsets, int n, SortOut so,
-                                                     const int* large, int large_cap) {
+__global__ void __launch_bounds__(1024) k_large_sort(float4* __restrict__ tmp, const int* offsets,
+                                                     int n, SortOut so, const int* large,
+                                                     int large_cap) {
     chain_wait();
     chain_next();
     __shared__ float4 sbuf[2048];
@@ -351,8 +363,8 @@ __global__ void __launch_bounds__(1024) k_large_sort(float4* from, float4* spare
         int o = min(max(offsets[c], 0), n);
         int e1 = min(max(offsets[c + 1], o), n);
         const int cnt = e1 - o;
-        float4* A = from + o;
-        float4* B = spare + o;
+        float4* A = tmp + o;
+        float4* B = so.out4 + o;
         const float4 sentinel = make_float4(__int_as_float(0x7f800000), 0.f, 0.f, __int_as_float(INT_MAX));
         for (int ch = 0; ch < cnt; ch += 2048) {
             const int len = min(2048, cnt - ch);
@@ -407,11 +419,22 @@ __global__ void __launch_bounds__(1024) k_large_sort(float4* from, float4* spare
     }
 }
 
-// ---------------------------------------------------------------- descriptors / candidates
-__global__ void __launch_bounds__(256) k_descriptors(const int* offsets, long long ncells,
-                                                     lj_cell_desc* __restrict__ cells) {
+// Zeroes counts behind the gate.
+__global__ void __launch_bounds__(256) k_zero(int* __restrict__ v, long long n, const unsigned* gate) {
     chain_wait();
     chain_next();
+    if (closed(gate)) return;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        v[i] = 0;
+}
+
+// ---------------------------------------------------------------- descriptors / candidates
+__global__ void __launch_bounds__(256) k_descriptors(const int* offsets, long long ncells,
+                                                     lj_cell_desc* __restrict__ cells,
+                                                     const unsigned* gate = nullptr) {
+    chain_wait();
+    chain_next();
+    if (closed(gate)) return;
     for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < ncells;
          c += (long long)gridDim.x * blockDim.x) {
         const int o0 = offsets[c], o1 = offsets[c + 1];
@@ -536,8 +559,9 @@ lj_status scan_prepare(lj_ctx* ctx, long long ncells) {
 }
 
 // The scan after scan_prepare on the same stream.
-lj_status scan_prepared(lj_ctx* ctx, const int* counts, long long ncells, int* offsets) {
+lj_status scan_prepared(lj_ctx* ctx, const int* counts, long long ncells, int* offsets, const unsigned* gate) {
     const long long ntiles = (ncells + kScanTile - 1) / kScanTile;
+    lj_status s = LJ_OK;
     if (ncells == 0) {
         if (cudaMemsetAsync(offsets, 0, sizeof(int), ctx->stream) != cudaSuccess) return LJ_ECUDA;
         return LJ_OK;
@@ -546,10 +570,9 @@ lj_status scan_prepared(lj_ctx* ctx, const int* counts, long long ncells, int* o
     unsigned long long* states = reinterpret_cast<unsigned long long*>(static_cast<char*>(ctx->scan_state) + 256);
     const int vec_ok = ((reinterpret_cast<uintptr_t>(counts) | reinterpret_cast<uintptr_t>(offsets)) & 15) == 0;
     chain_launch(k_scan, (unsigned)ntiles, kScanThreads, 0, ctx->stream, counts, offsets, ncells, ntiles, states, counter,
-                 vec_ok, ctx->d_status);
+                 vec_ok, ctx->d_status, gate);
 #ifdef LJ_CHECKS
-    const lj_status s = last_launch_status();
-    if (s != LJ_OK) return s;
+    if ((s = last_launch_status()) != LJ_OK) return s;
     k_chk_scan<<<grid_for(ctx, ncells, 256), 256, 0, ctx->stream>>>(counts, offsets, ncells, ctx->d_status);
 #endif
     return last_launch_status();
@@ -557,7 +580,7 @@ lj_status scan_prepared(lj_ctx* ctx, const int* counts, long long ncells, int* o
 
 lj_status launch_scan(lj_ctx* ctx, const int* counts, long long ncells, int* offsets) {
     const lj_status s = scan_prepare(ctx, ncells);
-    return s != LJ_OK ? s : scan_prepared(ctx, counts, ncells, offsets);
+    return s != LJ_OK ? s : scan_prepared(ctx, counts, ncells, offsets, nullptr);
 }
 
 }  // namespace ljc
@@ -574,7 +597,7 @@ extern "C" lj_status lj_count_cells(lj_ctx* ctx, const lj_grid* g, int n, const 
     if (cudaMemsetAsync(counts, 0, sizeof(int) * (size_t)nc, ctx->stream) != cudaSuccess) return LJ_ECUDA;
     if (n == 0) return LJ_OK;
     k_count<false><<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(to_dev(*g), x, y, z, stride, n, counts, nullptr,
-                                                                  ctx->d_status);
+                                                                  ctx->d_status, nullptr);
     return last_launch_status();
 }
 
@@ -678,17 +701,22 @@ static lj_status check_sorted(lj_ctx* ctx, long long nc, int n, lj_order order, 
 }
 #endif
 
-// The ticket path after its count kernel: scan, scatter, within-cell sort.
+// The ticket path after its count kernel: scan, scatter, within-cell sort.  With a gate the kernels do
+// nothing unless it is open (each of the scatter's passes then costs 2 us, but one pass for all cells cost the
+// crowded builds that open it 45: 10M with 100,000 in one droplet 722 -> 676 us, by tickets alone 600).
 static lj_status ticket_finish(lj_ctx* ctx, long long nc, int n, const float* x, const float* y, const float* z,
                                int stride, lj_order order, int* counts, int* offsets, const SortOut& so,
-                               const GridDev& g, const BinSys* sys, const int* firsts, int nsys) {
+                               const GridDev& g, const BinSys* sys, const int* firsts, int nsys,
+                               const unsigned* gate) {
     lj_status s;
     cudaStream_t st = ctx->stream;
-    if ((s = scan_prepared(ctx, counts, nc, offsets)) != LJ_OK) return s;
+    if ((s = scan_prepared(ctx, counts, nc, offsets, gate)) != LJ_OK) return s;
     if (n == 0) return LJ_OK;
 #ifdef LJ_CHECKS
-    k_chk_tickets<<<grid_for(ctx, n, 256), 256, 0, st>>>(ctx->cell_ticket, counts, n, nc, ctx->d_status);
-    if ((s = last_launch_status()) != LJ_OK) return s;
+    if (!gate) {
+        k_chk_tickets<<<grid_for(ctx, n, 256), 256, 0, st>>>(ctx->cell_ticket, counts, n, nc, ctx->d_status);
+        if ((s = last_launch_status()) != LJ_OK) return s;
+    }
 #endif
     // passes: the tuning's scatter_passes, else enough that each pass writes about kScatterRegion bytes
     long long passes = ctx->tuning.scatter_passes;
@@ -697,23 +725,16 @@ static lj_status ticket_finish(lj_ctx* ctx, long long nc, int n, const float* x,
     for (long long q = 0; q < passes; ++q) {
         const int c_lo = (int)(nc * q / passes), c_hi = (int)(nc * (q + 1) / passes);
         chain_launch(k_scatter, grid_for(ctx, n, 256), 256, 0, st, x, y, z, stride, n, ctx->cell_ticket, offsets, ctx->tmp4,
-                     ctx->d_status, c_lo, c_hi);
+                     ctx->d_status, c_lo, c_hi, gate);
         if ((s = last_launch_status()) != LJ_OK) return s;
     }
     const int lcap = (int)ctx->large_cap;
     const auto rank = order == LJ_ORDER_X ? k_cell_rank<LJ_ORDER_X> : k_cell_rank<LJ_ORDER_INDEX>;
     chain_launch(rank, grid_for(ctx, n, 256), 256, 0, st, ctx->tmp4, offsets, g, sys, firsts, nsys, n, so,
-                 ctx->large_cells, lcap, ctx->d_status);
+                 ctx->large_cells, lcap, ctx->d_status, gate);
     if ((s = last_launch_status()) != LJ_OK) return s;
-    return launch_large_sort(ctx, order, ctx->tmp4, so.out4, offsets, n, so);
-}
-
-// Sorts the cells of the large list, whose records stand in `from` in their cell's places; `spare` holds as many.
-lj_status launch_large_sort(lj_ctx* ctx, lj_order order, float4* from, float4* spare, const int* offsets, int n,
-                            const SortOut& so) {
     const auto sort = order == LJ_ORDER_X ? k_large_sort<LJ_ORDER_X> : k_large_sort<LJ_ORDER_INDEX>;
-    chain_launch(sort, ctx->sm_count, 1024, kOneBlockPerSm, ctx->stream, from, spare, offsets, n, so, ctx->large_cells,
-                 (int)ctx->large_cap);
+    chain_launch(sort, ctx->sm_count, 1024, kOneBlockPerSm, st, ctx->tmp4, offsets, n, so, ctx->large_cells, lcap);
     return last_launch_status();
 }
 
@@ -743,10 +764,10 @@ lj_status bin_finish(lj_ctx* ctx, long long nc, int n, const float* x, const flo
                      float* sorted_xyzi, int* sorted_cell, const GridDev& g, const BinSys* sys, const int* firsts,
                      int nsys) {
     lj_status s = ticket_finish(ctx, nc, n, x, y, z, stride, order, counts, offsets,
-                                sort_out(sorted_xyzi, sorted_cell, sorted), g, sys, firsts, nsys);
+                                sort_out(sorted_xyzi, sorted_cell, sorted), g, sys, firsts, nsys, nullptr);
     if (s != LJ_OK) return s;
     if (cells) {
-        chain_launch(k_descriptors, grid_for(ctx, nc, 256), 256, 0, ctx->stream, offsets, nc, cells);
+        chain_launch(k_descriptors, grid_for(ctx, nc, 256), 256, 0, ctx->stream, offsets, nc, cells, nullptr);
         if ((s = last_launch_status()) != LJ_OK) return s;
     }
 #ifdef LJ_CHECKS
@@ -755,19 +776,32 @@ lj_status bin_finish(lj_ctx* ctx, long long nc, int n, const float* x, const flo
     return LJ_OK;
 }
 
-// The segment path.
+// The segment path, with the ticket path behind its gate for particles crowded into few segments.
 static lj_status bin_segments(lj_ctx* ctx, const SegPlan& plan, long long nc, int n, const float* x, const float* y,
                               const float* z, int stride, lj_order order, int* counts, int* offsets,
                               lj_cell_desc* cells, lj_particles* sorted, float* sorted_xyzi, int* sorted_cell,
                               const GridDev& g) {
     lj_status s = bin_scratch(ctx, n);
-    // (the scan's state is the ticket build's alone: a program that captures one after this finds its room made)
-    if (s == LJ_OK) s = grow_build(ctx, &ctx->scan_state, &ctx->scan_state_bytes, scan_bytes(nc));
     if (s != LJ_OK) return s;
+    const SortOut so = sort_out(sorted_xyzi, sorted_cell, sorted);
+    const unsigned* gate = nullptr;
+    if ((s = scan_prepare(ctx, nc)) != LJ_OK) return s;
     if (cudaMemsetAsync(ctx->large_cells, 0, sizeof(int), ctx->stream) != cudaSuccess) return LJ_ECUDA;
-    s = launch_segment_bin(ctx, plan, nc, n, x, y, z, stride, order, counts, offsets, cells,
-                           sort_out(sorted_xyzi, sorted_cell, sorted), g);
-    if (s != LJ_OK) return s;
+    if ((s = launch_segment_bin(ctx, plan, nc, n, x, y, z, stride, order, counts, offsets, cells, so, g, &gate)) != LJ_OK)
+        return s;
+    cudaStream_t st = ctx->stream;
+    chain_launch(k_zero, grid_for(ctx, nc, 256), 256, 0, st, counts, nc, gate);
+    if ((s = last_launch_status()) != LJ_OK) return s;
+    chain_launch(k_count<true>, grid_for(ctx, n, 256), 256, 0, st, g, x, y, z, stride, n, counts, ctx->cell_ticket,
+                 ctx->d_status, gate);
+    if ((s = last_launch_status()) != LJ_OK) return s;
+    if ((s = ticket_finish(ctx, nc, n, x, y, z, stride, order, counts, offsets, so, g, nullptr, nullptr, 0, gate)) !=
+        LJ_OK)
+        return s;
+    if (cells) {
+        chain_launch(k_descriptors, grid_for(ctx, nc, 256), 256, 0, st, offsets, nc, cells, gate);
+        if ((s = last_launch_status()) != LJ_OK) return s;
+    }
 #ifdef LJ_CHECKS
     if ((s = check_sorted(ctx, nc, n, order, sorted_xyzi, sorted_cell, offsets, g, true)) != LJ_OK) return s;
 #endif
@@ -806,7 +840,7 @@ extern "C" lj_status lj_bin(lj_ctx* ctx, const lj_grid* g, int n, const float* x
     if ((s = bin_prepare(ctx, n, nc, counts)) != LJ_OK) return s;
     if (n > 0) {
         k_count<true><<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(to_dev(*g), x, y, z, stride, n, counts,
-                                                                      ctx->cell_ticket, ctx->d_status);
+                                                                      ctx->cell_ticket, ctx->d_status, nullptr);
         if ((s = last_launch_status()) != LJ_OK) return s;
     }
     return bin_finish(ctx, nc, n, x, y, z, stride, order, counts, offsets, cells, sorted, sorted_xyzi, sorted_cell,
@@ -1061,7 +1095,7 @@ extern "C" lj_status lj_reorder(lj_ctx* ctx, int n, float* points, float radius)
     const float4* p4 = reinterpret_cast<const float4*>(points);
     k_reorder_count<<<grid_for(ctx, n, 256), 256, 0, st>>>(p4, n, rk, counts, ctx->cell_ticket, ctx->d_status);
     if ((s = last_launch_status()) != LJ_OK) return s;
-    if ((s = scan_prepared(ctx, counts, nkeys, offsets)) != LJ_OK) return s;
+    if ((s = scan_prepared(ctx, counts, nkeys, offsets, nullptr)) != LJ_OK) return s;
     k_scatter<<<grid_for(ctx, n, 256), 256, 0, st>>>(points, points + 1, points + 2, 4, n, ctx->cell_ticket, offsets,
                                                      ctx->tmp4, ctx->d_status, 0, INT_MAX);
     if ((s = last_launch_status()) != LJ_OK) return s;
@@ -1070,7 +1104,7 @@ extern "C" lj_status lj_reorder(lj_ctx* ctx, int n, float* points, float radius)
     k_reorder_rank<<<grid_for(ctx, n, 256), 256, 0, st>>>(ctx->tmp4, ctx->cell_ticket, offsets, n, so,
                                                           ctx->large_cells, lcap, ctx->d_status);
     if ((s = last_launch_status()) != LJ_OK) return s;
-    k_large_sort<LJ_ORDER_INDEX><<<ctx->sm_count, 1024, 0, st>>>(ctx->tmp4, sorted, offsets, n, so, ctx->large_cells, lcap);
+    k_large_sort<LJ_ORDER_INDEX><<<ctx->sm_count, 1024, 0, st>>>(ctx->tmp4, offsets, n, so, ctx->large_cells, lcap);
     if ((s = last_launch_status()) != LJ_OK) return s;
     k_reorder_emit<<<grid_for(ctx, n, 256), 256, 0, st>>>(sorted, keys, n, reinterpret_cast<float4*>(points));
     return last_launch_status();

@@ -33,14 +33,11 @@ struct SegPlan {
 };
 SegPlan segment_plan(const lj_ctx* ctx, int n, long long nc);
 bool segment_scratch(lj_ctx* ctx, const SegPlan& plan);
-// Enqueues the build in the plan's scratch; the context's large list is empty.
+// Enqueues the build in the plan's scratch; *gate (device) is nonzero afterwards when a segment was too large for it and the
+// ticket kernels have to run instead.
 lj_status launch_segment_bin(lj_ctx* ctx, const SegPlan& plan, long long nc, int n, const float* x, const float* y,
                              const float* z, int stride, lj_order order, int* counts, int* offsets,
-                             lj_cell_desc* cells, const SortOut& so, const GridDev& g);
-
-// Sorts the cells of the context's large list (bin.cu).
-lj_status launch_large_sort(lj_ctx* ctx, lj_order order, float4* from, float4* spare, const int* offsets, int n,
-                            const SortOut& so);
+                             lj_cell_desc* cells, const SortOut& so, const GridDev& g, const unsigned** gate);
 
 // Sets what the build's kernels need on the current device; lj_create calls it.
 lj_status bin_shared_limits();

@@ -5,12 +5,11 @@
 // shared memory:
 //
 //   k_seg_count    per-block histogram of segments; each block reserves its share of every segment, the
-//                  last one to finish writes the segments' starts and the lists of those too large for
-//                  the small sort kernel and for any block
+//                  last one to finish writes the segments' starts and the list of those too large for
+//                  the small sort kernel
 //   k_seg_scatter  records to their segment, each block to the slots it reserved
 //   k_seg_sort     per segment: cell counts, their prefix, the records grouped by cell and ranked by
 //                  key, all in shared memory; counts, offsets and every sorted output leave in order
-//   k_huge_*       the segments that no block can hold (particles crowded into few cells), by tickets
 //
 // The ticket path does one global atomic, a gather of its cell's offset and a 16-byte write to a random
 // place per particle (in passes over cell ranges that fit L2, each reading all tickets again), and ranks
@@ -34,24 +33,19 @@ constexpr int kSegCells = 8192;         // cells of a segment: its counters take
 constexpr int kSegAim = 768;            // particles per segment to aim for (up to twice that by the power of two)
 constexpr int kSegThreads = 1024;       // count and scatter
 constexpr int kSegSmall = 2048;         // records of a segment in the small sort kernel ...
-constexpr int kSegLarge = 10240;        // ... and in the large one; a segment above is huge
+constexpr int kSegLarge = 10240;        // ... and in the large one; a segment above opens the gate
 constexpr int kSmallParticles = 4096;  // a system that one block bins (of at most kSegCells cells)
 constexpr int kSegMinParticles = 4000000;
 constexpr long long kSegRegion = 56LL << 20;  // bytes of records one scatter pass writes (L2 holds 126 MB)
 
 struct SegScratch {
-    unsigned* head;    // [0] number of huge segments, [1] of large ones, [2] blocks that have counted, [3] warp rounds
-                       // of particles of several segments, [4] set when those are few: scatter in one pass, [5] records
-                       // of the huge segments
+    unsigned* gate;    // [0] gate, [1] number of large segments, [2] blocks that have counted, [3] warp rounds of
+                       // particles of several segments, [4] set when those are few: scatter in one pass
     int* total;        // [nseg] particles per segment while counting, then unused
     int* start;        // [nseg + 1]
-    int* large;        // [nseg] segments above kSegSmall, up to kSegLarge
-    int* huge;         // [nseg] segments above kSegLarge
-    int* before;       // [nseg] records of the huge segments that stand before it in that list
+    int* large;        // [nseg] segments above kSegSmall
     unsigned short* id;  // [n] each particle's segment
     int* base;         // [blocks * nseg] a block's first slot in each segment, from the segment's start
-    int* ticket;       // [n] a huge segment's record's place in its cell, in the place of id ...
-    int* perm;         // [n] ... and the records in cell order
 };
 }  // namespace
 
@@ -75,18 +69,14 @@ __device__ __forceinline__ int seg_take(int* h, int s, bool valid, unsigned& mix
     return valid ? atomicAdd(&h[s], 1) : 0;
 }
 
-// One block: exclusive prefix of the segments' totals, the large and the huge segments.
+// One block: exclusive prefix of the segments' totals, the large segments, the gate.
 __device__ __forceinline__ void seg_scan(int nseg, int n, const SegScratch& sc) {
     __shared__ int s_warp[kSegThreads / 32];
     __shared__ int s_large;
-    __shared__ unsigned long long s_huge;  // their number << 32 | records
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int PER = kSegMax / kSegThreads;
     const int first = tid * PER;
-    if (tid == 0) {
-        s_large = 0;
-        s_huge = 0;
-    }
+    if (tid == 0) s_large = 0;
     int sum = 0;
 #pragma unroll
     for (int k = 0; k < PER; k += 4) {  // total has room for a multiple of 64 entries, zeroed
@@ -116,22 +106,15 @@ __device__ __forceinline__ void seg_scan(int nseg, int n, const SegScratch& sc) 
     for (int k = 0; k < PER && first + k < nseg; ++k) {
         const int v = __ldcg(sc.total + first + k);
         sc.start[first + k] = run;
-        if (v > kSegLarge) {
-            const unsigned long long at = atomicAdd(&s_huge, (1ULL << 32) | (unsigned)v);
-            sc.huge[at >> 32] = first + k;
-            sc.before[at >> 32] = (int)(unsigned)at;
-        } else if (v > kSegSmall) {
-            sc.large[atomicAdd(&s_large, 1)] = first + k;
-        }
+        if (v > kSegSmall) sc.large[atomicAdd(&s_large, 1)] = first + k;
+        if (v > kSegLarge) sc.gate[0] = 1u;
         run += v;
     }
     __syncthreads();
     if (tid == 0) {
         sc.start[nseg] = n;
-        sc.head[0] = (unsigned)(s_huge >> 32);
-        sc.head[1] = (unsigned)s_large;
-        sc.head[5] = (unsigned)s_huge;
-        sc.head[4] = __ldcg(&sc.head[3]) <= (unsigned)n / 128u ? 1u : 0u;  // a quarter of the warps' rounds
+        sc.gate[1] = (unsigned)s_large;
+        sc.gate[4] = __ldcg(&sc.gate[3]) <= (unsigned)n / 128u ? 1u : 0u;  // a quarter of the warps' rounds
     }
 }
 
@@ -168,7 +151,7 @@ __global__ void __launch_bounds__(kSegThreads) k_seg_count(GridDev g, const floa
         }
     }
     if (bad) atomicOr(status, kFlagNonFinite);
-    if (mixed && lane_id() == 0) atomicAdd(&sc.head[3], mixed);
+    if (mixed && lane_id() == 0) atomicAdd(&sc.gate[3], mixed);
     __syncthreads();
     int* base = sc.base + (size_t)blockIdx.x * nseg;
     for (int i = threadIdx.x; i < nseg; i += kSegThreads) {
@@ -178,7 +161,7 @@ __global__ void __launch_bounds__(kSegThreads) k_seg_count(GridDev g, const floa
     __shared__ bool s_last;
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(&sc.head[2], 1u) == gridDim.x - 1;
+    if (threadIdx.x == 0) s_last = atomicAdd(&sc.gate[2], 1u) == gridDim.x - 1;
     __syncthreads();
     if (!s_last) return;
     __threadfence();
@@ -186,21 +169,17 @@ __global__ void __launch_bounds__(kSegThreads) k_seg_count(GridDev g, const floa
 }
 
 // Block b moves the particles it counted to the slots it reserved, as (x, y, z, index bits): those of
-// segments [seg_lo, seg_hi) only (see launch_segment_bin).  The first pass also zeroes the cells of huge segments.
+// segments [seg_lo, seg_hi) only (see launch_segment_bin).
 __global__ void __launch_bounds__(kSegThreads) k_seg_scatter(const float* __restrict__ x,
                                                              const float* __restrict__ y, const float* __restrict__ z,
-                                                             int stride, int n, int ncell, int shift, int nseg,
-                                                             SegScratch sc, float4* __restrict__ tmp,
-                                                             int* __restrict__ counts, unsigned* status, int seg_lo,
+                                                             int stride, int n, int nseg, SegScratch sc,
+                                                             float4* __restrict__ tmp, unsigned* status, int seg_lo,
                                                              int seg_hi) {
     extern __shared__ int s_next[];
     chain_wait();
     chain_next();
-    if (seg_lo == 0)
-        for (int h = blockIdx.x; h < (int)sc.head[0]; h += gridDim.x)
-            for (int c = sc.huge[h] << shift, e = min(c + (1 << shift), ncell), i = c + threadIdx.x; i < e; i += kSegThreads)
-                counts[i] = 0;
-    if (sc.head[4]) {  // nearly sorted particles: the writes of all segments are in order anyway
+    if (sc.gate[0]) return;
+    if (sc.gate[4]) {  // nearly sorted particles: the writes of all segments are in order anyway
         if (seg_lo > 0) return;
         seg_hi = nseg;
     }
@@ -432,8 +411,9 @@ __global__ void __launch_bounds__(THREADS, SMALL ? 6 : 1) k_seg_sort(GridDev g, 
     unsigned short* s_cell = reinterpret_cast<unsigned short*>(s_raw + (size_t)CAP * 16);
     chain_wait();
     chain_next();
+    if (sc.gate[0]) return;
     if (SMALL && blockIdx.x == 0 && threadIdx.x == 0) offsets[ncell] = n;
-    const int items = SMALL ? nseg : min((int)sc.head[1], nseg);
+    const int items = SMALL ? nseg : min((int)sc.gate[1], nseg);
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
         const int b = SMALL ? it : sc.large[it];
         const int s0 = sc.start[b], m = sc.start[b + 1] - s0;
@@ -443,136 +423,6 @@ __global__ void __launch_bounds__(THREADS, SMALL ? 6 : 1) k_seg_sort(GridDev g, 
             g, c0, W, s0, m, [&](int i) { return __ldcg(&tmp[s0 + i]); }, counts, offsets, vec != 0, cells, so, s_rec,
             s_cnt, s_cell);
         if (!SMALL) __syncthreads();
-    }
-}
-
-// ---------------------------------------------------------------- huge segments
-// A segment of more records than a block holds takes the ticket build on its own records: their cells counted with
-// tickets, the cells' offsets, the records' places in cell order, and a rank within the cell, or the sort of the
-// large cells (k_large_sort).  Each kernel goes over the records of all huge segments, one after the other.
-
-// Position of the f-th of them in the scattered records.
-__device__ __forceinline__ int huge_record(const SegScratch& sc, int f) {
-    int lo = 0, hi = (int)sc.head[0] - 1;
-    while (lo < hi) {  // the last segment with before <= f
-        const int mid = (lo + hi + 1) >> 1;
-        if (sc.before[mid] <= f)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    return sc.start[sc.huge[lo]] + (f - sc.before[lo]);
-}
-
-__global__ void __launch_bounds__(256) k_huge_count(GridDev g, SegScratch sc, const float4* tmp, int* counts) {
-    chain_wait();
-    chain_next();
-    const int m = (int)sc.head[5], lane = (int)(threadIdx.x & 31u);
-    for (long long f0 = ((long long)blockIdx.x * 256 + threadIdx.x) - lane; f0 < m; f0 += (long long)gridDim.x * 256) {
-        const bool valid = f0 + lane < m;
-        int i = 0, cell = -1 - lane;  // a key of its own for a lane without a record
-        if (valid) {
-            i = huge_record(sc, (int)f0 + lane);
-            const float4 r = tmp[i];
-            cell = cell_of(g, r.x, r.y, r.z);
-        }
-        const unsigned peers = __match_any_sync(0xffffffffu, cell);
-        const int leader = __ffs(peers) - 1;
-        int first = 0;
-        if (valid && lane == leader) first = atomicAdd(&counts[cell], __popc(peers));
-        first = __shfl_sync(0xffffffffu, first, leader);
-        if (valid) sc.ticket[i] = first + __popc(peers & lanemask_lt());
-    }
-}
-
-// One block per huge segment: offsets (and descriptors) of its cells.
-__global__ void __launch_bounds__(kSegThreads) k_huge_offsets(SegScratch sc, int ncell, int shift, const int* counts,
-                                                              int* __restrict__ offsets,
-                                                              lj_cell_desc* __restrict__ cells) {
-    __shared__ int s_warp[kSegThreads / 32];
-    chain_wait();
-    chain_next();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int h = blockIdx.x; h < (int)sc.head[0]; h += gridDim.x) {
-        const int c0 = sc.huge[h] << shift, W = min(1 << shift, ncell - c0);
-        int run = sc.start[sc.huge[h]];
-        for (int base = 0; base < W; base += kSegThreads) {
-            const int c = base + tid, v = c < W ? counts[c0 + c] : 0;
-            int inc = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += t;
-            }
-            if (lane == 31) s_warp[warp] = inc;
-            __syncthreads();
-            const int mine = s_warp[lane];
-            const int all = __reduce_add_sync(0xffffffffu, mine);
-            const int ahead = __reduce_add_sync(0xffffffffu, lane < warp ? mine : 0);
-            if (c < W) {
-                offsets[c0 + c] = run + ahead + inc - v;
-                if (cells) cells[c0 + c] = lj_cell_desc{v, run + ahead + inc - v};
-            }
-            run += all;
-            __syncthreads();
-        }
-    }
-}
-
-__global__ void __launch_bounds__(256) k_huge_place(GridDev g, SegScratch sc, const float4* tmp, const int* offsets, int n,
-                                                    unsigned* status) {
-    chain_wait();
-    chain_next();
-    const int m = (int)sc.head[5];
-    for (long long f = (long long)blockIdx.x * 256 + threadIdx.x; f < m; f += (long long)gridDim.x * 256) {
-        const int i = huge_record(sc, (int)f);
-        const float4 r = tmp[i];
-        const long long at = (long long)offsets[cell_of(g, r.x, r.y, r.z)] + sc.ticket[i];
-        if (at >= 0 && at < n)
-            sc.perm[at] = i;
-        else
-            atomicOr(status, kFlagRange);
-    }
-}
-
-// A record's rank is the number of its cell's records with a smaller key; the records of a cell above kRankMax go to
-// its places in out4 as they come, and the cell to the large list.
-template <int ORDER>
-__global__ void __launch_bounds__(256) k_huge_rank(GridDev g, SegScratch sc, const float4* tmp, const int* counts,
-                                                   const int* offsets, int n, SortOut so, int* large, int large_cap,
-                                                   unsigned* status) {
-    chain_wait();
-    chain_next();
-    const int m = (int)sc.head[5];
-    for (long long f = (long long)blockIdx.x * 256 + threadIdx.x; f < m; f += (long long)gridDim.x * 256) {
-        const int s = huge_record(sc, (int)f);
-        const float4 r = tmp[min(max(sc.perm[s], 0), n - 1)];
-        const int c = cell_of(g, r.x, r.y, r.z), ri = __float_as_int(r.w);
-        const int e0 = min(max(offsets[c], 0), n), e1 = min(e0 + max(counts[c], 0), n);
-        so.out_cell[s] = c;
-        if (e1 - e0 > kRankMax) {
-            so.out4[s] = r;
-            if (s == e0) {
-                const int slot = atomicAdd(&large[0], 1);
-                if (slot < large_cap)
-                    large[1 + slot] = c;
-                else
-                    atomicOr(status, kFlagRange);
-            }
-            continue;
-        }
-        int rank = 0;
-#pragma unroll 4
-        for (int j = e0; j < e1; ++j) {
-            const float4 t = tmp[min(max(sc.perm[j], 0), n - 1)];
-            rank += key_less<ORDER>(t.x, __float_as_int(t.w), r.x, ri) ? 1 : 0;
-        }
-        const int slot = e0 + rank;
-        so.out4[slot] = r;
-        if (so.sx) so.sx[slot] = r.x;
-        if (so.sy) so.sy[slot] = r.y;
-        if (so.sz) so.sz[slot] = r.z;
-        if (so.sidx) so.sidx[slot] = ri;
     }
 }
 
@@ -639,9 +489,9 @@ lj_status launch_small_bin(lj_ctx* ctx, long long nc, int n, const float* x, con
 }
 
 // Segments of a power of two of cells, kSegAim to twice as many particles on average.  Taken from
-// kSegMinParticles particles up (below, its launches, of which those for crowded segments mostly find no work, cost
-// what it saves: see the figures above), for grids of at most kSegMax * kSegCells cells and at most 256 particles
-// per cell, and not where the caller sets the number of scatter passes.
+// kSegMinParticles particles up (below, its launches and those behind the gate cost what it saves: see
+// the figures above), for grids of at most kSegMax * kSegCells cells and at most 256 particles per cell,
+// and not where the caller sets the number of scatter passes.
 SegPlan segment_plan(const lj_ctx* ctx, int n, long long nc) {
     SegPlan p{0, 0};
     if (n < kSegMinParticles || ctx->tuning.scatter_passes > 0 || (long long)n > 256 * nc) return p;
@@ -680,7 +530,7 @@ static size_t seg_array(const SegPlan& plan) { return ((size_t)plan.nseg * sizeo
 // nothing may be allocated): the caller takes the ticket path, which needs less and which an earlier, larger
 // build of any grid has made room for.
 bool segment_scratch(lj_ctx* ctx, const SegPlan& plan) {
-    const size_t need = 256 + 5 * seg_array(plan) + 256 + (size_t)ctx->sm_count * plan.nseg * sizeof(int);
+    const size_t need = 256 + 3 * seg_array(plan) + 256 + (size_t)ctx->sm_count * plan.nseg * sizeof(int);
     if (ctx->seg && need <= ctx->seg_bytes) return true;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(ctx->stream, &capturing) != cudaSuccess) {
@@ -692,22 +542,19 @@ bool segment_scratch(lj_ctx* ctx, const SegPlan& plan) {
 
 lj_status launch_segment_bin(lj_ctx* ctx, const SegPlan& plan, long long nc, int n, const float* x, const float* y,
                              const float* z, int stride, lj_order order, int* counts, int* offsets,
-                             lj_cell_desc* cells, const SortOut& so, const GridDev& g) {
+                             lj_cell_desc* cells, const SortOut& so, const GridDev& g, const unsigned** gate) {
     const int blocks = ctx->sm_count;
     const size_t seg = seg_array(plan);
     lj_status s;
     char* p = static_cast<char*>(ctx->seg);
     SegScratch sc;
-    sc.head = reinterpret_cast<unsigned*>(p);
+    sc.gate = reinterpret_cast<unsigned*>(p);
     sc.total = reinterpret_cast<int*>(p + 256);
     sc.large = reinterpret_cast<int*>(p + 256 + seg);
-    sc.huge = reinterpret_cast<int*>(p + 256 + 2 * seg);
-    sc.before = reinterpret_cast<int*>(p + 256 + 3 * seg);
-    sc.start = reinterpret_cast<int*>(p + 256 + 4 * seg);  // nseg + 1 entries
-    sc.base = reinterpret_cast<int*>(p + 256 + 5 * seg + 256);
-    sc.id = reinterpret_cast<unsigned short*>(ctx->cell_ticket);  // read by the scatter for the last time
-    sc.ticket = reinterpret_cast<int*>(ctx->cell_ticket);
-    sc.perm = sc.ticket + n;
+    sc.start = reinterpret_cast<int*>(p + 256 + 2 * seg);  // nseg + 1 entries
+    sc.base = reinterpret_cast<int*>(p + 256 + 3 * seg + 256);
+    sc.id = reinterpret_cast<unsigned short*>(ctx->cell_ticket);  // the tickets' place: used behind the gate only
+    *gate = sc.gate;
     cudaStream_t st = ctx->stream;
     if (cudaMemsetAsync(p, 0, 256 + seg, st) != cudaSuccess) return LJ_ECUDA;
     const size_t hist = (size_t)plan.nseg * sizeof(int);
@@ -718,27 +565,12 @@ lj_status launch_segment_bin(lj_ctx* ctx, const SegPlan& plan, long long nc, int
     const long long passes = std::max(1LL, std::min(8LL, ((long long)n * 16 + kSegRegion - 1) / kSegRegion));
     for (long long q = 0; q < passes; ++q) {
         const int s_lo = (int)(plan.nseg * q / passes), s_hi = (int)(plan.nseg * (q + 1) / passes);
-        chain_launch(k_seg_scatter, blocks, kSegThreads, kOneBlockPerSm, st, x, y, z, stride, n, (int)nc, plan.shift, plan.nseg,
-                     sc, ctx->tmp4, counts, ctx->d_status, s_lo, s_hi);
+        chain_launch(k_seg_scatter, blocks, kSegThreads, kOneBlockPerSm, st, x, y, z, stride, n, plan.nseg, sc, ctx->tmp4,
+                     ctx->d_status, s_lo, s_hi);
         if ((s = last_launch_status()) != LJ_OK) return s;
     }
-    s = order == LJ_ORDER_X ? launch_seg_sorts<LJ_ORDER_X>(ctx, plan, nc, n, sc, counts, offsets, cells, so, g)
-                            : launch_seg_sorts<LJ_ORDER_INDEX>(ctx, plan, nc, n, sc, counts, offsets, cells, so, g);
-    if (s != LJ_OK) return s;
-    // huge segments, where there are any: at most n / kSegLarge
-    const int grid = grid_for(ctx, n, 256);
-    chain_launch(k_huge_count, grid, 256, 0, st, g, sc, ctx->tmp4, counts);
-    if ((s = last_launch_status()) != LJ_OK) return s;
-    chain_launch(k_huge_offsets, std::min(blocks, n / kSegLarge), kSegThreads, 0, st, sc, (int)nc, plan.shift, counts, offsets,
-                 cells);
-    if ((s = last_launch_status()) != LJ_OK) return s;
-    chain_launch(k_huge_place, grid, 256, 0, st, g, sc, ctx->tmp4, offsets, n, ctx->d_status);
-    if ((s = last_launch_status()) != LJ_OK) return s;
-    const auto rank = order == LJ_ORDER_X ? k_huge_rank<LJ_ORDER_X> : k_huge_rank<LJ_ORDER_INDEX>;
-    chain_launch(rank, grid, 256, 0, st, g, sc, ctx->tmp4, counts, offsets, n, so, ctx->large_cells, (int)ctx->large_cap,
-                 ctx->d_status);
-    if ((s = last_launch_status()) != LJ_OK) return s;
-    return launch_large_sort(ctx, order, so.out4, ctx->tmp4, offsets, n, so);
+    return order == LJ_ORDER_X ? launch_seg_sorts<LJ_ORDER_X>(ctx, plan, nc, n, sc, counts, offsets, cells, so, g)
+                               : launch_seg_sorts<LJ_ORDER_INDEX>(ctx, plan, nc, n, sc, counts, offsets, cells, so, g);
 }
 
 }  // namespace ljc

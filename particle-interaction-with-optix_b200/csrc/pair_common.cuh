@@ -269,7 +269,8 @@ lj_status launch_compat_cells(lj_ctx* ctx, const lj_grid* g, int n, const float*
                               const int* off, float* v);
 // Exclusive scan of counts[ncells] into offsets[0..ncells] on the context's stream (bin.cu).
 lj_status launch_scan(lj_ctx* ctx, const int* counts, long long ncells, int* offsets);
-// The same in two steps, for a caller that has kernels to launch between the scan's memset and the scan.
+// The same in two steps, for a caller that has kernels to launch between the scan's memset and the scan;
+// gate: null, or the word that has to be nonzero for the scan to run.
 lj_status scan_prepare(lj_ctx* ctx, long long ncells);
-lj_status scan_prepared(lj_ctx* ctx, const int* counts, long long ncells, int* offsets);
+lj_status scan_prepared(lj_ctx* ctx, const int* counts, long long ncells, int* offsets, const unsigned* gate);
 }  // namespace ljc

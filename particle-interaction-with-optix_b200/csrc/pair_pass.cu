@@ -253,7 +253,7 @@ lj_status launch_pair_cellpair(lj_ctx* ctx, const lj_grid* g, const PairParams& 
     if ((s = scan_prepare(ctx, nk)) != LJ_OK) return s;
     k_cellpair_flags<<<grid_for(ctx, nk, 256), 256, 0, st>>>(cs, off, ncell, kb, ke, flag, ctx->d_status);
     if ((s = last_launch_status()) != LJ_OK) return s;
-    if ((s = scan_prepared(ctx, flag, nk, pos)) != LJ_OK) return s;
+    if ((s = scan_prepared(ctx, flag, nk, pos, nullptr)) != LJ_OK) return s;
     chain_launch(k_cellpair_list, grid_for(ctx, nk, 256), 256, 0, st, flag, pos, (int)nk, kb, list);
     if ((s = last_launch_status()) != LJ_OK) return s;
     unsigned* counter = static_cast<unsigned*>(ctx->red);
