@@ -65,13 +65,13 @@ SCATTER_REGION = 56 << 20   # bytes of scattered records per binning scatter pas
 def bin_launches(n: int, ncells: int) -> int:
     """Kernels one lj_bin launches: one for a small system (up to 4096 particles and 8192 cells); by segments
     of cells (4 million particles and more, up to 256 per cell, up to 16384 x 8192 cells) count, the scatter
-    passes, two sorts, and behind the gate zero, count, scan, the scatter passes, rank, large-cell sort; by
+    passes, two sorts, and behind the gate zero, count, scan, scatter, rank, large-cell sort; by
     tickets count, scan, the scatter passes, rank, large-cell sort."""
     passes = max(1, min(8, -(-16 * n // SCATTER_REGION)))
     if 1 <= n <= 4096 and ncells <= 8192:
         return 1
     if n >= 4_000_000 and n <= 256 * ncells and ncells <= 16384 * 8192:
-        return 3 + passes + 5 + passes
+        return 3 + passes + 6
     return 4 + min(passes, ncells)
 
 

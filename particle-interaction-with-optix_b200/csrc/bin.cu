@@ -702,8 +702,7 @@ static lj_status check_sorted(lj_ctx* ctx, long long nc, int n, lj_order order, 
 #endif
 
 // The ticket path after its count kernel: scan, scatter, within-cell sort.  With a gate the kernels do
-// nothing unless it is open (each of the scatter's passes then costs 2 us, but one pass for all cells cost the
-// crowded builds that open it 45: 10M with 100,000 in one droplet 722 -> 676 us, by tickets alone 600).
+// nothing unless it is open, and the scatter takes one pass.
 static lj_status ticket_finish(lj_ctx* ctx, long long nc, int n, const float* x, const float* y, const float* z,
                                int stride, lj_order order, int* counts, int* offsets, const SortOut& so,
                                const GridDev& g, const BinSys* sys, const int* firsts, int nsys,
@@ -719,7 +718,7 @@ static lj_status ticket_finish(lj_ctx* ctx, long long nc, int n, const float* x,
     }
 #endif
     // passes: the tuning's scatter_passes, else enough that each pass writes about kScatterRegion bytes
-    long long passes = ctx->tuning.scatter_passes;
+    long long passes = gate ? 1 : ctx->tuning.scatter_passes;
     if (passes <= 0) passes = ((long long)n * (long long)sizeof(float4) + kScatterRegion - 1) / kScatterRegion;
     passes = std::max(1LL, std::min(passes, std::min(8LL, nc)));
     for (long long q = 0; q < passes; ++q) {
