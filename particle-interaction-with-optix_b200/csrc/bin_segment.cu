@@ -15,9 +15,10 @@
 // place per particle (in passes over cell ranges that fit L2, each reading all tickets again), and ranks
 // each record against its cell through L1.  Here the atomics and the gathers stay in shared memory and
 // the dense counts and offsets are written once, without being zeroed or read.  Measured on B200, whole
-// build, ticket path -> segments: 10M at 10 per cell 554 -> 468 us, at 80 per cell 766 -> 572; 4M on a
-// sphere shell of 64M cells 436 -> 345; 4.2M at 16 per cell 235 -> 214; but 3M at 14 per cell 172 -> 193
-// and 1M at 10 per cell 71 -> 85, hence kSegMinParticles.  At 10M: count 51 us, scatter 3 x 72 (bound by
+// build, ticket path -> segments: 10M at 10 per cell 548 -> 456 us, at 80 per cell 787 -> 556, sorted already
+// 337 -> 273; 4M on a sphere shell of 64M cells 423 -> 330; 4.2M at 16 per cell 228 -> 198; behind the open
+// gate (10M, 100,000 of them in one cell) 3791 -> 3913; but 3M at 14 per cell 172 -> 193 and 1M at 10 per cell
+// 71 -> 85, hence kSegMinParticles.  At 10M: count 62 us, scatter 3 x 73 (bound by
 // 16-byte writes to random sectors, about 65 per ns; the time does not depend on the instructions,
 // the loads in flight or the occupancy), sort 132 (instructions and shared-memory wavefronts, 70% of
 // the issue slots).

@@ -28,7 +28,7 @@
 // uniform particles: 484 against 514 us at 10 per cell, 828 against 1013 at 30, 1805 against 2378 at
 // 80, but 401 against 367 at 5 and 379 against 285 at 2 (rows too thin to fill the lanes); at 12 per
 // cell 18 against 40 us for 1,000 particles and 47 against 79 for 100,000, where a warp's 16 targets
-// instead of 64 leave fewer SMs idle; 10M at 10 per cell 2.12 against 2.33 ms.
+// instead of 64 leave fewer SMs idle; 10M at 10 per cell 2.14 against 2.33 ms.
 #pragma once
 
 #include <algorithm>
@@ -45,7 +45,7 @@ constexpr int kCluGroup = 16;        // targets that share their candidate range
 constexpr int kCluList = 256;        // accepted candidates a warp holds in shared memory
 constexpr int kCluSegment = 64;      // cells of a row from whose start clusters are counted (far targets stay apart;
                                      // a segment's last group is half empty: 10M at 10 per cell loses 1% at 16 cells)
-constexpr int kCluWarpsPerSm = 28;   // 72 registers per thread (64 spill: 2.98 against 2.86 ms for a 10M step)
+constexpr int kCluWarpsPerSm = 28;   // 72 registers per thread (64 spill: a 10M step takes 4% longer)
 
 // A warp's shared memory: the accepted candidates by coordinate, and the candidate ranges.
 struct CluSmem {
@@ -125,7 +125,7 @@ __device__ __forceinline__ void clu_walk(const CluSmem& sm, int cnt, int s, floa
 // Groups per warp for a launch of `waves` waves of one-group warps: the square root balances what a warp
 // pays once (its segment, the block's totals) against the last, partly empty wave.  Measured, pair stage at
 // 10 per cell, best of 1 to 16 groups: 1 at 1.5 waves (100,000 particles), 3 at 6, 4 at 15 and 25, 6 to 8
-// at 45, 8 at 90; 10M (150 waves) 2.17 ms at 4 groups, 2.04 at 16.
+// at 45, 8 at 90; 10M (150 waves) 2.22 ms at 4 groups, 2.14 at 12 and 16, 2.15 at 8 and 24.
 inline int clu_groups_per_warp(double waves) { return std::max(1, (int)(std::sqrt(waves) + 0.5)); }
 
 // Blocks to make room for in a launch over nk targets of `waves` waves, of which each is one_wave blocks without
