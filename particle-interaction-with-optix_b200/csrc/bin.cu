@@ -354,9 +354,9 @@ __global__ void __launch_bounds__(1024) k_large_sort(float4* __restrict__ tmp, c
                                                      int n, SortOut so, const int* large,
                                                      int large_cap) {
     chain_wait();
-    chain_next();
     __shared__ float4 sbuf[2048];
     const int count = min(large[0], large_cap);
+    if (count <= 0) chain_next();  // else the pair kernel's first blocks would share the SMs without a large cell
     const int tid = threadIdx.x;
     for (int li = blockIdx.x; li < count; li += gridDim.x) {
         const int c = large[1 + li];
@@ -433,7 +433,6 @@ __global__ void __launch_bounds__(256) k_descriptors(const int* offsets, long lo
                                                      lj_cell_desc* __restrict__ cells,
                                                      const unsigned* gate = nullptr) {
     chain_wait();
-    chain_next();
     if (closed(gate)) return;
     for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < ncells;
          c += (long long)gridDim.x * blockDim.x) {

@@ -177,7 +177,13 @@ namespace ljc {
 // Launch chaining inside one call's kernel sequence: a kernel launched with chain_launch may be scheduled
 // while its predecessor's last blocks still run; it calls chain_wait before its first access to memory
 // (which returns when every earlier grid it depends on has completed and its writes are visible), and
-// chain_next lets its own successor be scheduled in turn.  What earlier kernels of the chain may write during
+// chain_next lets its own successor be scheduled in turn.  A successor that is scheduled while SMs come free one
+// after the other puts as many of its first blocks on those as fit, so a kernel whose successor may be a pair
+// kernel does not call chain_next before its uneven work is done, or at all: then the successor comes when every
+// SM is free.  Crowded cells put a pair kernel's work into few neighbouring blocks, which then queue on few SMs (u^4
+// particles towards a corner, kernel 12 behind its list, 840,000 of them 6.8 ms, with chain_next in the list's
+// kernel 12.3; 300,000 cluster walks behind one another 0.61 ms, with chain_next 0.72); evenly filled cells take
+// the same time either way.  What earlier kernels of the chain may write during
 // that time -- all but the caller's positions of a build, which a kernel launched without the attribute reads
 // first -- is read with ordinary loads: not with __ldg, nor through a const pointer marked __restrict__, since
 // the read-only path is for data that is constant for the kernel's whole life and its loads may be moved in

@@ -19,7 +19,6 @@ __global__ void __launch_bounds__(32 * kCluWarps, kCluWarpsPerSm / kCluWarps)
                    lj_totals* totals, unsigned* status) {
     __shared__ __align__(16) CluSmem sm[kCluWarps];
     chain_wait();
-    chain_next();
     if (pp.gate && *pp.gate != pp.want) return;
     const int w = (int)(threadIdx.x >> 5);
     const long long first = a0 + (long long)blockIdx.x * stretch;
@@ -49,7 +48,8 @@ __global__ void __launch_bounds__(32 * kCluWarps, kCluWarpsPerSm / kCluWarps)
                                   }
                               });
     }
-    __syncwarp();
+    __syncthreads();
+    chain_next();  // every walk of the grid has ended when this counts: what follows may share the totals' time
     reduce_totals<32 * kCluWarps>(0.5 * (double)pp.e4 * te, 0.5 * (double)pp.e24 * tw, tp, part, counter, totals);
 }
 

@@ -139,7 +139,6 @@ __global__ void __launch_bounds__(256) k_cellpair_flags(const int* cs, const int
 __global__ void __launch_bounds__(256) k_cellpair_list(const int* flag, const int* pos,
                                                        int nk, int kb, int* __restrict__ list) {
     chain_wait();
-    chain_next();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nk; i += gridDim.x * blockDim.x) {
         const int q = pos[i];
         if (flag[i] && q >= 0 && q < nk) list[q] = kb + i;

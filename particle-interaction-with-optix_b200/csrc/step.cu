@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(256) k_verlet_carry(float4* __restrict__ rec, 
                                                       const int* __restrict__ ids, int n, float* __restrict__ vel,
                                                       unsigned* status) {
     chain_wait();
-    chain_next();
+    if ((long long)gridDim.x * blockDim.x >= n) chain_next();  // one round each: the blocks end together
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
         float4 r = rec[s];
         int o = __float_as_int(r.w);
